@@ -78,12 +78,16 @@ static unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 // ========================================================== kernels ======
 
 // Collocation of one (batch, function block) pair per CTA.  Lane l of a warp
-// owns the four consecutive functions f = 4l .. 4l+3 of the block (so the
-// functions of a shell share one radial factor, RadialCache); warp w owns
-// points g = w + 8j.  Output PhiT[pair][comp][g][f], comp 0 = value,
-// 1..3 = gradient (GRAD only); each warp store covers 32 x 4 consecutive f.
+// owns the four consecutive functions f = 4l .. 4l+3 of the block; warp w owns
+// points g = w + 8j.  Per point the warp first evaluates the radial factor of
+// each of the block's shells once (block_radials), since the plan order gives
+// a lane four functions of different shells.  Output PhiT[pair][comp][g][f],
+// comp 0 = value, 1..3 = gradient (GRAD only); each warp store covers 32 x 4
+// consecutive f.
 template <bool GRAD>
-__global__ void __launch_bounds__(256) colloc_fp64_kernel(const StoFunc *__restrict__ sto, const double *__restrict__ px,
+__global__ void __launch_bounds__(256) colloc_fp64_kernel(const StoFunc *__restrict__ sto, const int *__restrict__ fshell,
+                                                          const StoShell *__restrict__ bshell,
+                                                          const int *__restrict__ bnshell, const double *__restrict__ px,
                                                           const double *__restrict__ py, const double *__restrict__ pz,
                                                           const int *__restrict__ pair_batch,
                                                           const int *__restrict__ pair_blk, long p0,
@@ -92,28 +96,24 @@ __global__ void __launch_bounds__(256) colloc_fp64_kernel(const StoFunc *__restr
   const int b = pair_batch[p], I = pair_blk[p];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ double sx[kBatch], sy[kBatch], sz[kBatch];
+  __shared__ BlockFuncs B;
+  __shared__ double wR[8][128], wC[8][128];
   for (int g = threadIdx.x; g < kBatch; g += blockDim.x) {
     sx[g] = px[(long)b * kBatch + g];
     sy[g] = py[(long)b * kBatch + g];
     sz[g] = pz[(long)b * kBatch + g];
   }
+  load_block_funcs(B, sto, fshell, bshell, bnshell, I, threadIdx.x, blockDim.x);
   __syncthreads();
-  StoFunc f[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) f[c] = sto[I * kBlockF + 4 * lane + c];
   const size_t tile = (size_t)kBatch * kBlockF;
   double *o = out + (size_t)blockIdx.x * (GRAD ? 4 : 1) * tile;
   for (int g = warp; g < kBatch; g += 8) {
     const double x = sx[g], y = sy[g], z = sz[g];
-    RadialCache rc;
     double v[4][4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (GRAD)
-        sto_value_grad_cached(f[c], x, y, z, rc, v[0][c], v[1][c], v[2][c], v[3][c]);
-      else
-        v[0][c] = sto_value_cached(f[c], x, y, z, rc);
-    }
+    __syncwarp();
+    block_radials<GRAD, false>(B, lane, x, y, z, wR[warp], wC[warp]);
+    __syncwarp();
+    block_funcs_eval4<GRAD>(B, lane, x, y, z, wR[warp], wC[warp], v[0], v[1], v[2], v[3]);
     const size_t idx = (size_t)g * kBlockF + 4 * lane;
 #pragma unroll
     for (int k = 0; k < (GRAD ? 4 : 1); ++k) {
@@ -134,43 +134,60 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Density of one 64-point tile of one batch for one spin, FP64.
-// T(g,i) = sum_f PhiT(g,f) C(f,i) over the batch's significant blocks (and
-// the three gradient components), then rho = sum_i occ_i T^2 and
-// grad rho = 2 sum_i occ_i T grad T (density.hpp:188-255).  Thread (ty, tx)
-// owns points g = ty + 16a (a < 4) and orbitals i = tx + 16c (c < 4) of the
-// CTA's 64-orbital tile.  The orbital tile is the fastest index of the grid,
-// so the CTAs of one 64-point slab run together and its PhiT rows come from
-// L2 after the first (at 2850 orbitals a slab serves 45 tiles); each CTA adds
-// its tile's share of rho and grad rho atomically (they are zeroed by the
-// caller).  A K step is 16 functions of one block: the
-// PhiT rows (16 contiguous functions per component and point) and the rows
-// of the function-major orbitals Cf (64 contiguous orbitals per function)
-// stream into shared memory with 16-byte cp.async copies through a ring of
-// kDStages stages while the previous steps are multiplied.
-constexpr int kDKs = 16, kDStages = 3;
-template <bool GRAD>
-constexpr int kDStageDoubles = (GRAD ? 4 : 1) * 64 * kDKs + kDKs * 64;
-template <bool GRAD>
-constexpr int kDSmemBytes = kDStages * kDStageDoubles<GRAD> * 8;
+// D += A B on the FP64 tensor path: A 8 x 4 (thread t holds row t / 4,
+// column t % 4), B 4 x 8 (row t % 4, column t / 4), D 8 x 8 (row t / 4,
+// columns 2 (t % 4) and + 1)
+__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
 
-template <bool GRAD>
-__global__ void __launch_bounds__(256) density_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ Cf,
-                                                           const double *__restrict__ occ, int nocc, int nocc_pad,
-                                                           int nbf_pad, const int *__restrict__ pair_off,
-                                                           const int *__restrict__ pair_blk, long b0, long p0,
-                                                           double *__restrict__ rho, double *__restrict__ grad,
-                                                           long npad) {
-  constexpr int NC = GRAD ? 4 : 1;
-  constexpr int SD = kDStageDoubles<GRAD>;
-  extern __shared__ __align__(16) double dsm[];  // [stage][Ps: NC x 64 points x 16 | Cs: 16 x 64 orbitals]
+// Density of one slab of one batch for one spin, FP64: T(g, i) = sum_f
+// PhiT(g, f) C(f, i) over the batch's significant blocks (and the three
+// gradient components), then rho = sum_i occ_i T^2 and grad rho =
+// 2 sum_i occ_i T grad T (density.hpp:188-255).  A CTA takes 64 points with
+// gradients or all 256 without, and NT = 8 NN orbitals.  Its 256 (component,
+// point) rows go 32 to a warp as four 8-row DMMA tiles -- the four components
+// of eight points, so a thread holds T and grad T of the same point and
+// orbitals.  A K step is 16 functions of one block: the rows of PhiT and of
+// the function-major orbitals Cf stream into shared memory by 16-byte
+// cp.async through a ring of STAGES; rows are padded by four doubles, which
+// makes both fragment reads free of bank conflicts.  The orbital tile is the
+// fastest grid index, so the CTAs of one slab run together and read its PhiT
+// rows from L2; each adds its share of rho and grad rho atomically (zeroed by
+// the caller).
+//
+// Bound: FP64 pipe from about 16 orbitals on, PhiT from HBM below.  The
+// orbital tile is ceil(nocc / ntile / 8) * 8 wide instead of a fixed 64, so 5
+// to 40 occupied orbitals do not pay for 64 columns; up to 32 columns the
+// accumulators leave room for two CTAs an SM.
+constexpr int kDKs = 16;
+template <int NN>
+struct DShape {
+  static constexpr int NT = 8 * NN, LDP = kDKs + 4, LDC = NT + 4;
+  static constexpr int STAGES = NN <= 4 ? 2 : 3, CTAS = NN <= 4 ? 2 : 1;
+  static constexpr int kStage = 256 * LDP + kDKs * LDC;  // doubles
+  static constexpr int kSmem = STAGES * kStage * 8;
+};
+
+template <bool GRAD, int NN>
+__global__ void __launch_bounds__(256, DShape<NN>::CTAS)
+    density_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ Cf, const double *__restrict__ occ,
+                        int nocc, int nocc_pad, int nbf_pad, const int *__restrict__ pair_off,
+                        const int *__restrict__ pair_blk, long b0, long p0, double *__restrict__ rho,
+                        double *__restrict__ grad, long npad) {
+  using Sh = DShape<NN>;
+  constexpr int NC = GRAD ? 4 : 1, NT = Sh::NT, LDP = Sh::LDP, LDC = Sh::LDC, ST = Sh::STAGES;
+  constexpr int SLABS = GRAD ? 4 : 1;  // slabs of a batch
+  extern __shared__ __align__(16) double dsm[];  // [stage][Ps: 256 rows x LDP | Cs: 16 x LDC]
   const int spin = blockIdx.y;
-  const int ntile = nocc_pad / 64;
-  const int i0 = (blockIdx.x % ntile) * 64;
+  const int ntile = nocc_pad / NT;
+  const int i0 = (blockIdx.x % ntile) * NT;
   const long bq = blockIdx.x / ntile;
-  const long b = b0 + bq / 4;
-  const int g0 = (int)(bq % 4) * 64;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const long b = b0 + bq / SLABS;
+  const int g0 = (int)(bq % SLABS) * 64;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double *C = Cf + (size_t)spin * nbf_pad * nocc_pad;
   const double *oc = occ + (size_t)spin * nocc;
   const int q0 = pair_off[b], q1 = pair_off[b + 1];
@@ -179,84 +196,81 @@ __global__ void __launch_bounds__(256) density_fp64_kernel(const double *__restr
   if (total == 0) return;  // no significant function: nothing to add
   auto issue = [&](int t, int st) {
     if (t < total) {
-      const int r = t;
-      const int q = q0 + r / (kBlockF / kDKs), f0 = (r % (kBlockF / kDKs)) * kDKs;
+      const int q = q0 + t / (kBlockF / kDKs), f0 = (t % (kBlockF / kDKs)) * kDKs;
       const double *P = phiT + (size_t)(q - p0) * NC * tile + (size_t)g0 * kBlockF + f0;
-      double *Ps = dsm + st * SD, *Cs = Ps + NC * 64 * kDKs;
-      for (int e = threadIdx.x; e < NC * 64 * (kDKs / 2); e += 256) {
-        const int row = e / (kDKs / 2), part = e % (kDKs / 2);  // row = (comp, point)
-        cp_async16(Ps + row * kDKs + 2 * part, P + (size_t)(row / 64) * tile + (size_t)(row % 64) * kBlockF + 2 * part);
+      double *Ps = dsm + st * Sh::kStage, *Cs = Ps + 256 * LDP;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int e = threadIdx.x + 256 * r, row = e / (kDKs / 2), part = e % (kDKs / 2);
+        // GRAD: row = 32 (point / 8) + 8 comp + point % 8
+        const int c = GRAD ? (row / 8) % 4 : 0, pt = GRAD ? 8 * (row / 32) + row % 8 : row;
+        cp_async16(Ps + row * LDP + 2 * part, P + c * tile + (size_t)pt * kBlockF + 2 * part);
       }
       const double *Cr = C + (size_t)(pair_blk[q] * kBlockF + f0) * nocc_pad + i0;
-      for (int e = threadIdx.x; e < kDKs * 32; e += 256) {
-        const int k = e / 32, part = e % 32;
-        cp_async16(Cs + k * 64 + 2 * part, Cr + (size_t)k * nocc_pad + 2 * part);
+      for (int e = threadIdx.x; e < kDKs * NT / 2; e += 256) {
+        const int k = e / (NT / 2), part = e % (NT / 2);
+        cp_async16(Cs + k * LDC + 2 * part, Cr + (size_t)k * nocc_pad + 2 * part);
       }
     }
     cp_async_commit();
   };
 #pragma unroll
-  for (int st = 0; st < kDStages - 1; ++st) issue(st, st);
-  double acc[NC][4][4];
+  for (int st = 0; st < ST - 1; ++st) issue(st, st);
+  double acc[4][NN][2];
 #pragma unroll
-  for (int c = 0; c < NC; ++c)
+  for (int m = 0; m < 4; ++m)
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[c][a][j] = 0.0;
+    for (int n = 0; n < NN; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
+  const int fr = lane >> 2, fk = lane & 3;
   for (int t = 0; t < total; ++t) {
-    cp_async_wait<kDStages - 2>();
+    cp_async_wait<ST - 2>();
     __syncthreads();  // step t is visible; the stage refilled below was read in step t - 1
-    issue(t + kDStages - 1, (t + kDStages - 1) % kDStages);
-    const double *Ps = dsm + (t % kDStages) * SD, *Cs = Ps + NC * 64 * kDKs;
+    issue(t + ST - 1, (t + ST - 1) % ST);
+    const double *Ps = dsm + (t % ST) * Sh::kStage, *Cs = Ps + 256 * LDP;
 #pragma unroll
-    for (int k = 0; k < kDKs; ++k) {
-      double bv[4];
+    for (int k = 0; k < kDKs; k += 4) {
+      double av[4], bv[NN];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Cs[k * 64 + tx + 16 * j];
+      for (int m = 0; m < 4; ++m) av[m] = Ps[(32 * warp + 8 * m + fr) * LDP + k + fk];
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
+      for (int n = 0; n < NN; ++n) bv[n] = Cs[(k + fk) * LDC + 8 * n + fr];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const double av = Ps[(c * 64 + ty + 16 * a) * kDKs + k];
+      for (int m = 0; m < 4; ++m)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[c][a][j] = fma(av, bv[j], acc[c][a][j]);
-        }
-    }
-    if (t == total - 1) {
-      // contract over this orbital tile
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        double sm[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int i = i0 + tx + 16 * j;
-          const double o = i < nocc ? oc[i] : 0.0;
-          const double tv = acc[0][a][j];
-          sm[0] += o * tv * tv;
-          if (GRAD) {
-            sm[1] += o * tv * acc[NC > 1 ? 1 : 0][a][j];
-            sm[2] += o * tv * acc[NC > 2 ? 2 : 0][a][j];
-            sm[3] += o * tv * acc[NC > 3 ? 3 : 0][a][j];
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-          for (int off = 8; off; off >>= 1) sm[k] += __shfl_xor_sync(0xffffffffu, sm[k], off);
-        if (tx == 0) {
-          const long g = b * kBatch + g0 + ty + 16 * a;
-          atomicAdd(&rho[(size_t)spin * npad + g], sm[0]);
-          if (GRAD) {
-            atomicAdd(&grad[((size_t)spin * 3 + 0) * npad + g], 2.0 * sm[1]);
-            atomicAdd(&grad[((size_t)spin * 3 + 1) * npad + g], 2.0 * sm[2]);
-            atomicAdd(&grad[((size_t)spin * 3 + 2) * npad + g], 2.0 * sm[3]);
-          }
-        }
-      }
+        for (int n = 0; n < NN; ++n) dmma884(acc[m][n], av[m], bv[n]);
     }
   }
   cp_async_wait<0>();
+  // contract over this orbital tile: the four lanes of a row hold its columns
+  double sm[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int n = 0; n < NN; ++n)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = i0 + 8 * n + 2 * fk + h;
+      const double o = i < nocc ? oc[i] : 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) sm[m] += o * acc[GRAD ? 0 : m][n][h] * acc[m][n][h];
+    }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    sm[m] += __shfl_xor_sync(0xffffffffu, sm[m], 1);
+    sm[m] += __shfl_xor_sync(0xffffffffu, sm[m], 2);
+  }
+  if (fk == 0) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (GRAD) {
+        const long g = b * kBatch + g0 + 8 * warp + fr;
+        if (m == 0)
+          atomicAdd(&rho[(size_t)spin * npad + g], sm[0]);
+        else
+          atomicAdd(&grad[((size_t)spin * 3 + m - 1) * npad + g], 2.0 * sm[m]);
+      } else {
+        atomicAdd(&rho[(size_t)spin * npad + b * kBatch + 32 * warp + 8 * m + fr], sm[m]);
+      }
+    }
+  }
 }
 
 // Orbitals in function-major order for density_fp64_kernel:
@@ -272,7 +286,7 @@ __global__ void transpose_orbitals_kernel(const double *__restrict__ Ct, int noc
   }
   __syncthreads();
   for (int r = threadIdx.y; r < 32; r += blockDim.y)
-    Cf[((size_t)spin * nbf_pad + f0 + r) * nocc_pad + i0 + threadIdx.x] = t[threadIdx.x][r];
+    if (i0 + threadIdx.x < nocc_pad) Cf[((size_t)spin * nbf_pad + f0 + r) * nocc_pad + i0 + threadIdx.x] = t[threadIdx.x][r];
 }
 
 // Functional on points [0, n) of the arrays given (plane stride npad; callers
@@ -381,94 +395,136 @@ __device__ __forceinline__ bool block_has(const uint32_t *m, int I) { return (m[
 
 // V contraction of the FP64 build: Vbar(I, J) += sum_b PhiT_b,I^T Z_b,J over
 // the chunk's batches b where blocks I and J are both significant
-// (xc_integrals.hpp:677-706), one 128 x 128 output tile per CTA (8 x 8 per
-// thread).  The operand rows of a pair, PhiT[g][f] and Z^T[g][f], are 1 KB
-// rows of 128 functions per point, so each 16-point K step of both operands
-// (32 KB) streams into shared memory with 16-byte cp.async copies through a
-// ring of kVStages stages while the previous steps are multiplied.
-constexpr int kVKs = 16, kVStages = 4;
-constexpr int kVStageDoubles = 2 * kVKs * kBlockF;
+// (xc_integrals.hpp:677-706), one 128 x 128 output tile per CTA: eight warps
+// of 64 x 32, DMMA tiles of 8 x 8 x 4.  The operand rows of a pair, PhiT[g][f]
+// and Z^T[g][f], are 1 KB rows of 128 functions per point, so each 16-point K
+// step of both operands (32 KB) streams into shared memory with 16-byte
+// cp.async copies through a ring of kVStages stages while the previous steps
+// are multiplied; rows are padded by four doubles (conflict-free fragments).
+//
+// Split over batches: a basis of one to a few blocks has only nz nblk^2
+// output tiles, far fewer than SMs.  With nsplit > 1 the batches of a tile
+// are dealt to nsplit CTAs, each of which writes its partial tile to part[]
+// (thread-major, coalesced); vpart_reduce_kernel adds the parts in order, so
+// the result does not depend on scheduling.
+//
+// Bound: FP64 pipe.  Whole FP64 builds, before (CUDA-core tiles, one CTA per
+// output tile, 64-column density, a radial factor per function) and after:
+// one water LDA + J 14.3 -> 0.77 ms (the V contraction was 13.4 of it, on two
+// SMs), (H2O)_5 open-shell PBE 70.3 -> 6.3 ms (64.3 of it, on eight SMs).
+constexpr int kVKs = 16, kVStages = 4, kVLd = kBlockF + 4;
+constexpr int kVStageDoubles = 2 * kVKs * kVLd;
 constexpr int kVSmemBytes = kVStages * kVStageDoubles * 8;
 
-// next K step of a V unit: step k of batch b, batches without both blocks skipped
-__device__ __forceinline__ void vstep_next(const uint32_t *__restrict__ mask, int mask_words, long b1, int I, int J,
-                                           long &b, int &k) {
+// next K step of a V unit: step k of batch b, batches without both blocks
+// skipped; b walks with stride db
+__device__ __forceinline__ void vstep_next(const uint32_t *__restrict__ mask, int mask_words, long b1, int db, int I,
+                                           int J, long &b, int &k) {
   if (++k < kBatch / kVKs) return;
   k = 0;
-  for (++b; b < b1; ++b) {
+  for (b += db; b < b1; b += db) {
     const uint32_t *m = mask + b * mask_words;
     if (block_has(m, I) && block_has(m, J)) return;
   }
 }
 
-__global__ void __launch_bounds__(256) vgemm_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ zT,
-                                                         int phi_stride_tiles, int z_stride, const int *__restrict__ pair_off,
-                                                         const uint32_t *__restrict__ mask, int mask_words, long b0,
-                                                         long b1, long p0, int nbf_pad, double *__restrict__ V) {
-  extern __shared__ __align__(16) double vsm[];  // [stage][A | B][kVKs][128]
-  const int J = blockIdx.x, I = blockIdx.y, zi = blockIdx.z;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+// element e of thread t of a tile: rows and columns of warp (t / 32)'s 64 x 32 part
+__device__ __forceinline__ void vtile_element(int t, int e, int &r, int &c) {
+  const int lane = t & 31, warp = t >> 5;
+  r = 64 * (warp & 1) + 8 * (e >> 3) + (lane >> 2);
+  c = 32 * (warp >> 1) + 8 * ((e >> 1) & 3) + 2 * (lane & 3) + (e & 1);
+}
+
+__global__ void __launch_bounds__(256, 1)
+    vgemm_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ zT, int phi_stride_tiles,
+                      int z_stride, const int *__restrict__ pair_off, const uint32_t *__restrict__ mask,
+                      int mask_words, long b0, long b1, long p0, int nsplit, int nbf_pad, double *__restrict__ V,
+                      double *__restrict__ part) {
+  extern __shared__ __align__(16) double vsm[];  // [stage][A | B][kVKs][kVLd]
+  const int J = blockIdx.x, I = blockIdx.y, zi = blockIdx.z / nsplit, sp = blockIdx.z % nsplit;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t tile = (size_t)kBatch * kBlockF;
-  // first step: the first batch with both blocks significant
-  long lb = b0 - 1;
+  // first step: the split's first batch with both blocks significant
+  long lb = b0 + sp - nsplit;
   int lk = kBatch / kVKs - 1;
-  vstep_next(mask, mask_words, b1, I, J, lb, lk);
-  if (lb >= b1) return;
+  vstep_next(mask, mask_words, b1, nsplit, I, J, lb, lk);
+  if (lb >= b1 && nsplit == 1) return;
   long cb = lb;
   int ck = lk;
-  // issue the copies of step (lb, lk) into stage st; returns false past the end
   auto issue = [&](int st) {
     if (lb < b1) {
       const uint32_t *m = mask + lb * mask_words;
       const long qb = pair_off[lb] - p0;
       const double *A = phiT + (size_t)(qb + block_pos(m, I)) * phi_stride_tiles * tile + (size_t)lk * kVKs * kBlockF;
       const double *B = zT + ((size_t)(qb + block_pos(m, J)) * z_stride + zi) * tile + (size_t)lk * kVKs * kBlockF;
-      double *dA = vsm + st * kVStageDoubles, *dB = dA + kVKs * kBlockF;
+      double *dA = vsm + st * kVStageDoubles, *dB = dA + kVKs * kVLd;
 #pragma unroll
       for (int r = 0; r < (kVKs * kBlockF / 2) / 256; ++r) {
-        const int e = 2 * (threadIdx.x + 256 * r);
-        cp_async16(dA + e, A + e);
-        cp_async16(dB + e, B + e);
+        const int e = 2 * (threadIdx.x + 256 * r), d = (e / kBlockF) * kVLd + e % kBlockF;
+        cp_async16(dA + d, A + e);
+        cp_async16(dB + d, B + e);
       }
-      vstep_next(mask, mask_words, b1, I, J, lb, lk);
+      vstep_next(mask, mask_words, b1, nsplit, I, J, lb, lk);
     }
     cp_async_commit();  // an empty group past the end keeps the group count uniform
   };
 #pragma unroll
   for (int st = 0; st < kVStages - 1; ++st) issue(st);
-  double acc[8][8];
+  double acc[8][4][2];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int fr = lane >> 2, fk = lane & 3, r0 = 64 * (warp & 1) + fr, c0 = 32 * (warp >> 1) + fr;
   for (int it = 0; cb < b1; ++it) {
     cp_async_wait<kVStages - 2>();
     __syncthreads();  // step it is visible; the stage refilled below was read in step it - 1
     issue((it + kVStages - 1) % kVStages);
-    const double *As = vsm + (it % kVStages) * kVStageDoubles, *Bs = As + kVKs * kBlockF;
+    const double *As = vsm + (it % kVStages) * kVStageDoubles, *Bs = As + kVKs * kVLd;
 #pragma unroll
-    for (int k = 0; k < kVKs; ++k) {
-      double a[8], bb[8];
+    for (int k = 0; k < kVKs; k += 4) {
+      double a[8], bb[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = As[k * kBlockF + ty + 16 * i];
+      for (int i = 0; i < 8; ++i) a[i] = As[(k + fk) * kVLd + r0 + 8 * i];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) bb[j] = Bs[k * kBlockF + tx + 16 * j];
+      for (int j = 0; j < 4; ++j) bb[j] = Bs[(k + fk) * kVLd + c0 + 8 * j];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) dmma884(acc[i][j], a[i], bb[j]);
     }
-    vstep_next(mask, mask_words, b1, I, J, cb, ck);
+    vstep_next(mask, mask_words, b1, nsplit, I, J, cb, ck);
   }
   cp_async_wait<0>();
+  if (nsplit > 1) {
+    double *o = part + ((((size_t)zi * gridDim.y + I) * gridDim.x + J) * nsplit + sp) * kBlockF * kBlockF + threadIdx.x;
+#pragma unroll
+    for (int e = 0; e < 64; ++e) o[e * 256] = acc[e >> 3][(e >> 1) & 3][e & 1];
+    return;
+  }
   double *Vz = V + (size_t)zi * nbf_pad * nbf_pad;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const size_t r = (size_t)I * 128 + ty + 16 * i, c = (size_t)J * 128 + tx + 16 * j;
-      Vz[r + c * nbf_pad] += acc[i][j];
-    }
+  for (int e = 0; e < 64; ++e) {
+    int r, c;
+    vtile_element(threadIdx.x, e, r, c);
+    Vz[(size_t)I * 128 + r + ((size_t)J * 128 + c) * nbf_pad] += acc[e >> 3][(e >> 1) & 3][e & 1];
+  }
+}
+
+// Vbar += the parts of a split vgemm_fp64_kernel, in split order: block
+// (tile, element e of every thread), one output element per thread
+__global__ void __launch_bounds__(256) vpart_reduce_kernel(const double *__restrict__ part, int nsplit, int nblk,
+                                                           int nbf_pad, double *__restrict__ V) {
+  const int t = blockIdx.x, J = t % nblk, I = (t / nblk) % nblk, zi = t / (nblk * nblk);
+  const double *p = part + (size_t)t * nsplit * kBlockF * kBlockF + threadIdx.x;
+  double *Vz = V + (size_t)zi * nbf_pad * nbf_pad;
+  const int e = blockIdx.y;
+  double s = 0.0;
+#pragma unroll 8
+  for (int k = 0; k < nsplit; ++k) s += p[((size_t)k * 64 + e) * 256];
+  int r, c;
+  vtile_element(threadIdx.x, e, r, c);
+  Vz[(size_t)I * 128 + r + ((size_t)J * 128 + c) * nbf_pad] += s;
 }
 
 // out(i, j) = Vp(pi, pj) + Vp(pj, pi), p = finv[.] the plan position of
@@ -532,7 +588,7 @@ __global__ void pack_orbitals_kernel(const double *__restrict__ C, const double 
   if (bad) atomicOr(nonfinite, 1);
 }
 
-// y_a += sum over a slice of points of w_g rho_g V_a(g) for the functions of
+// y[slice][a] = sum over a slice of points of w_g rho_g V_a(g) for the functions of
 // one aux shell: the radial factor once per point, then C S_lm per m
 // (coulomb.hpp:84-85).  Every thread of a block works on the same shell, so
 // the solid-harmonic branch is uniform.
@@ -540,7 +596,7 @@ __global__ void aux_y_shell_kernel(const AuxShell *__restrict__ shells, const in
                                    const double *__restrict__ px, const double *__restrict__ py,
                                    const double *__restrict__ pz, const double *__restrict__ w,
                                    const double *__restrict__ rho, int nspin, long npad, long slice,
-                                   const float *__restrict__ rtab, double *__restrict__ y) {
+                                   const float *__restrict__ rtab, int naux, double *__restrict__ y) {
   const int shell = list[blockIdx.x];
   const AuxShell sh = shells[shell];
   const AuxFunc &f = sh.f;
@@ -573,7 +629,7 @@ __global__ void aux_y_shell_kernel(const AuxShell *__restrict__ shells, const in
     if (threadIdx.x < 32) {
       s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
       for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (threadIdx.x == 0) atomicAdd(y + sh.first + k, s);
+      if (threadIdx.x == 0) y[(size_t)blockIdx.y * naux + sh.first + k] = s;
     }
   }
 }
@@ -605,7 +661,7 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const Aux
                                    const double *__restrict__ px, const double *__restrict__ py,
                                    const double *__restrict__ pz, const double *__restrict__ w,
                                    const double *__restrict__ rho, int nspin, long npad, long slice,
-                                   const float *__restrict__ rtab, double *__restrict__ y) {
+                                   const float *__restrict__ rtab, int naux, double *__restrict__ y) {
   constexpr int NM = 2 * L + 1, QM = aux_group_max(L);
   const AuxGroup G = groups[blockIdx.x];
   const long g0 = blockIdx.y * slice, g1 = min(npad, g0 + slice);
@@ -678,7 +734,7 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const Aux
       if (threadIdx.x < 32) {
         s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
         for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) atomicAdd(y + shells[G.first + q].first + m, s);
+        if (threadIdx.x == 0) y[(size_t)blockIdx.y * naux + shells[G.first + q].first + m] = s;
       }
     }
   }
@@ -713,6 +769,16 @@ __device__ __forceinline__ double aux_group_v(const AuxGroup &G, const AuxShell 
     }
   }
   return s;
+}
+
+// y_a = the sum of its slices' shares, in slice order (the fit amplifies
+// rounding differences of y, so the sum does not depend on scheduling)
+__global__ void aux_y_reduce_kernel(const double *__restrict__ part, int nsl, int naux, double *__restrict__ y) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= naux) return;
+  double s = 0.0;
+  for (int k = 0; k < nsl; ++k) s += part[(size_t)k * naux + a];
+  y[a] = s;
 }
 
 // v_g = w_g sum_a c_a V_a(g) over the groups, then the loose shells
@@ -1128,6 +1194,7 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
   P.xc = make_spec(opts);
   P.gga = spec_is_gga(P.xc);
   NKX_CUDA(cudaGetDevice(&P.device));
+  NKX_CUDA(cudaDeviceGetAttribute(&P.nsm, cudaDevAttrMultiProcessorCount, P.device));
   NKX_CUDA(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
   for (auto &e : P.ev) NKX_CUDA(cudaEventCreate(&e));
   P.nbf = prim->nbf;
@@ -1500,12 +1567,9 @@ __global__ void core_z_kernel(const double *__restrict__ phiT, const double *__r
 void launch_colloc(Plan &P, const Chunk &c, cudaStream_t s) {
   const long np = c.p1 - c.p0;
   if (np <= 0) return;
-  if (P.gga)
-    colloc_fp64_kernel<true><<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_px, P.d_py, P.d_pz, P.d_pair_batch,
-                                                          P.d_pair_blk, c.p0, P.ws_phi);
-  else
-    colloc_fp64_kernel<false><<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_px, P.d_py, P.d_pz, P.d_pair_batch,
-                                                           P.d_pair_blk, c.p0, P.ws_phi);
+  auto *kernel = P.gga ? colloc_fp64_kernel<true> : colloc_fp64_kernel<false>;
+  kernel<<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_px, P.d_py, P.d_pz,
+                                      P.d_pair_batch, P.d_pair_blk, c.p0, P.ws_phi);
   NKX_LAUNCH_CHECK();
   ++P.launches;
 }
@@ -1543,9 +1607,17 @@ static const float *coulomb_table(Plan &P, bool mixed, cudaStream_t s) {
 
 void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
     const float *rtab = coulomb_table(P, mixed, s);
-    NKX_CUDA(cudaMemsetAsync(P.d_y, 0, sizeof(double) * P.naux, s));
-    const long nsl = std::max<long>(1, std::min<long>(64, (P.npad + 4095) / 4096));
+    // point slices: 64 or one per 4096 points, and more (down to 1024 points
+    // each) where an l has few groups, so that four blocks an SM are in flight
+    // (one water has 3 groups an l: 17 slices kept 51 of 148 SMs busy)
+    long nsl = std::max<long>(1, std::min<long>(64, (P.npad + 4095) / 4096));
+    auto more_slices = [&](int groups) {
+      if (groups > 0) nsl = std::max(nsl, std::min((4L * P.nsm + groups - 1) / groups, P.npad / 1024));
+    };
+    for (int L = 0; L <= 3; ++L) more_slices(P.h_group_off[L + 1] - P.h_group_off[L]);
+    more_slices(P.nloose);
     const long slice = (P.npad + nsl - 1) / nsl;
+    if (!P.d_ypart) P.d_ypart = P.alloc<double>((size_t)nsl * P.naux);
     for (int L = 0; L <= 3; ++L) {
       const int n = P.h_group_off[L + 1] - P.h_group_off[L];
       if (n == 0) continue;
@@ -1554,27 +1626,27 @@ void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
       switch (L) {
         case 0:
           if (rtab)
-            aux_y_group_kernel<0, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<0, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           else
-            aux_y_group_kernel<0, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<0, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           break;
         case 1:
           if (rtab)
-            aux_y_group_kernel<1, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<1, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           else
-            aux_y_group_kernel<1, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<1, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           break;
         case 2:
           if (rtab)
-            aux_y_group_kernel<2, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<2, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           else
-            aux_y_group_kernel<2, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<2, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           break;
         default:
           if (rtab)
-            aux_y_group_kernel<3, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<3, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           else
-            aux_y_group_kernel<3, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.d_y);
+            aux_y_group_kernel<3, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
           break;
       }
       NKX_LAUNCH_CHECK();
@@ -1583,10 +1655,13 @@ void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
     if (P.nloose > 0) {
       aux_y_shell_kernel<<<dim3(P.nloose, (unsigned)nsl), 256, 0, s>>>(P.d_ashell, P.d_loose, P.d_px, P.d_py, P.d_pz,
                                                                       P.d_w, P.d_rho, nspin, P.npad, slice, rtab,
-                                                                      P.d_y);
+                                                                      P.naux, P.d_ypart);
       NKX_LAUNCH_CHECK();
       ++P.launches;
     }
+    aux_y_reduce_kernel<<<nblk(P.naux, 128), 128, 0, s>>>(P.d_ypart, (int)nsl, P.naux, P.d_y);
+    NKX_LAUNCH_CHECK();
+    ++P.launches;
 }
 
 void coulomb_solve(Plan &P, cudaStream_t s, bool mixed) {
@@ -1625,39 +1700,84 @@ void coulomb_solve(Plan &P, cudaStream_t s, bool mixed) {
     ++P.launches;
 }
 
+template <bool GRAD, int NN>
+static void launch_density_fp64(Plan &P, const Chunk &c, int nspin, int nocc, int nocc_pad, cudaStream_t s) {
+  NKX_CUDA(cudaFuncSetAttribute(density_fp64_kernel<GRAD, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                DShape<NN>::kSmem));
+  const dim3 grid((unsigned)((c.b1 - c.b0) * (GRAD ? 4 : 1) * (nocc_pad / (8 * NN))), nspin);
+  density_fp64_kernel<GRAD, NN><<<grid, 256, DShape<NN>::kSmem, s>>>(P.ws_phi, P.d_Cf, P.d_occ, nocc, nocc_pad,
+                                                                    P.nbf_pad, P.d_pair_off, P.d_pair_blk, c.b0, c.p0,
+                                                                    P.d_rho, P.d_grad, P.npad);
+}
+template <bool GRAD>
+static void launch_density_nn(Plan &P, const Chunk &c, int nn, int nspin, int nocc, int nocc_pad, cudaStream_t s) {
+  switch (nn) {
+    case 1: return launch_density_fp64<GRAD, 1>(P, c, nspin, nocc, nocc_pad, s);
+    case 2: return launch_density_fp64<GRAD, 2>(P, c, nspin, nocc, nocc_pad, s);
+    case 3: return launch_density_fp64<GRAD, 3>(P, c, nspin, nocc, nocc_pad, s);
+    case 4: return launch_density_fp64<GRAD, 4>(P, c, nspin, nocc, nocc_pad, s);
+    case 5: return launch_density_fp64<GRAD, 5>(P, c, nspin, nocc, nocc_pad, s);
+    case 6: return launch_density_fp64<GRAD, 6>(P, c, nspin, nocc, nocc_pad, s);
+    case 7: return launch_density_fp64<GRAD, 7>(P, c, nspin, nocc, nocc_pad, s);
+    default: return launch_density_fp64<GRAD, 8>(P, c, nspin, nocc, nocc_pad, s);
+  }
+}
+
+// The FP64 V contraction of one chunk: nz planes of zT (stride z_stride
+// tiles) against PhiT into V.  Batches are split over as few CTAs per tile
+// as fill at least nine tenths of the last wave (a basis of one block and
+// one plane: one CTA per SM instead of one in all).
+static void launch_vgemm_fp64(Plan &P, const Chunk &c, const double *phiT, const double *zT, int phi_stride,
+                              int z_stride, int nz, double *V, cudaStream_t s) {
+  const long parts = (long)nz * P.nblk * P.nblk, nsm = P.nsm;
+  int nsplit = 1;
+  double best = 0.0;
+  for (long k = 1; k == 1 || (k <= c.b1 - c.b0 && parts * k <= 2 * nsm); ++k) {
+    const double fill = (double)(parts * k) / (double)((parts * k + nsm - 1) / nsm * nsm);
+    if (fill > best + 1e-9) {
+      best = fill;
+      nsplit = (int)k;
+    }
+    if (best >= 0.9) break;
+  }
+  if (nsplit > 1 && !P.d_vpart) P.d_vpart = P.alloc<double>((size_t)2 * nsm * kBlockF * kBlockF);
+  NKX_CUDA(cudaFuncSetAttribute(vgemm_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVSmemBytes));
+  vgemm_fp64_kernel<<<dim3(P.nblk, P.nblk, nz * nsplit), 256, kVSmemBytes, s>>>(
+      phiT, zT, phi_stride, z_stride, P.d_pair_off, P.d_mask, P.mask_words, c.b0, c.b1, c.p0, nsplit, P.nbf_pad, V,
+      P.d_vpart);
+  ++P.launches;
+  if (nsplit > 1) {
+    vpart_reduce_kernel<<<dim3((unsigned)parts, 64), 256, 0, s>>>(P.d_vpart, nsplit, P.nblk, P.nbf_pad, V);
+    ++P.launches;
+  }
+  NKX_LAUNCH_CHECK();
+}
+
 // FP64 pass A: collocation + density of every chunk into d_rho / d_grad
 void fp64_density_pass(Plan &P, int nspin, int nocc, cudaStream_t s, StageTimer &T) {
-  const int nocc_pad = (nocc + 63) / 64 * 64;
+  // orbital tiles of at most 64, equally wide, in multiples of 8
+  const int ntile = (nocc + 63) / 64, nn = ((nocc + ntile - 1) / ntile + 7) / 8;
+  const int nocc_pad = ntile * 8 * nn;
   if ((size_t)nocc_pad * P.nbf_pad * 2 > P.cf_cap) {
     P.cf_cap = (size_t)nocc_pad * P.nbf_pad * 2;
     P.d_Cf = P.alloc<double>(P.cf_cap);
   }
-  transpose_orbitals_kernel<<<dim3(P.nbf_pad / 32, nocc_pad / 32, nspin), dim3(32, 8), 0, s>>>(P.d_Ct, nocc, nocc_pad,
+  transpose_orbitals_kernel<<<dim3(P.nbf_pad / 32, (nocc_pad + 31) / 32, nspin), dim3(32, 8), 0, s>>>(P.d_Ct, nocc, nocc_pad,
                                                                                              P.nbf_pad, P.d_Cf);
   NKX_LAUNCH_CHECK();
   ++P.launches;
-  NKX_CUDA(cudaFuncSetAttribute(density_fp64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kDSmemBytes<true>));
-  NKX_CUDA(cudaFuncSetAttribute(density_fp64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kDSmemBytes<false>));
   // the density kernels add their orbital tiles' shares
   NKX_CUDA(cudaMemsetAsync(P.d_rho, 0, sizeof(double) * nspin * P.npad, s));
   if (P.gga) NKX_CUDA(cudaMemsetAsync(P.d_grad, 0, sizeof(double) * 3 * nspin * P.npad, s));
   for (const Chunk &c : P.chunks) {
-    const long nb = c.b1 - c.b0;
     if (c.p1 - c.p0 > 0) {
       T.begin(ST_COLLOC, s);
       launch_colloc(P, c, s);
       T.end(s);
     }
     T.begin(ST_DENSITY, s);
-    dim3 grid((unsigned)(nb * 4 * (nocc_pad / 64)), nspin);
-    if (P.gga)
-      density_fp64_kernel<true><<<grid, 256, kDSmemBytes<true>, s>>>(P.ws_phi, P.d_Cf, P.d_occ, nocc, nocc_pad, P.nbf_pad, P.d_pair_off,
-                                                     P.d_pair_blk, c.b0, c.p0, P.d_rho, P.d_grad, P.npad);
-    else
-      density_fp64_kernel<false><<<grid, 256, kDSmemBytes<false>, s>>>(P.ws_phi, P.d_Cf, P.d_occ, nocc, nocc_pad, P.nbf_pad, P.d_pair_off,
-                                                      P.d_pair_blk, c.b0, c.p0, P.d_rho, P.d_grad, P.npad);
+    P.gga ? launch_density_nn<true>(P, c, nn, nspin, nocc, nocc_pad, s)
+          : launch_density_nn<false>(P, c, nn, nspin, nocc, nocc_pad, s);
     NKX_LAUNCH_CHECK();
     ++P.launches;
     T.end(s);
@@ -1669,7 +1789,6 @@ void fock_build_fp64(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool s
   const bool multi = P.chunks.size() > 1;
   const int nzs = nspin + (separateJ ? 1 : 0);
   if (!P.ws_z) P.ws_z = P.alloc<double>(std::max<long>(1, P.max_chunk_pairs) * 3 * (size_t)kBatch * kBlockF);
-  NKX_CUDA(cudaFuncSetAttribute(vgemm_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVSmemBytes));
   if (phase != 2) {
     // ---- pass A: collocation + density, and this plan's share of the J fit vector
     fp64_density_pass(P, nspin, nocc, s, T);
@@ -1717,11 +1836,7 @@ void fock_build_fp64(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool s
     ++P.launches;
     T.end(s);
     T.begin(ST_VGEMM, s);
-    vgemm_fp64_kernel<<<dim3(P.nblk, P.nblk, nzs), 256, kVSmemBytes, s>>>(P.ws_phi, P.ws_z, P.gga ? 4 : 1, nzs, P.d_pair_off,
-                                                                P.d_mask, P.mask_words, c.b0, c.b1, c.p0, P.nbf_pad,
-                                                                P.d_V);
-    NKX_LAUNCH_CHECK();
-    ++P.launches;
+    launch_vgemm_fp64(P, c, P.ws_phi, P.ws_z, P.gga ? 4 : 1, nzs, nzs, P.d_V, s);
     T.end(s);
   }
   (void)tile;
@@ -2243,7 +2358,6 @@ NKX_API nkx_status nkx_plan_core_hamiltonian(nkx_plan *plan, const nkx_molecule 
     NKX_CUDA(cudaMemcpyAsync(dc, mol->xyz, sizeof(double) * 3 * mol->natoms, cudaMemcpyHostToDevice, s));
     NKX_CUDA(cudaMemcpyAsync(dz, zc.data(), sizeof(double) * mol->natoms, cudaMemcpyHostToDevice, s));
     if (!P.ws_z) P.ws_z = P.alloc<double>(std::max<long>(1, P.max_chunk_pairs) * 3 * tile);
-    NKX_CUDA(cudaFuncSetAttribute(vgemm_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVSmemBytes));
     core_vne_kernel<<<nblk(P.npad, 256), 256, 0, s>>>(P.d_px, P.d_py, P.d_pz, P.d_w, P.npad, dc, dz, mol->natoms,
                                                      P.d_vj);
     NKX_LAUNCH_CHECK();
@@ -2258,14 +2372,12 @@ NKX_API nkx_status nkx_plan_core_hamiltonian(nkx_plan *plan, const nkx_molecule 
         launch_colloc(P, c, s);
         // S (plane 0) and V_n (plane 1)
         core_z_kernel<<<(unsigned)np, 256, 0, s>>>(P.ws_phi, P.d_w, P.d_vj, P.d_pair_batch, c.p0, 0, P.ws_z);
-        vgemm_fp64_kernel<<<dim3(P.nblk, P.nblk, 2), 256, kVSmemBytes, s>>>(
-            P.ws_phi, P.ws_z, 4, 3, P.d_pair_off, P.d_mask, P.mask_words, c.b0, c.b1, c.p0, P.nbf_pad, P.d_V);
+        launch_vgemm_fp64(P, c, P.ws_phi, P.ws_z, 4, 3, 2, P.d_V, s);
         // T (plane 2): the three gradient components into one output
         core_z_kernel<<<(unsigned)np, 256, 0, s>>>(P.ws_phi, P.d_w, P.d_vj, P.d_pair_batch, c.p0, 1, P.ws_z);
         for (int k = 0; k < 3; ++k)
-          vgemm_fp64_kernel<<<dim3(P.nblk, P.nblk, 1), 256, kVSmemBytes, s>>>(
-              P.ws_phi + (size_t)(k + 1) * tile, P.ws_z + (size_t)k * tile, 4, 3, P.d_pair_off, P.d_mask,
-              P.mask_words, c.b0, c.b1, c.p0, P.nbf_pad, P.d_V + 2 * nn);
+          launch_vgemm_fp64(P, c, P.ws_phi + (size_t)(k + 1) * tile, P.ws_z + (size_t)k * tile, 4, 3, 1,
+                            P.d_V + 2 * nn, s);
         NKX_LAUNCH_CHECK();
       }
     } catch (...) {

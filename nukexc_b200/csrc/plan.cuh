@@ -39,7 +39,7 @@ struct BuildGraph {
 };
 
 struct Plan {
-  int device = 0;
+  int device = 0, nsm = 148;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   std::vector<void *> allocs;
@@ -102,6 +102,7 @@ struct Plan {
   size_t cf_cap = 0;
   // accumulators / outputs
   double *d_V = nullptr, *d_E = nullptr, *d_out = nullptr;
+  double *d_vpart = nullptr;  // partial tiles of a split FP64 V contraction (2 nsm tiles)
   // caller-order density outputs (nkx_plan_density)
   long *d_perm = nullptr;
   double *d_dens_out = nullptr;
@@ -111,6 +112,7 @@ struct Plan {
   double metric_svd_thr = 0.0;
   int K = 0, lwork = 0;
   double *d_L = nullptr, *d_X = nullptr, *d_t = nullptr, *d_y = nullptr, *d_c = nullptr, *d_work = nullptr;
+  double *d_ypart = nullptr;  // per-slice shares of y
   int *d_info = nullptr, *d_piv = nullptr;
   std::vector<int> h_piv;
   double metric_min_diag = 0.0;

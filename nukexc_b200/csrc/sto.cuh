@@ -254,19 +254,26 @@ __device__ __forceinline__ void sto_value_grad_hess_cached(const StoFunc &f, dou
 }
 
 // radial factors of every shell of the block at one point, shared by the
-// warp: R[s] = r^k e^(-zeta r) and, with GRAD, C[s] = (k/r - zeta)/r (0 at r = 0),
-// from 1/r = rsqrt(r^2) (1 ulp) and exp_neg
-template <bool GRAD>
+// warp: R[s] = r^k e^(-zeta r) and, with GRAD, C[s] = (k/r - zeta)/r (0 at r = 0).
+// FAST (the mixed-precision collocation): from 1/r = rsqrt(r^2) (1 ulp) and
+// exp_neg; else sqrt, exp and the divisions of sto_value_grad
+template <bool GRAD, bool FAST = true>
 __device__ __forceinline__ void block_radials(const BlockFuncs &B, int lane, double x, double y, double z,
                                               double *__restrict__ R, double *__restrict__ C) {
   for (int s = lane; s < B.nshell; s += 32) {
     const double dx = x - B.scx[s], dy = y - B.scy[s], dz = z - B.scz[s];
     const double r2 = dx * dx + dy * dy + dz * dz;
-    const double ri = r2 > 0.0 ? rsqrt(r2) : 0.0;
-    const double r = r2 * ri;
     const int k = B.sk[s];
-    R[s] = ipow(r, k) * exp_neg(-B.szeta[s] * r);
-    if (GRAD) C[s] = (k * ri - B.szeta[s]) * ri;
+    if constexpr (FAST) {
+      const double ri = r2 > 0.0 ? rsqrt(r2) : 0.0;
+      const double r = r2 * ri;
+      R[s] = ipow(r, k) * exp_neg(-B.szeta[s] * r);
+      if (GRAD) C[s] = (k * ri - B.szeta[s]) * ri;
+    } else {
+      const double r = sqrt(r2);
+      R[s] = ipow(r, k) * exp(-B.szeta[s] * r);
+      if (GRAD) C[s] = r > 0.0 ? (k / r - B.szeta[s]) / r : 0.0;
+    }
   }
 }
 
