@@ -720,7 +720,9 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const Aux
     }
   }
   }
-  __shared__ double red[32];
+  // every sum over its warp first, then all of them over the warps behind
+  // one barrier (two barriers a sum took most of a short slice's time)
+  __shared__ double red[8][QM * NM];
 #pragma unroll
   for (int q = 0; q < QM; ++q) {
     if (q >= G.n) break;
@@ -728,15 +730,14 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const Aux
     for (int m = 0; m < NM; ++m) {
       double s = acc[q][m];
       for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      __syncthreads();
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) y[(size_t)blockIdx.y * naux + shells[G.first + q].first + m] = s;
-      }
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q * NM + m] = s;
     }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < G.n * NM; e += blockDim.x) {
+    double s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][e];
+    y[(size_t)blockIdx.y * naux + shells[G.first + e / NM].first + e % NM] = s;
   }
 }
 
