@@ -1725,23 +1725,12 @@ static void launch_density_nn(Plan &P, const Chunk &c, int nn, int nspin, int no
 }
 
 // The FP64 V contraction of one chunk: nz planes of zT (stride z_stride
-// tiles) against PhiT into V.  Batches are split over as few CTAs per tile
-// as fill at least nine tenths of the last wave (a basis of one block and
-// one plane: one CTA per SM instead of one in all).
+// tiles) against PhiT into V.
 static void launch_vgemm_fp64(Plan &P, const Chunk &c, const double *phiT, const double *zT, int phi_stride,
                               int z_stride, int nz, double *V, cudaStream_t s) {
-  const long parts = (long)nz * P.nblk * P.nblk, nsm = P.nsm;
-  int nsplit = 1;
-  double best = 0.0;
-  for (long k = 1; k == 1 || (k <= c.b1 - c.b0 && parts * k <= 2 * nsm); ++k) {
-    const double fill = (double)(parts * k) / (double)((parts * k + nsm - 1) / nsm * nsm);
-    if (fill > best + 1e-9) {
-      best = fill;
-      nsplit = (int)k;
-    }
-    if (best >= 0.9) break;
-  }
-  if (nsplit > 1 && !P.d_vpart) P.d_vpart = P.alloc<double>((size_t)2 * nsm * kBlockF * kBlockF);
+  const long parts = (long)nz * P.nblk * P.nblk;
+  const int nsplit = batch_split(parts, c.b1 - c.b0, P.nsm);
+  if (nsplit > 1 && !P.d_vpart) P.d_vpart = P.alloc<double>((size_t)4 * P.nsm * kBlockF * kBlockF);
   NKX_CUDA(cudaFuncSetAttribute(vgemm_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVSmemBytes));
   vgemm_fp64_kernel<<<dim3(P.nblk, P.nblk, nz * nsplit), 256, kVSmemBytes, s>>>(
       phiT, zT, phi_stride, z_stride, P.d_pair_off, P.d_mask, P.mask_words, c.b0, c.b1, c.p0, nsplit, P.nbf_pad, V,

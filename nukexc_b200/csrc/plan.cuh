@@ -102,7 +102,7 @@ struct Plan {
   size_t cf_cap = 0;
   // accumulators / outputs
   double *d_V = nullptr, *d_E = nullptr, *d_out = nullptr;
-  double *d_vpart = nullptr;  // partial tiles of a split FP64 V contraction (2 nsm tiles)
+  double *d_vpart = nullptr;  // partial tiles of a split FP64 V contraction (4 nsm tiles)
   // caller-order density outputs (nkx_plan_density)
   long *d_perm = nullptr;
   double *d_dens_out = nullptr;
@@ -209,6 +209,24 @@ __global__ void functional_kernel(XcSpec s, bool gga, int nspin, long npad, long
 inline int density_width(const Plan &P, int nocc) {
   if (P.tune.dens_n) return P.tune.dens_n;
   return ((nocc + 127) / 128) * 128 >= 1024 ? 128 : 64;
+}
+// Units a V output tile's batches are dealt to: the fewest that fill nine
+// tenths of the last wave of `nsm` CTAs, up to four waves (else the best
+// found).  `parts` tiles alone leave SMs idle where a basis has few blocks
+// (one water: 1 tile) or spill into a nearly empty wave ((H2O)_8 with a J
+// plane: 18 tiles in 9 shares each took two waves for 162 units, 8 take one).
+inline int batch_split(long parts, long nbatch, int nsm) {
+  int nsplit = 1;
+  double best = 0.0;
+  for (long k = 1; parts > 0 && (k == 1 || (k <= nbatch && parts * k <= 4L * nsm)); ++k) {
+    const double fill = (double)(parts * k) / (double)((parts * k + nsm - 1) / nsm * nsm);
+    if (fill > best + 1e-9) {
+      best = fill;
+      nsplit = (int)k;
+    }
+    if (best >= 0.9) break;
+  }
+  return nsplit;
 }
 void mixed_gradient_begin(Plan &P, int nspin, int nocc, cudaStream_t s);
 const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc, double *edens, cudaStream_t s,

@@ -2148,8 +2148,7 @@ void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool 
     a.nt = P.tune.v_n;
     a.ew = a.nt == 128 ? P.tune.v_warps : 8;
     const long parts = tiles * (kBlockF / a.nt);
-    a.nsplit = (parts == 0 || parts >= M.nsm) ? 1 : (int)std::min<long>({(M.nsm + parts - 1) / parts, c.b1 - c.b0, 16L});
-    a.nsplit = std::max(1, a.nsplit);
+    a.nsplit = batch_split(parts, c.b1 - c.b0, M.nsm);
     a.nunits = parts * a.nsplit;
     launch_i8(M, M.m_ph, a.nt == 128 ? M.m_z : M.m_z64, a, s);
     ++P.launches;
