@@ -1,0 +1,35 @@
+// FP64 tensor-core fragments and the asynchronous copies that feed them.
+#pragma once
+
+#include <cstdint>
+
+#include <cuda_runtime.h>
+
+namespace nkx {
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+// the same, or 16 zero bytes when !in (src is then not read)
+__device__ __forceinline__ void cp_async16_fill(void *dst, const void *src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// D += A B on the FP64 tensor path: A 8 x 4 (thread t holds row t / 4,
+// column t % 4), B 4 x 8 (row t % 4, column t / 4), D 8 x 8 (row t / 4,
+// columns 2 (t % 4) and + 1)
+__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+}  // namespace nkx

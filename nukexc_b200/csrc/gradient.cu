@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "dmma.cuh"
 #include "nkx.h"
 #include "plan.cuh"
 #include "sto.cuh"
@@ -35,255 +36,238 @@ nkx_status run_guarded(const char *where, const std::function<void()> &fn);
 
 static inline unsigned gblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// T[(bl, spin, comp)][i][g] = sum_f Phi_comp(g, f) C(i, f) over the batch's
-// significant blocks: one 64-point x 64-orbital tile per thread block,
-// thread (ty, tx) owning points ty + 16a and orbitals tx + 16j.
-template <bool GRAD>
-__global__ void __launch_bounds__(256) orbital_values_kernel(const double *__restrict__ phiT,
-                                                             const double *__restrict__ Ct, int nocc, int nocc_pad,
-                                                             int nbf_pad, const int *__restrict__ pair_off,
-                                                             const int *__restrict__ pair_blk, long sb0, long p0,
-                                                             int nspin, double *__restrict__ T) {
-  constexpr int NC = GRAD ? 4 : 1;
-  constexpr int KS = 16;
-  __shared__ double Ps[NC][KS][64 + 1];
-  __shared__ double Cs[KS][64 + 1];
-  const int spin = blockIdx.y;
-  const long bl = blockIdx.x / 4, b = sb0 + bl;
-  const int g0 = (blockIdx.x % 4) * 64, i0 = blockIdx.z * 64;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const double *C = Ct + (size_t)spin * nocc * nbf_pad;
-  const size_t tile = (size_t)kBatch * kBlockF;
-  double acc[NC][4][4];
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[c][a][j] = 0.0;
-  for (int q = pair_off[b]; q < pair_off[b + 1]; ++q) {
-    const int I = pair_blk[q];
-    const double *P = phiT + (size_t)(q - p0) * NC * tile;
-    for (int f0 = 0; f0 < kBlockF; f0 += KS) {
-      for (int e = threadIdx.x; e < NC * 64 * KS; e += 256) {
-        const int c = e / (64 * KS), r = (e / KS) % 64, k = e % KS;
-        Ps[c][k][r] = P[c * tile + (size_t)(g0 + r) * kBlockF + f0 + k];
-      }
-      for (int e = threadIdx.x; e < 64 * KS; e += 256) {
-        const int r = e / KS, k = e % KS, i = i0 + r;
-        Cs[k][r] = i < nocc ? C[(size_t)i * nbf_pad + I * kBlockF + f0 + k] : 0.0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < KS; ++k) {
-        double bv[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = Cs[k][tx + 16 * j];
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            const double av = Ps[c][k][ty + 16 * a];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[c][a][j] += av * bv[j];
-          }
-      }
-      __syncthreads();
-    }
-  }
-  double *Tb = T + ((size_t)(bl * nspin + spin) * NC) * nocc_pad * kBatch;
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        Tb[((size_t)c * nocc_pad + i0 + tx + 16 * j) * kBatch + g0 + ty + 16 * a] = acc[c][a][j];
+// (C occ)[spin][i][f], the B operand of x_fp64_kernel
+__global__ void scale_orbitals_kernel(const double *__restrict__ Ct, const double *__restrict__ occ, int nbf_pad,
+                                      long n, double *__restrict__ out) {
+  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (e < n) out[e] = Ct[e] * occ[e / nbf_pad];
 }
 
-// Basis-centre and point-motion terms of one (batch, block) pair.  Thread
-// (ty, tx) owns functions 4 ty .. 4 ty + 3 of the block and, per 16-point
-// subtile, points 2 tx, 2 tx + 1.  X and grad X come from a small FP64 GEMM
-// of C (block rows) with occ * T staged in shared memory, or (XIN) are read
-// from X[pair][spin][comp][g][mu] made by the tensor cores.  Contributions
-// are summed per owner atom (points) and per function atom in shared memory
-// and leave the block as a few global atomics.
-template <bool GRAD, bool XIN = false>
-__global__ void __launch_bounds__(256) grad_pair_kernel(
-    const StoFunc *__restrict__ sto, const int *__restrict__ fatom, const double *__restrict__ px,
+// X_c(g, mu) = sum_i T_c(g, i) occ_i C(mu, i) in FP64, one 128-point x
+// 128-function tile of one (pair, spin, component) per CTA: eight warps of
+// 64 x 32 on DMMA tiles, the i rows of T (256 points) and of C occ (128
+// functions) streamed by 16-byte cp.async, 16 orbitals a step (rows past
+// nocc filled with zeros).  Bound: FP64 pipe.
+constexpr int kXKs = 16, kXStages = 3, kXLd = kBlockF + 4;
+constexpr int kXSmem = kXStages * 2 * kXKs * kXLd * 8;
+__global__ void __launch_bounds__(256, 1)
+    x_fp64_kernel(const double *__restrict__ T, const double *__restrict__ Cocc, int nocc, int nocc_pad, int nbf_pad,
+                  int nspin, int nc, const int *__restrict__ pair_batch, const int *__restrict__ pair_blk, long pstart,
+                  long sb0, double *__restrict__ X) {
+  extern __shared__ __align__(16) double xsm[];  // [stage][A | B][kXKs][kXLd]
+  const long q = blockIdx.x / 2;
+  const int half = blockIdx.x % 2, sc = blockIdx.y, s = sc / nc;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *A = T + ((size_t)(pair_batch[pstart + q] - sb0) * nspin * nc + sc) * nocc_pad * kBatch + 128 * half;
+  const double *Bp = Cocc + (size_t)s * nocc * nbf_pad + (size_t)pair_blk[pstart + q] * kBlockF;
+  const int total = (nocc + kXKs - 1) / kXKs;
+  auto issue = [&](int t, int st) {
+    if (t < total) {
+      double *dA = xsm + st * 2 * kXKs * kXLd, *dB = dA + kXKs * kXLd;
+#pragma unroll
+      for (int r = 0; r < (kXKs * kBlockF / 2) / 256; ++r) {
+        const int e = threadIdx.x + 256 * r, k = e / 64, part = 2 * (e % 64), i = t * kXKs + k;
+        const bool in = i < nocc;
+        cp_async16_fill(dA + k * kXLd + part, A + (size_t)(in ? i : 0) * kBatch + part, in);
+        cp_async16_fill(dB + k * kXLd + part, Bp + (size_t)(in ? i : 0) * nbf_pad + part, in);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int st = 0; st < kXStages - 1; ++st) issue(st, st);
+  double acc[8][4][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int fr = lane >> 2, fk = lane & 3, r0 = 64 * (warp & 1) + fr, c0 = 32 * (warp >> 1) + fr;
+  for (int t = 0; t < total; ++t) {
+    cp_async_wait<kXStages - 2>();
+    __syncthreads();  // step t is visible; the stage refilled below was read in step t - 1
+    issue(t + kXStages - 1, (t + kXStages - 1) % kXStages);
+    const double *As = xsm + (t % kXStages) * 2 * kXKs * kXLd, *Bs = As + kXKs * kXLd;
+#pragma unroll
+    for (int k = 0; k < kXKs; k += 4) {
+      double av[8], bv[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) av[i] = As[(k + fk) * kXLd + r0 + 8 * i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bv[j] = Bs[(k + fk) * kXLd + c0 + 8 * j];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma884(acc[i][j], av[i], bv[j]);
+    }
+  }
+  cp_async_wait<0>();
+  double *o = X + ((size_t)q * nspin * nc + sc) * kBatch * kBlockF + (size_t)(128 * half + r0) * kBlockF +
+              32 * (warp >> 1) + 2 * fk;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<double2 *>(o + (size_t)8 * i * kBlockF + 8 * j) = make_double2(acc[i][j][0], acc[i][j][1]);
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Basis-centre and point-motion terms of one (batch, block) pair and spin,
+// from X[pair][spin][comp][g][mu].  Lane l of a warp takes functions 4l .. 4l + 3,
+// whose slots share a solid harmonic over the warp (the plan order), and a
+// warp 32 of the batch's points, in the order of their owner atoms: the
+// point-motion sum of a run of points with one owner stays in registers and
+// is reduced over the warp when the owner changes.  Per point the warp forms
+// each shell's radial factor R, R'/(r R) = C and D = ((R'' / R) - C) / r^2
+// once; with S the harmonic, A = 4 c0 X + 2 c . grad X and B = 2 X,
+//   t = R [(C S A + B (D S d.c + C c.grad S)) d + (A + B C d.c) grad S
+//          + B C S c + B (hess S) c],   d = r - centre,
+// which needs no second derivative of phi itself.  FAST (the mixed-precision
+// gradient) takes e^x from exp_neg.
+//
+// Bound: FP64 issue.  (H2O)_8 PBE: 17.4 ms per gradient with each thread
+// evaluating its functions' radial factors and all six second derivatives,
+// 2.63 ms now (X alone is 6.2 GB of HBM reads, 1 ms).
+template <bool GRAD, bool FAST>
+__global__ void __launch_bounds__(256, 2) grad_pair_kernel(
+    const StoFunc *__restrict__ sto, const int *__restrict__ fshell, const StoShell *__restrict__ bshell,
+    const int *__restrict__ bnshell, const int *__restrict__ fatom, const double *__restrict__ px,
     const double *__restrict__ py, const double *__restrict__ pz, const int *__restrict__ owner,
-    const int *__restrict__ pair_batch, const int *__restrict__ pair_blk, long pstart, long sb0,
-    const double *__restrict__ Ct, const double *__restrict__ occ, int nocc, int nocc_pad, int nbf_pad, int nspin,
-    const double *__restrict__ T, const double *__restrict__ coef, long npad, double *__restrict__ F,
-    const double *__restrict__ Xin = nullptr) {
+    const int *__restrict__ pair_batch, const int *__restrict__ pair_blk, long pstart, int nspin,
+    int spin, const double *__restrict__ coef, long npad, const double *__restrict__ Xin, double *__restrict__ F) {
   constexpr int NC = GRAD ? 4 : 1;
-  __shared__ double Cs[16][kBlockF];
-  __shared__ double Ts[16][NC][16];
-  __shared__ StoFunc sfn[kBlockF];
-  __shared__ int s_owner[kBatch], rep_pt[kBatch], s_fatom[kBlockF], rep_f[kBlockF];
-  __shared__ double tp[kBatch][3], tfs[kBlockF][3];
+  __shared__ BlockFuncs B;
+  __shared__ double rad[8][3][128];  // R, C, D per warp; at the end the warps' function sums
+  __shared__ int s_owner[kBatch], s_fatom[kBlockF], rep_f[kBlockF];
+  __shared__ short order[kBatch];
+  __shared__ double tfs[kBlockF][3];
   const long p = pstart + blockIdx.x;
   const int b = pair_batch[p], I = pair_blk[p];
-  const long bl = b - sb0;
-  const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  load_block_funcs(B, sto, fshell, bshell, bnshell, I, tid, 256);
+  s_owner[tid] = owner[(long)b * kBatch + tid];
+  if (tid < kBlockF) s_fatom[tid] = fatom[I * kBlockF + tid];
+  __syncthreads();
   {
-    const int g = tid;
-    s_owner[g] = owner[(long)b * kBatch + g];
-    tp[g][0] = tp[g][1] = tp[g][2] = 0.0;
+    const int own = s_owner[tid];
+    int rank = 0;
+    for (int h = 0; h < kBatch; ++h) rank += s_owner[h] < own || (s_owner[h] == own && h < tid);
+    order[rank] = (short)tid;
     if (tid < kBlockF) {
-      s_fatom[tid] = fatom[I * kBlockF + tid];
-      sfn[tid] = sto[I * kBlockF + tid];
+      int rf = 0;
+      while (s_fatom[rf] != s_fatom[tid]) ++rf;
+      rep_f[tid] = rf;
       tfs[tid][0] = tfs[tid][1] = tfs[tid][2] = 0.0;
     }
   }
   __syncthreads();
-  {
-    const int g = tid;
-    int r = g;
-    for (int h = 0; h < g; ++h)
-      if (s_owner[h] == s_owner[g]) {
-        r = h;
-        break;
-      }
-    rep_pt[g] = r;
-    if (tid < kBlockF) {
-      int rf = tid;
-      for (int h = 0; h < tid; ++h)
-        if (s_fatom[h] == s_fatom[tid]) {
-          rf = h;
-          break;
-        }
-      rep_f[tid] = rf;
-    }
-  }
-  __syncthreads();
-  double tf[4][3];
+  double *wR = rad[warp][0], *wC = rad[warp][1], *wD = rad[warp][2];
+  double tf[4][3], tq[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-  for (int a = 0; a < 4; ++a) tf[a][0] = tf[a][1] = tf[a][2] = 0.0;
-  for (int s = 0; s < nspin; ++s) {
-    const double *C = Ct + (size_t)s * nocc * nbf_pad;
-    const double *oc = occ + (size_t)s * nocc;
-    const double *Tb = T + ((size_t)(bl * nspin + s) * NC) * nocc_pad * kBatch;
-    const double *cs = coef + (size_t)s * 4 * npad;
-    for (int st = 0; st < kBatch / 16; ++st) {
-      double acc[4][2][NC];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int c = 0; c < NC; ++c) acc[a][q][c] = 0.0;
-      if (XIN) {
-        const double *Xs = Xin + ((size_t)blockIdx.x * nspin + s) * NC * kBatch * kBlockF;
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            const double2 *xp =
-                reinterpret_cast<const double2 *>(Xs + ((size_t)c * kBatch + st * 16 + 2 * tx + q) * kBlockF + 4 * ty);
-            const double2 u = xp[0], v = xp[1];
-            acc[0][q][c] = u.x;
-            acc[1][q][c] = u.y;
-            acc[2][q][c] = v.x;
-            acc[3][q][c] = v.y;
-          }
-      }
-      for (int i0 = 0; !XIN && i0 < nocc; i0 += 16) {
-        for (int e = tid; e < 16 * kBlockF; e += 256) {
-          const int k = e >> 7, m = e & 127, i = i0 + k;
-          Cs[k][m] = i < nocc ? C[(size_t)i * nbf_pad + I * kBlockF + m] : 0.0;
-        }
-        for (int e = tid; e < 16 * NC * 16; e += 256) {
-          const int k = e / (NC * 16), c = (e / 16) % NC, gl = e & 15, i = i0 + k;
-          Ts[k][c][gl] = i < nocc ? oc[i] * Tb[((size_t)c * nocc_pad + i) * kBatch + st * 16 + gl] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int k = 0; k < 16; ++k) {
-          double cv[4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) cv[a] = Cs[k][4 * ty + a];
-#pragma unroll
-          for (int q = 0; q < 2; ++q)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-              const double tv = Ts[k][c][2 * tx + q];
-#pragma unroll
-              for (int a = 0; a < 4; ++a) acc[a][q][c] += cv[a] * tv;
-            }
-        }
-        __syncthreads();
-      }
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int g = st * 16 + 2 * tx + q;
-        const long gg = (long)b * kBatch + g;
-        const double x = px[gg], y = py[gg], z = pz[gg];
-        const double c0 = cs[gg];
-        double ck[3] = {0.0, 0.0, 0.0};
-        if (GRAD) {
-          ck[0] = cs[npad + gg];
-          ck[1] = cs[2 * npad + gg];
-          ck[2] = cs[3 * npad + gg];
-        }
-        double tq[3] = {0.0, 0.0, 0.0};
-        HessRadialCache rc;  // the thread's four functions at this point
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const StoFunc &fn = sfn[4 * ty + a];
-          const double X = acc[a][q][0];
-          double t[3];
-          if (GRAD) {
-            double v, gr[3], h[6];
-            // the mixed gradient (XIN) takes e^x from exp_neg
-            sto_value_grad_hess_cached<XIN>(fn, x, y, z, rc, v, gr, h);
-            const double H[3][3] = {{h[0], h[1], h[2]}, {h[1], h[3], h[4]}, {h[2], h[4], h[5]}};
-            const double dX[3] = {acc[a][q][NC > 1 ? 1 : 0], acc[a][q][NC > 2 ? 2 : 0], acc[a][q][NC > 3 ? 3 : 0]};
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              double u = 0.0;
-#pragma unroll
-              for (int k = 0; k < 3; ++k) u += ck[k] * (H[j][k] * X + gr[j] * dX[k]);
-              t[j] = 4.0 * c0 * gr[j] * X + 2.0 * u;
-            }
-          } else {
-            double v, gr[3];
-            sto_value_grad(fn, x, y, z, v, gr[0], gr[1], gr[2]);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) t[j] = 4.0 * c0 * gr[j] * X;
-          }
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            tf[a][j] += t[j];
-            tq[j] += t[j];
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) atomicAdd(&tp[rep_pt[g]][j], tq[j]);
-      }
-    }
-  }
-  // the eight tx lanes of a ty hold the same functions: reduce, then one add
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int c = 0; c < 4; ++c) tf[c][0] = tf[c][1] = tf[c][2] = 0.0;
+  int cur = s_owner[order[32 * warp]];
+  auto flush = [&]() {
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      double v = tf[a][j];
-      v += __shfl_xor_sync(0xffffffffu, v, 1);
-      v += __shfl_xor_sync(0xffffffffu, v, 2);
-      v += __shfl_xor_sync(0xffffffffu, v, 4);
-      if (tx == 0) atomicAdd(&tfs[rep_f[4 * ty + a]][j], v);
+      const double v = warp_sum(tq[j]);
+      if (lane == 0 && v != 0.0) atomicAdd(&F[3 * cur + j], v);
+      tq[j] = 0.0;
     }
-  __syncthreads();
-  {
-    const int g = tid;
-    if (rep_pt[g] == g)
-      for (int j = 0; j < 3; ++j)
-        if (tp[g][j] != 0.0) atomicAdd(&F[3 * s_owner[g] + j], tp[g][j]);
-    if (tid < kBlockF && rep_f[tid] == tid)
-      for (int j = 0; j < 3; ++j)
-        if (tfs[tid][j] != 0.0) atomicAdd(&F[3 * s_fatom[tid] + j], -tfs[tid][j]);
+  };
+  for (int k = 0; k < 32; ++k) {
+    const int g = order[32 * warp + k];
+    if (s_owner[g] != cur) {
+      flush();
+      cur = s_owner[g];
+    }
+    const long gg = (long)b * kBatch + g;
+    const double x = px[gg], y = py[gg], z = pz[gg];
+    double X[4][NC], cf[4] = {0.0, 0.0, 0.0, 0.0};
+    const double *Xs = Xin + (((size_t)blockIdx.x * nspin + spin) * NC * kBatch + g) * kBlockF + 4 * lane;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double2 *xp = reinterpret_cast<const double2 *>(Xs + (size_t)c * kBatch * kBlockF);
+      const double2 u = xp[0], v = xp[1];
+      X[0][c] = u.x;
+      X[1][c] = u.y;
+      X[2][c] = v.x;
+      X[3][c] = v.y;
+      cf[c] = coef[((size_t)spin * 4 + c) * npad + gg];
+    }
+    __syncwarp();
+    for (int s = lane; s < B.nshell; s += 32) {
+      const double dx = x - B.scx[s], dy = y - B.scy[s], dz = z - B.scz[s];
+      const double r2 = dx * dx + dy * dy + dz * dz, r = sqrt(r2), zeta = B.szeta[s];
+      const int kk = B.sk[s];
+      wR[s] = ipow(r, kk) * (FAST ? exp_neg(-zeta * r) : exp(-zeta * r));
+      double C = 0.0, D = 0.0;
+      if (r > 0.0) {
+        const double ir = 1.0 / r, a = kk * ir - zeta;
+        C = a * ir;
+        D = ((a * a - kk * ir * ir) - C) * (ir * ir);
+      }
+      wC[s] = C;
+      wD[s] = D;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int sh = B.sh[c][lane], l = B.l[c][lane], m = B.m[c][lane];
+      const double d[3] = {x - B.scx[sh], y - B.scy[sh], z - B.scz[sh]};
+      const double R = B.norm[c][lane] * wR[sh], C = wC[sh];
+      double S, gS[3];
+      solid_harmonic_grad(l, m, d[0], d[1], d[2], S, gS[0], gS[1], gS[2]);
+      double t[3];
+      if constexpr (GRAD) {
+        const double Bx = 2.0 * X[c][0];
+        const double A = 4.0 * cf[0] * X[c][0] + 2.0 * (cf[1] * X[c][1] + cf[2] * X[c][2] + cf[3] * X[c][3]);
+        const double dc = d[0] * cf[1] + d[1] * cf[2] + d[2] * cf[3];
+        const double gc = gS[0] * cf[1] + gS[1] * cf[2] + gS[2] * cf[3];
+        const double CS = C * S;
+        const double pd = CS * A + Bx * (wD[sh] * S * dc + C * gc), pg = A + Bx * C * dc, pc = Bx * CS;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) t[j] = pd * d[j] + pg * gS[j] + pc * cf[1 + j];
+        if (l >= 2) {
+          double h[6];
+          solid_harmonic_hess(l, m, d[0], d[1], d[2], h[0], h[1], h[2], h[3], h[4], h[5]);
+          t[0] += Bx * (h[0] * cf[1] + h[1] * cf[2] + h[2] * cf[3]);
+          t[1] += Bx * (h[1] * cf[1] + h[3] * cf[2] + h[4] * cf[3]);
+          t[2] += Bx * (h[2] * cf[1] + h[4] * cf[2] + h[5] * cf[3]);
+        }
+      } else {
+        const double A = 4.0 * cf[0] * X[c][0];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) t[j] = A * (gS[j] + C * S * d[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        tf[c][j] = fma(R, t[j], tf[c][j]);
+        tq[j] = fma(R, t[j], tq[j]);
+      }
+    }
   }
+  flush();
+  __syncthreads();  // every warp is past its radial factors
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) rad[warp][j][4 * lane + c] = tf[c][j];
+  __syncthreads();
+  for (int e = tid; e < 3 * kBlockF; e += 256) {
+    const int j = e / kBlockF, f = e % kBlockF;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += rad[w][j][f];
+    atomicAdd(&tfs[rep_f[f]][j], v);
+  }
+  __syncthreads();
+  if (tid < kBlockF && rep_f[tid] == tid)
+    for (int j = 0; j < 3; ++j)
+      if (tfs[tid][j] != 0.0) atomicAdd(&F[3 * s_fatom[tid] + j], -tfs[tid][j]);
 }
 
 // Becke-weight term: for point g with owner o, Q = P_o / Z, Z = sum_i P_i,
@@ -502,87 +486,274 @@ __global__ void becke_grad_kernel(const double *__restrict__ C, int natoms, cons
   }
 }
 
-struct GradState {
-  double *T = nullptr, *edens = nullptr, *F = nullptr;
-  long cap_batches = 0;
-  int nocc_pad = 0, nspin = 0;
-  std::vector<void *> bufs;
-  ~GradState() {
-    for (void *p : bufs) cudaFree(p);
+// The Becke-weight term of molecules of up to kGradCap atoms, one warp per 32
+// points, with the screening of becke_grad_kernel: atoms with
+// r < r_min + 2 Rc of any of the points are candidates.
+// The candidates are listed once; shared memory holds per candidate and point the distance, the cell function
+// P and the weight D.  With a_ij = f a kappa_i s'(mu_ij) / (s(mu_ij) R_ij) the
+// terms of all pairs collapse to
+//   F_k += -D_k u_k,  F_o += sum_k D_k u_k,   D_k = sum_j a_kj - sum_i a_ik,
+//   F_i -= G_ij e_ij, F_j += G_ij e_ij,       G_ij = sum_points a_ij mu_ij
+// (e_ij terms only where |R_i - R_j| is below the clamp), so a pair costs one
+// scalar per point, and one warp reduction when it is not clamped; vectors
+// appear once per atom.  Each warp strides over the points and adds its sums
+// to F once.
+//
+// Bound: FP64 issue.  (H2O)_8: 7.2 ms per gradient with a thread per point
+// (vector atomics in shared memory per pair), 1.91 ms now.
+constexpr int kGradCap = 64;
+__global__ void __launch_bounds__(32)
+    becke_grad_warp_kernel(const double *__restrict__ C, int natoms, const double *__restrict__ px,
+                           const double *__restrict__ py, const double *__restrict__ pz, const double *__restrict__ w,
+                           const int *__restrict__ owner, const double *__restrict__ edens, long npad, double clamp,
+                           double *__restrict__ F) {
+  extern __shared__ double gsm[];  // r, P, D [natoms][32], F [3 natoms], list [natoms]
+  double *rs = gsm, *Ps = rs + natoms * 32, *Ds = Ps + natoms * 32, *Fa = Ds + natoms * 32;
+  int *list = reinterpret_cast<int *>(Fa + 3 * natoms);
+  const int lane = threadIdx.x;
+  for (int e = lane; e < 3 * natoms; e += 32) Fa[e] = 0.0;
+  __syncwarp();
+  const double Rc = clamp > 0.0 ? clamp : 1e300;
+  for (long g0 = blockIdx.x * 32L; g0 < npad; g0 += gridDim.x * 32L) {  // npad is a multiple of 256
+    const long g = g0 + lane;
+    const double r[3] = {px[g], py[g], pz[g]};
+    const double wg = w[g], eg = edens[g];
+    const int o = owner[g];
+    auto dist = [&](int a) {
+      const double dx = r[0] - C[3 * a], dy = r[1] - C[3 * a + 1], dz = r[2] - C[3 * a + 2];
+      return sqrt(dx * dx + dy * dy + dz * dz);
+    };
+    double r2min = 1e300;
+    for (int a = 0; a < natoms; ++a) {
+      const double dx = r[0] - C[3 * a], dy = r[1] - C[3 * a + 1], dz = r[2] - C[3 * a + 2];
+      r2min = fmin(r2min, dx * dx + dy * dy + dz * dz);
+    }
+    const double rmin = sqrt(r2min), lim = rmin + 2.0 * Rc;
+    const bool live = wg != 0.0 && eg != 0.0 && dist(o) < rmin + Rc;  // else no term, or P_o == 0
+    if (!__any_sync(0xffffffffu, live)) continue;
+    int nl = 0;
+    for (int a = 0; a < natoms; ++a) {
+      const double ra = dist(a);
+      if (!__any_sync(0xffffffffu, live && ra < lim)) continue;
+      rs[nl * 32 + lane] = ra;
+      Ds[nl * 32 + lane] = 0.0;
+      if (lane == 0) list[nl] = a;
+      ++nl;
+    }
+    __syncwarp();
+    // |R_i - R_j| of candidates a and c0 + lane (inverse of the clamped one)
+    auto inverse = [&](int i, int c, double &dij) {
+      dij = 0.0;
+      if (c >= nl || list[c] == i) return 0.0;
+      const int j = list[c];
+      const double dx = C[3 * i] - C[3 * j], dy = C[3 * i + 1] - C[3 * j + 1], dz = C[3 * i + 2] - C[3 * j + 2];
+      dij = sqrt(dx * dx + dy * dy + dz * dz);
+      return 1.0 / fmin(dij, Rc);
+    };
+    double Z = 0.0, Po = 0.0;
+    for (int a = 0; a < nl; ++a) {
+      const double ri = rs[a * 32 + lane];
+      const bool cell = live && ri < rmin + Rc;  // else P_i = 0 exactly
+      double P = cell ? 1.0 : 0.0;
+      const int i = list[a];
+      if (__any_sync(0xffffffffu, cell)) {
+        const double reach = cell ? ri + Rc : -1.0;
+        for (int c0 = 0; c0 < nl; c0 += 32) {
+          double dij;
+          const double iR = inverse(i, c0 + lane, dij);
+          const int n = min(32, nl - c0);
+          for (int t = 0; t < n; ++t) {
+            const double rj = rs[(c0 + t) * 32 + lane];
+            if (!__any_sync(0xffffffffu, rj < reach) || c0 + t == a) continue;
+            double mu = (ri - rj) * __shfl_sync(0xffffffffu, iR, t), sv, dsv;
+            mu = mu > 1.0 ? 1.0 : (mu < -1.0 ? -1.0 : mu);
+            becke_s_ds(mu, sv, dsv);
+            P *= sv;
+          }
+        }
+      }
+      Ps[a * 32 + lane] = P;
+      Z += P;
+      if (i == o) Po = P;
+    }
+    const bool on = live && Po > 0.0 && Z > 0.0;
+    const double Q = on ? Po / Z : 0.0, fa = on ? eg * (wg / Q) : 0.0, iZ = on ? 1.0 / Z : 0.0;
+    for (int a = 0; a < nl; ++a) {
+      const double ri = rs[a * 32 + lane];
+      const int i = list[a];
+      const double kappa = Q * ((i == o ? 1.0 : 0.0) - Ps[a * 32 + lane] * iZ);
+      const bool cell = on && kappa != 0.0 && ri > 0.0;
+      if (!__any_sync(0xffffffffu, cell)) continue;
+      const double reach = cell ? ri + Rc : -1.0, fk = cell ? fa * kappa : 0.0;
+      double A = 0.0;
+      for (int c0 = 0; c0 < nl; c0 += 32) {
+        double dij;
+        const double iR = inverse(i, c0 + lane, dij);
+        const int n = min(32, nl - c0);
+        for (int t = 0; t < n; ++t) {
+          const double rj = rs[(c0 + t) * 32 + lane];
+          if (!__any_sync(0xffffffffu, rj < reach) || c0 + t == a) continue;
+          const double iRt = __shfl_sync(0xffffffffu, iR, t), dt = __shfl_sync(0xffffffffu, dij, t);
+          const double mu = (ri - rj) * iRt;
+          double sv, ds, lam = 0.0;
+          becke_s_ds(mu, sv, ds);
+          if (rj > 0.0 && mu > -1.0 && mu < 1.0 && sv > 0.0) lam = fk * ds / sv * iRt;
+          A += lam;
+          Ds[(c0 + t) * 32 + lane] -= lam;
+          if (dt < Rc) {
+            const double G = warp_sum(lam * mu);
+            if (lane < 3 && G != 0.0) {
+              const int j = list[c0 + t];
+              const double e = G * (C[3 * i + lane] - C[3 * j + lane]) / dt;
+              atomicAdd(&Fa[3 * i + lane], -e);
+              atomicAdd(&Fa[3 * j + lane], e);
+            }
+          }
+        }
+      }
+      Ds[a * 32 + lane] += A;
+    }
+    // the u terms: per atom over the points, and per point to its owner
+    double Fo[3] = {0.0, 0.0, 0.0};
+    for (int a = 0; a < nl; ++a) {
+      const double ra = rs[a * 32 + lane], D = Ds[a * 32 + lane];
+      const double h = ra > 0.0 ? D / ra : 0.0;
+      if (!__any_sync(0xffffffffu, h != 0.0)) continue;
+      const int i = list[a];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const double v = h * (r[k] - C[3 * i + k]);
+        Fo[k] += v;
+        const double t = warp_sum(v);
+        if (lane == 0 && t != 0.0) atomicAdd(&Fa[3 * i + k], -t);
+      }
+    }
+    // lanes of one owner together (most warps have a single one)
+    unsigned todo = __ballot_sync(0xffffffffu, on);
+    while (todo) {
+      const int own = __shfl_sync(0xffffffffu, o, __ffs(todo) - 1);
+      const bool mine = on && o == own;
+      todo &= ~__ballot_sync(0xffffffffu, mine);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const double t = warp_sum(mine ? Fo[k] : 0.0);
+        if (lane == 0 && t != 0.0) atomicAdd(&Fa[3 * own + k], t);
+      }
+    }
+    __syncwarp();
   }
-  double *alloc(size_t n) {
+  for (int e = lane; e < 3 * natoms; e += 32)
+    if (Fa[e] != 0.0) atomicAdd(&F[e], Fa[e]);
+}
+
+static void launch_becke_grad(Plan &P, const double *edens, double clamp, double *F, cudaStream_t s) {
+  if (P.natoms <= kGradCap) {
+    const size_t smem = (size_t)P.natoms * (3 * 32 * sizeof(double) + 3 * sizeof(double) + sizeof(int));
+    NKX_CUDA(cudaFuncSetAttribute(becke_grad_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // as many warps as fit an SM's shared memory at once, at most 32
+    const long per_sm = std::min<long>(32, (long)((200 << 10) / (smem + 1024)));
+    const unsigned grid = (unsigned)std::min<long>(P.npad / 32, per_sm * P.nsm);
+    becke_grad_warp_kernel<<<grid, 32, smem, s>>>(P.d_centers, P.natoms, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_owner,
+                                                  edens, P.npad, clamp, F);
+  } else {
+    const size_t fs_bytes = sizeof(double) * 3 * (size_t)P.natoms;
+    const bool smem = fs_bytes <= 48 * 1024;
+    becke_grad_kernel<<<gblk(P.npad, 128), 128, smem ? fs_bytes : 0, s>>>(P.d_centers, P.natoms, P.d_px, P.d_py,
+                                                                         P.d_pz, P.d_w, P.d_owner, edens, P.npad,
+                                                                         clamp, smem, F);
+  }
+  NKX_LAUNCH_CHECK();
+}
+
+struct GradState {
+  double *T = nullptr, *X = nullptr, *Cocc = nullptr, *edens = nullptr, *F = nullptr;
+  size_t T_cap = 0, X_cap = 0, C_cap = 0;
+  ~GradState() {
+    for (double *p : {T, X, Cocc, edens, F}) cudaFree(p);
+  }
+  static double *alloc(size_t n) {
     double *p = nullptr;
     if (cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       throw Error{NKX_ERR_ALLOC, "gradient workspace allocation of " + std::to_string(n * 8) + " bytes failed"};
     }
-    bufs.push_back(p);
     return p;
+  }
+  static void ensure(double *&p, size_t &cap, size_t n) {
+    if (n <= cap) return;
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    p = alloc(n);
+    cap = n;
   }
 };
 
 void destroy_grad_state(void *p) { delete static_cast<GradState *>(p); }
 
-// orbital-value tiles of at most this many bytes per sub-range of batches
-constexpr size_t kGradTBytes = (size_t)2 << 30;
-
-static GradState &grad_state(Plan &P, int nspin, int nocc, bool need_T) {
+static GradState &grad_state(Plan &P) {
   if (!P.grad_state) {
     GradState *G = new GradState();
     P.grad_state = G;
-    G->edens = G->alloc(P.npad);
-    G->F = G->alloc(3 * (size_t)P.natoms);
+    G->edens = GradState::alloc(P.npad);
+    G->F = GradState::alloc(3 * (size_t)P.natoms);
   }
-  GradState &G = *static_cast<GradState *>(P.grad_state);
-  if (!need_T) return G;
-  const int NC = P.gga ? 4 : 1;
-  const int nocc_pad = ((nocc + 63) / 64) * 64;
-  long maxb = 1;
-  for (const Chunk &c : P.chunks) maxb = std::max(maxb, c.b1 - c.b0);
-  const size_t per_batch = (size_t)nspin * NC * nocc_pad * kBatch * sizeof(double);
-  const long cap = std::max<long>(1, std::min<long>(maxb, (long)(kGradTBytes / per_batch)));
-  if (nocc_pad != G.nocc_pad || nspin != G.nspin || cap > G.cap_batches) {
-    G.nocc_pad = nocc_pad;
-    G.nspin = nspin;
-    G.cap_batches = cap;
-    G.T = G.alloc((size_t)cap * per_batch / sizeof(double));
-  }
-  return G;
+  return *static_cast<GradState *>(P.grad_state);
 }
 
-// FP64 part of the gradient: the density of the FP64 build, the functional,
-// then per chunk the FP64 collocation, the orbital values T and the pair terms.
-static void fp64_gradient_chunks(Plan &P, GradState &G, int nspin, int nocc, cudaStream_t s, StageTimer &Tm) {
-  fp64_density_pass(P, nspin, nocc, s, Tm);
-  functional_kernel<<<gblk(P.npad, 256), 256, 0, s>>>(P.xc, P.gga, nspin, P.npad, P.npad, P.d_w, P.d_rho, P.d_grad, nullptr,
-                                                     P.d_coef, P.d_E, G.edens);
+template <bool FAST>
+static void launch_grad_pairs(Plan &P, long q0, long q1, int nspin, const double *X, double *F, cudaStream_t s) {
+  auto *kernel = P.gga ? grad_pair_kernel<true, FAST> : grad_pair_kernel<false, FAST>;
+  for (int spin = 0; spin < nspin; ++spin) {
+    kernel<<<(unsigned)(q1 - q0), 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_fatom, P.d_px, P.d_py,
+                                               P.d_pz, P.d_owner, P.d_pair_batch, P.d_pair_blk, q0, nspin, spin,
+                                               P.d_coef, P.npad, X, F);
+    NKX_LAUNCH_CHECK();
+    ++P.launches;
+  }
+}
+
+// T and X of the FP64 gradient go through buffers of at most this many bytes
+constexpr size_t kGradTBytes = (size_t)2 << 30, kGradXBytes = (size_t)4 << 30;
+
+// FP64 part of the gradient: per chunk the FP64 collocation, then per range
+// of its batches the orbital values T with the density, the functional,
+// X = (C occ) T of the range's pairs, and the pair terms.
+static void fp64_gradient_chunks(Plan &P, GradState &G, int nspin, int nocc, cudaStream_t s) {
+  const int NC = P.gga ? 4 : 1;
+  int nn = 0;
+  const int nocc_pad = fp64_orbital_pad(nocc, &nn);
+  const size_t t1 = (size_t)nspin * NC * nocc_pad * kBatch, x1 = (size_t)nspin * NC * kBatch * kBlockF;
+  const long cap_b = std::max<long>(1, (long)(kGradTBytes / 8 / t1));
+  const long cap_q = std::max<long>(P.nblk, (long)(kGradXBytes / 8 / x1));
+  fp64_density_begin(P, nspin, nocc, s);
+  G.ensure(G.Cocc, G.C_cap, (size_t)nspin * nocc * P.nbf_pad);
+  const long nC = (long)nspin * nocc * P.nbf_pad;
+  scale_orbitals_kernel<<<gblk(nC, 256), 256, 0, s>>>(P.d_Ct, P.d_occ, P.nbf_pad, nC, G.Cocc);
   NKX_LAUNCH_CHECK();
   ++P.launches;
+  NKX_CUDA(cudaFuncSetAttribute(x_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem));
   for (const Chunk &c : P.chunks) {
-    if (c.p1 <= c.p0) continue;
     launch_colloc(P, c, s);
-    for (long sb0 = c.b0; sb0 < c.b1; sb0 += G.cap_batches) {
-      const long sb1 = std::min(c.b1, sb0 + G.cap_batches);
-      const long q0 = P.h_pair_off[sb0], q1 = P.h_pair_off[sb1];
+    for (long b0 = c.b0, b1; b0 < c.b1; b0 = b1) {
+      const long q0 = P.h_pair_off[b0];
+      b1 = b0 + 1;
+      while (b1 < c.b1 && b1 - b0 < cap_b && P.h_pair_off[b1 + 1] - q0 <= cap_q) ++b1;
+      const long q1 = P.h_pair_off[b1];
+      G.ensure(G.T, G.T_cap, (size_t)(b1 - b0) * t1);
+      G.ensure(G.X, G.X_cap, (size_t)(q1 - q0) * x1);
+      fp64_density_range(P, b0, b1, c.p0, nspin, nocc, G.T, s);
+      const long g0 = b0 * kBatch, n = (b1 - b0) * kBatch;
+      functional_kernel<<<gblk(n, 256), 256, 0, s>>>(P.xc, P.gga, nspin, P.npad, n, P.d_w + g0, P.d_rho + g0,
+                                                     P.d_grad + g0, nullptr, P.d_coef + g0, P.d_E, G.edens + g0);
+      NKX_LAUNCH_CHECK();
+      ++P.launches;
       if (q1 <= q0) continue;
-      const dim3 og((unsigned)((sb1 - sb0) * 4), nspin, G.nocc_pad / 64);
-      if (P.gga)
-        orbital_values_kernel<true><<<og, 256, 0, s>>>(P.ws_phi, P.d_Ct, nocc, G.nocc_pad, P.nbf_pad, P.d_pair_off,
-                                                       P.d_pair_blk, sb0, c.p0, nspin, G.T);
-      else
-        orbital_values_kernel<false><<<og, 256, 0, s>>>(P.ws_phi, P.d_Ct, nocc, G.nocc_pad, P.nbf_pad, P.d_pair_off,
-                                                        P.d_pair_blk, sb0, c.p0, nspin, G.T);
+      x_fp64_kernel<<<dim3((unsigned)(2 * (q1 - q0)), nspin * NC), 256, kXSmem, s>>>(
+          G.T, G.Cocc, nocc, nocc_pad, P.nbf_pad, nspin, NC, P.d_pair_batch, P.d_pair_blk, q0, b0, G.X);
       NKX_LAUNCH_CHECK();
-      if (P.gga)
-        grad_pair_kernel<true><<<(unsigned)(q1 - q0), 256, 0, s>>>(
-            P.d_sto, P.d_fatom, P.d_px, P.d_py, P.d_pz, P.d_owner, P.d_pair_batch, P.d_pair_blk, q0, sb0, P.d_Ct,
-            P.d_occ, nocc, G.nocc_pad, P.nbf_pad, nspin, G.T, P.d_coef, P.npad, G.F);
-      else
-        grad_pair_kernel<false><<<(unsigned)(q1 - q0), 256, 0, s>>>(
-            P.d_sto, P.d_fatom, P.d_px, P.d_py, P.d_pz, P.d_owner, P.d_pair_batch, P.d_pair_blk, q0, sb0, P.d_Ct,
-            P.d_occ, nocc, G.nocc_pad, P.nbf_pad, nspin, G.T, P.d_coef, P.npad, G.F);
-      NKX_LAUNCH_CHECK();
-      P.launches += 2;
+      ++P.launches;
+      launch_grad_pairs<false>(P, q0, q1, nspin, G.X, G.F, s);
     }
   }
 }
@@ -599,47 +770,28 @@ static void xc_gradient(Plan &P, int precision, int nspin, int nocc, const doubl
   NKX_REQUIRE(P.natoms > 0 && P.d_owner, NKX_ERR_ARG, "the gradient needs a plan created with atoms and point owners");
   NKX_REQUIRE(P.all_funcs_on_atoms, NKX_ERR_ARG, "the gradient needs every basis function centred on an atom");
   P.launches = 0;
-  StageTimer Tm;
   NKX_CUDA(cudaMemsetAsync(P.d_status, 0, sizeof(int) * 2, s));
   upload_orbitals(P, nspin, nocc, C, occ, mem, s);
   const bool mixed = precision == NKX_PREC_MIXED;
-  GradState &G = grad_state(P, nspin, nocc, !mixed);
+  GradState &G = grad_state(P);
   NKX_CUDA(cudaMemsetAsync(P.d_E, 0, sizeof(double), s));
   NKX_CUDA(cudaMemsetAsync(G.F, 0, sizeof(double) * 3 * P.natoms, s));
   if (mixed) {
     // Mixed precision: per chunk, the orbital values T_c come from the int8
     // digit contraction on the tensor cores, which also gives rho, grad rho
     // and the functional of the chunk's points, and so do X = C (occ T) and
-    // its gradient; the pair terms with the STO Hessians and the Becke term
-    // are FP64.
+    // its gradient; the pair terms and the Becke term are FP64.
     mixed_gradient_begin(P, nspin, nocc, s);
     for (const Chunk &c : P.chunks) {
-      int npadT = 0;
-      const double *X = nullptr;
-      const double *T = mixed_gradient_chunk(P, c, nspin, nocc, G.edens, s, &npadT, &X);
-      const long q0 = c.p0, q1 = c.p1;
-      if (q1 <= q0) continue;
-      if (P.gga)
-        grad_pair_kernel<true, true><<<(unsigned)(q1 - q0), 256, 0, s>>>(
-            P.d_sto, P.d_fatom, P.d_px, P.d_py, P.d_pz, P.d_owner, P.d_pair_batch, P.d_pair_blk, q0, c.b0, P.d_Ct,
-            P.d_occ, nocc, npadT, P.nbf_pad, nspin, T, P.d_coef, P.npad, G.F, X);
-      else
-        grad_pair_kernel<false, true><<<(unsigned)(q1 - q0), 256, 0, s>>>(
-            P.d_sto, P.d_fatom, P.d_px, P.d_py, P.d_pz, P.d_owner, P.d_pair_batch, P.d_pair_blk, q0, c.b0, P.d_Ct,
-            P.d_occ, nocc, npadT, P.nbf_pad, nspin, T, P.d_coef, P.npad, G.F, X);
-      NKX_LAUNCH_CHECK();
-      ++P.launches;
+      const double *X = mixed_gradient_chunk(P, c, nspin, nocc, G.edens, s);
+      if (c.p1 > c.p0) launch_grad_pairs<true>(P, c.p0, c.p1, nspin, X, G.F, s);
     }
   } else {
-    fp64_gradient_chunks(P, G, nspin, nocc, s, Tm);
+    fp64_gradient_chunks(P, G, nspin, nocc, s);
   }
   const size_t fs_bytes = sizeof(double) * 3 * (size_t)P.natoms;
-  const bool smem = fs_bytes <= 48 * 1024;
-  becke_grad_kernel<<<gblk(P.npad, 128), 128, smem ? fs_bytes : 0, s>>>(P.d_centers, P.natoms, P.d_px, P.d_py,
-                                                                         P.d_pz, P.d_w, P.d_owner, G.edens, P.npad,
-                                                                         clamp, smem, G.F);
-  NKX_LAUNCH_CHECK();
-  P.launches += 2;
+  launch_becke_grad(P, G.edens, clamp, G.F, s);
+  ++P.launches;
   NKX_CUDA(cudaMemcpyAsync(grad, G.F, fs_bytes, cudaMemcpyDeviceToHost, s));
   int status[2] = {0, 0};
   NKX_CUDA(cudaMemcpyAsync(status, P.d_status, sizeof(status), cudaMemcpyDeviceToHost, s));

@@ -32,6 +32,7 @@
 #include <numeric>
 #include <vector>
 
+#include "dmma.cuh"
 #include "functionals.cuh"
 #include "host_setup.hpp"
 #include "plan.cuh"
@@ -124,25 +125,6 @@ __global__ void __launch_bounds__(256) colloc_fp64_kernel(const StoFunc *__restr
   }
 }
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// D += A B on the FP64 tensor path: A 8 x 4 (thread t holds row t / 4,
-// column t % 4), B 4 x 8 (row t % 4, column t / 4), D 8 x 8 (row t / 4,
-// columns 2 (t % 4) and + 1)
-__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
-}
-
 // Density of one slab of one batch for one spin, FP64: T(g, i) = sum_f
 // PhiT(g, f) C(f, i) over the batch's significant blocks (and the three
 // gradient components), then rho = sum_i occ_i T^2 and grad rho =
@@ -156,7 +138,8 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
 // makes both fragment reads free of bank conflicts.  The orbital tile is the
 // fastest grid index, so the CTAs of one slab run together and read its PhiT
 // rows from L2; each adds its share of rho and grad rho atomically (zeroed by
-// the caller).
+// the caller).  With T (the gradient) the orbital values are also written,
+// T[(b - b0, spin, comp)][i][g].
 //
 // Bound: FP64 pipe from about 16 orbitals on, PhiT from HBM below.  The
 // orbital tile is ceil(nocc / ntile / 8) * 8 wide instead of a fixed 64, so 5
@@ -176,7 +159,7 @@ __global__ void __launch_bounds__(256, DShape<NN>::CTAS)
     density_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ Cf, const double *__restrict__ occ,
                         int nocc, int nocc_pad, int nbf_pad, const int *__restrict__ pair_off,
                         const int *__restrict__ pair_blk, long b0, long p0, double *__restrict__ rho,
-                        double *__restrict__ grad, long npad) {
+                        double *__restrict__ grad, long npad, double *__restrict__ T) {
   using Sh = DShape<NN>;
   constexpr int NC = GRAD ? 4 : 1, NT = Sh::NT, LDP = Sh::LDP, LDC = Sh::LDC, ST = Sh::STAGES;
   constexpr int SLABS = GRAD ? 4 : 1;  // slabs of a batch
@@ -193,7 +176,7 @@ __global__ void __launch_bounds__(256, DShape<NN>::CTAS)
   const int q0 = pair_off[b], q1 = pair_off[b + 1];
   const size_t tile = (size_t)kBatch * kBlockF;
   const int total = (q1 - q0) * (kBlockF / kDKs);  // K steps of the orbital tile
-  if (total == 0) return;  // no significant function: nothing to add
+  if (total == 0) return;  // no significant function: nothing to add (and no pair that reads T)
   auto issue = [&](int t, int st) {
     if (t < total) {
       const int q = q0 + t / (kBlockF / kDKs), f0 = (t % (kBlockF / kDKs)) * kDKs;
@@ -241,6 +224,17 @@ __global__ void __launch_bounds__(256, DShape<NN>::CTAS)
     }
   }
   cp_async_wait<0>();
+  if (T) {
+    double *Tb = T + ((size_t)(b - b0) * gridDim.y + spin) * NC * nocc_pad * kBatch;
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          Tb[((size_t)(GRAD ? m : 0) * nocc_pad + i0 + 8 * n + 2 * fk + h) * kBatch +
+             (GRAD ? g0 + 8 * warp + fr : 32 * warp + 8 * m + fr)] = acc[m][n][h];
+  }
   // contract over this orbital tile: the four lanes of a row hold its columns
   double sm[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -1702,26 +1696,45 @@ void coulomb_solve(Plan &P, cudaStream_t s, bool mixed) {
 }
 
 template <bool GRAD, int NN>
-static void launch_density_fp64(Plan &P, const Chunk &c, int nspin, int nocc, int nocc_pad, cudaStream_t s) {
+static void launch_density_fp64(Plan &P, long b0, long b1, long p0, int nspin, int nocc, int nocc_pad, double *T,
+                                cudaStream_t s) {
   NKX_CUDA(cudaFuncSetAttribute(density_fp64_kernel<GRAD, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 DShape<NN>::kSmem));
-  const dim3 grid((unsigned)((c.b1 - c.b0) * (GRAD ? 4 : 1) * (nocc_pad / (8 * NN))), nspin);
+  const dim3 grid((unsigned)((b1 - b0) * (GRAD ? 4 : 1) * (nocc_pad / (8 * NN))), nspin);
   density_fp64_kernel<GRAD, NN><<<grid, 256, DShape<NN>::kSmem, s>>>(P.ws_phi, P.d_Cf, P.d_occ, nocc, nocc_pad,
-                                                                    P.nbf_pad, P.d_pair_off, P.d_pair_blk, c.b0, c.p0,
-                                                                    P.d_rho, P.d_grad, P.npad);
+                                                                    P.nbf_pad, P.d_pair_off, P.d_pair_blk, b0, p0,
+                                                                    P.d_rho, P.d_grad, P.npad, T);
 }
-template <bool GRAD>
-static void launch_density_nn(Plan &P, const Chunk &c, int nn, int nspin, int nocc, int nocc_pad, cudaStream_t s) {
-  switch (nn) {
-    case 1: return launch_density_fp64<GRAD, 1>(P, c, nspin, nocc, nocc_pad, s);
-    case 2: return launch_density_fp64<GRAD, 2>(P, c, nspin, nocc, nocc_pad, s);
-    case 3: return launch_density_fp64<GRAD, 3>(P, c, nspin, nocc, nocc_pad, s);
-    case 4: return launch_density_fp64<GRAD, 4>(P, c, nspin, nocc, nocc_pad, s);
-    case 5: return launch_density_fp64<GRAD, 5>(P, c, nspin, nocc, nocc_pad, s);
-    case 6: return launch_density_fp64<GRAD, 6>(P, c, nspin, nocc, nocc_pad, s);
-    case 7: return launch_density_fp64<GRAD, 7>(P, c, nspin, nocc, nocc_pad, s);
-    default: return launch_density_fp64<GRAD, 8>(P, c, nspin, nocc, nocc_pad, s);
-  }
+
+// orbital tiles of at most 64, equally wide, in multiples of 8: *nn eighths
+// of a tile; returns the padded orbital count
+int fp64_orbital_pad(int nocc, int *nn) {
+  const int ntile = (nocc + 63) / 64;
+  *nn = ((nocc + ntile - 1) / ntile + 7) / 8;
+  return ntile * 8 * *nn;
+}
+
+// The FP64 density of batches [b0, b1) of a chunk whose collocation is in
+// ws_phi (first pair p0), after fp64_density_begin
+void fp64_density_range(Plan &P, long b0, long b1, long p0, int nspin, int nocc, double *T, cudaStream_t s) {
+  int nn = 0;
+  const int np = fp64_orbital_pad(nocc, &nn);
+  auto go = [&](auto grad) {
+    constexpr bool G = decltype(grad)::value;
+    switch (nn) {
+      case 1: return launch_density_fp64<G, 1>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      case 2: return launch_density_fp64<G, 2>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      case 3: return launch_density_fp64<G, 3>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      case 4: return launch_density_fp64<G, 4>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      case 5: return launch_density_fp64<G, 5>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      case 6: return launch_density_fp64<G, 6>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      case 7: return launch_density_fp64<G, 7>(P, b0, b1, p0, nspin, nocc, np, T, s);
+      default: return launch_density_fp64<G, 8>(P, b0, b1, p0, nspin, nocc, np, T, s);
+    }
+  };
+  P.gga ? go(std::true_type{}) : go(std::false_type{});
+  NKX_LAUNCH_CHECK();
+  ++P.launches;
 }
 
 // The FP64 V contraction of one chunk: nz planes of zT (stride z_stride
@@ -1743,22 +1756,25 @@ static void launch_vgemm_fp64(Plan &P, const Chunk &c, const double *phiT, const
   NKX_LAUNCH_CHECK();
 }
 
-// FP64 pass A: collocation + density of every chunk into d_rho / d_grad
-void fp64_density_pass(Plan &P, int nspin, int nocc, cudaStream_t s, StageTimer &T) {
-  // orbital tiles of at most 64, equally wide, in multiples of 8
-  const int ntile = (nocc + 63) / 64, nn = ((nocc + ntile - 1) / ntile + 7) / 8;
-  const int nocc_pad = ntile * 8 * nn;
+// function-major orbitals, and rho / grad rho cleared for the kernels' shares
+void fp64_density_begin(Plan &P, int nspin, int nocc, cudaStream_t s) {
+  int nn = 0;
+  const int nocc_pad = fp64_orbital_pad(nocc, &nn);
   if ((size_t)nocc_pad * P.nbf_pad * 2 > P.cf_cap) {
     P.cf_cap = (size_t)nocc_pad * P.nbf_pad * 2;
     P.d_Cf = P.alloc<double>(P.cf_cap);
   }
-  transpose_orbitals_kernel<<<dim3(P.nbf_pad / 32, (nocc_pad + 31) / 32, nspin), dim3(32, 8), 0, s>>>(P.d_Ct, nocc, nocc_pad,
-                                                                                             P.nbf_pad, P.d_Cf);
+  transpose_orbitals_kernel<<<dim3(P.nbf_pad / 32, (nocc_pad + 31) / 32, nspin), dim3(32, 8), 0, s>>>(
+      P.d_Ct, nocc, nocc_pad, P.nbf_pad, P.d_Cf);
   NKX_LAUNCH_CHECK();
   ++P.launches;
-  // the density kernels add their orbital tiles' shares
   NKX_CUDA(cudaMemsetAsync(P.d_rho, 0, sizeof(double) * nspin * P.npad, s));
   if (P.gga) NKX_CUDA(cudaMemsetAsync(P.d_grad, 0, sizeof(double) * 3 * nspin * P.npad, s));
+}
+
+// FP64 pass A: collocation + density of every chunk into d_rho / d_grad
+void fp64_density_pass(Plan &P, int nspin, int nocc, cudaStream_t s, StageTimer &T) {
+  fp64_density_begin(P, nspin, nocc, s);
   for (const Chunk &c : P.chunks) {
     if (c.p1 - c.p0 > 0) {
       T.begin(ST_COLLOC, s);
@@ -1766,10 +1782,7 @@ void fp64_density_pass(Plan &P, int nspin, int nocc, cudaStream_t s, StageTimer 
       T.end(s);
     }
     T.begin(ST_DENSITY, s);
-    P.gga ? launch_density_nn<true>(P, c, nn, nspin, nocc, nocc_pad, s)
-          : launch_density_nn<false>(P, c, nn, nspin, nocc, nocc_pad, s);
-    NKX_LAUNCH_CHECK();
-    ++P.launches;
+    fp64_density_range(P, c.b0, c.b1, c.p0, nspin, nocc, nullptr, s);
     T.end(s);
   }
 }

@@ -196,6 +196,9 @@ enum { ST_COLLOC = 0, ST_DENSITY = 1, ST_FUNC = 2, ST_COULOMB = 3, ST_ZBUILD = 4
 bool mixed_available(const Plan &P);
 void upload_orbitals(Plan &P, int nspin, int nocc, const double *C, const double *occ, int mem, cudaStream_t s);
 void fp64_density_pass(Plan &P, int nspin, int nocc, cudaStream_t s, StageTimer &T);
+int fp64_orbital_pad(int nocc, int *nn);
+void fp64_density_begin(Plan &P, int nspin, int nocc, cudaStream_t s);
+void fp64_density_range(Plan &P, long b0, long b1, long p0, int nspin, int nocc, double *T, cudaStream_t s);
 void launch_colloc(Plan &P, const Chunk &c, cudaStream_t s);
 void destroy_grad_state(void *p);
 __global__ void functional_kernel(XcSpec s, bool gga, int nspin, long npad, long n, const double *__restrict__ w,
@@ -229,8 +232,7 @@ inline int batch_split(long parts, long nbatch, int nsm) {
   return nsplit;
 }
 void mixed_gradient_begin(Plan &P, int nspin, int nocc, cudaStream_t s);
-const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc, double *edens, cudaStream_t s,
-                                   int *nocc_pad, const double **X);
+const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc, double *edens, cudaStream_t s);
 void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool separateJ, cudaStream_t s,
                       StageTimer &T, int phase);
 // mixed: read the aux radial factors from the plan's FP32 table (made on first use)

@@ -1869,10 +1869,9 @@ void mixed_gradient_begin(Plan &P, int nspin, int nocc, cudaStream_t s) {
 // value and (GGA) the three gradient components on the tensor cores (the
 // density contraction with all components), rho and grad rho of the chunk's
 // points from them, and the functional there (Z coefficients, energy, energy
-// density edens).  Returns T[(bl, s, c)][i][g] (bl from the chunk's first
-// batch, i padded to *nocc_pad), resident until the next chunk.
-const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc, double *edens, cudaStream_t s,
-                                   int *nocc_pad, const double **X) {
+// density edens).  Returns X[pair][spin][comp][g][mu] of the chunk's pairs,
+// resident until the next chunk.
+const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc, double *edens, cudaStream_t s) {
   MixedState &M = mixed_state(P, nocc);
   const int nc = P.gga ? 4 : 1;
   const long np = c.p1 - c.p0, nb = c.b1 - c.b0;
@@ -1960,9 +1959,7 @@ const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc,
     launch_i8(M, M.m_t0, M.m_co, x, s);
     ++P.launches;
   }
-  *nocc_pad = M.nocc_pad;
-  *X = M.X;
-  return M.T;
+  return M.X;
 }
 
 void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool separateJ, cudaStream_t s,
