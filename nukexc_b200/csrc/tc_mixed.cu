@@ -136,6 +136,28 @@ __device__ __forceinline__ double level_sum(uint32_t l0, uint32_t l1, uint32_t l
   return __longlong_as_double(S + 0x4338000000000000LL) - 0x1.8p52;
 }
 
+// The same sum for K <= 256 with fewer instructions: a = 2^8 L0 + L1 and
+// b = 2^8 L2 + L3 fit int32.  With |X| <= 2^30 the digits obey |d0| <= 64 and,
+// where |d0| = 64, d1 has the sign that brings X back, so per product
+// |d0 e0| <= 2^12, |d0 e1 + d1 e0| <= 2^14, |d0 e2 + d1 e1 + d2 e0| <= 32576
+// (d0 = 64, d1 = e1 = -128, e2 = 127, d2 = -128, e0 = -63) and |L3's four|
+// <= 49152, the last two not together: 256 (256 32576 + 49152) = 2^31 is not
+// reached.  (H2O)_64 PBE: V 325 -> 304 ms per build with this and the
+// exponent-field scales below (the card is at its power limit during V, so every
+// instruction of the read-back counts even where it overlaps the MMAs).
+__device__ __forceinline__ double quad_sum(uint32_t l0, uint32_t l1, uint32_t l2, uint32_t l3) {
+  const int a = (int)l0 * 256 + (int)l1, b = (int)l2 * 256 + (int)l3;
+  const long long S = (long long)a * 65536 + b;
+  return __longlong_as_double(S + 0x4338000000000000LL) - 0x1.8p52;
+}
+// Power-of-two scale s_a s_b 2^-36 from the high words of s_a and s_b: the
+// exponent fields add.  Clamped at 0 (a product below 2^-1022 is zero) and at
+// 0x7ff00000 (infinity).
+__device__ __forceinline__ int scale_row_word(double sa) { return __double2hiint(sa) - ((1023 + 36) << 20); }
+__device__ __forceinline__ double scale_product(int row_word, int col_word) {
+  return __hiloint2double(__viaddmin_s32_relu(row_word, col_word, 0x7ff00000), 0);
+}
+
 struct UnitIter {
   int I = 0, J = 0, zi = 0, sp = 0, hc = 0;  // V: row block, column block, Z plane, batch split, column part
   long bl = 0;                     // density: batch within chunk
@@ -278,7 +300,7 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
   __shared__ uint32_t tmem_base_sh;
   __shared__ volatile int abort_flag;
   // V and density: the column scales of each epilogue warp's current group
-  __shared__ __align__(16) double colscale[MODE == TC_MODE_V || MODE == TC_MODE_DENSITY ? Sh::EW * CW : 2];
+  __shared__ __align__(16) int colscale[MODE == TC_MODE_V || MODE == TC_MODE_DENSITY ? Sh::EW * CW : 4];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -557,22 +579,21 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
         if (!mbar_wait(&tfull_bar[buf], use & 1, a.err, 6, &abort_flag, a.wait_ns)) return;
         tc_fence_after();
         __syncwarp();
-        // exact combine of the four levels, S = sum_L 2^(8 (3 - L)) Acc_L:
-        // |Acc_L| < 2^24 for K <= 256, so |S| < 2^49 (level_sum); the product
-        // is s_a s_b 2^-36 S (one rounding per group and element)
+        // exact combine of the four levels, S = sum_L 2^(8 (3 - L)) Acc_L
+        // (quad_sum); the product is s_a s_b 2^-36 S (one rounding per group
+        // and element)
         if constexpr (MODE == TC_MODE_V || MODE == TC_MODE_DENSITY) {
-          // s_a is the thread's row scale; the warp's CW column scales are
-          // staged in shared memory once per group and read back as
-          // broadcasts, two per 16-byte load (instead of two shuffles per
-          // element).  Slices of four columns are software-pipelined: the
-          // loads of slice h + 1 are in flight while slice h is combined, and
-          // TMEM is released as soon as the last slice has arrived in
+          // the high words of the warp's CW column scales are staged in
+          // shared memory once per group and read back as broadcasts, four
+          // per 16-byte load.  Slices of four columns are software-pipelined:
+          // the loads of slice h + 1 are in flight while slice h is combined,
+          // and TMEM is released as soon as the last slice has arrived in
           // registers.
           if (live) {
-            const double sa = sa_g * kTwoM36;
-            double *cs = colscale + (warp - 2) * CW;
+            const int ha = scale_row_word(sa_g);
+            int *cs = colscale + (warp - 2) * CW;
 #pragma unroll
-            for (int k = 0; k < CW / 32; ++k) cs[32 * k + lane] = sb_g[k];
+            for (int k = 0; k < CW / 32; ++k) cs[32 * k + lane] = __double2hiint(sb_g[k]);
             __syncwarp();
             const uint32_t tb = tmem + lane_addr + buf * 4 * N + CW * cq;
             constexpr int NS = CW / 4;
@@ -586,12 +607,11 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
             };
             auto combine = [&](int h, const uint32_t(&x0)[4], const uint32_t(&x1)[4], const uint32_t(&x2)[4],
                                const uint32_t(&x3)[4]) {
-              const double2 c01 = *reinterpret_cast<const double2 *>(cs + 4 * h);
-              const double2 c23 = *reinterpret_cast<const double2 *>(cs + 4 * h + 2);
-              const double sc[4] = {c01.x, c01.y, c23.x, c23.y};
+              const int4 c4 = *reinterpret_cast<const int4 *>(cs + 4 * h);
+              const int hc[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
               for (int j = 0; j < 4; ++j)
-                acc[4 * h + j] = fma(level_sum(x0[j], x1[j], x2[j], x3[j]), sa * sc[j], acc[4 * h + j]);
+                acc[4 * h + j] = fma(quad_sum(x0[j], x1[j], x2[j], x3[j]), scale_product(ha, hc[j]), acc[4 * h + j]);
             };
             issue(0, p0, p1, p2, p3);
 #pragma unroll
