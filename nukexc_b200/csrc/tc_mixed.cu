@@ -52,7 +52,10 @@ constexpr double kTwoM36 = 0x1p-36;
 // (grad rho = 2 sum_mu grad phi_mu Y_mu, summed in the Y pass's epilogue)
 // TC_MODE_X (mixed XC gradient): X_c(g, mu) = sum_i T_c(g, i) (C occ)(mu, i)
 // for the value and the three gradient components, written in FP64
-enum { TC_MODE_V = 0, TC_MODE_DENSITY = 1, TC_MODE_GRAD = 2, TC_MODE_X = 3 };
+// TC_MODE_RHO: the density mode with the contraction over the orbitals in its
+// epilogue: a unit takes all components of its points in turn, keeps T_0 in
+// shared memory and writes per point only sum_i occ_i T_0 T_c of its columns
+enum { TC_MODE_V = 0, TC_MODE_DENSITY = 1, TC_MODE_GRAD = 2, TC_MODE_X = 3, TC_MODE_RHO = 4 };
 
 // Shape by the MMA width N.  N = 128: one TMEM buffer of 4 levels x 128
 // columns, 16 epilogue warps, 3 stages of 64 KB.  N = 64: two buffers of
@@ -83,6 +86,10 @@ struct TcShape {
   static constexpr uint32_t kIdesc = idesc_i8(128, N);
   static constexpr int kSmem = kStages * kStageBytes + 1024;
 };
+// TC_MODE_RHO: N = 64 with one stage fewer and T_0 of the epilogue threads,
+// [32 columns][thread]
+constexpr int kRhoStages = 3;
+constexpr int kRhoSmem = kRhoStages * TcShape<64>::kStageBytes + 32 * TcShape<64>::kEpiThreads * 8 + 1024;
 
 struct TcArgs {
   int mode;
@@ -99,6 +106,12 @@ struct TcArgs {
   // components are contracted, ncs are stored per pair in qphT / sphT
   int nspin, ncomp, ncs, ntile_i, nocc_pad;
   double *T;
+  // rho mode: occ[s][i] (nocc of them), output Rp[part][spin][comp][point of
+  // the chunk] with part = (orbital tile, column group), rstride points a plane
+  const double *occ;
+  int nocc;
+  double *Rp;
+  long rstride;
   // grad mode: sA = st0[(bl, s, h)][128] (T0 row scales), sB = sco[s][mu]
   // (C occ row scales); grad phi from the pass-A digits qphT[pair][comp][digit][g][f]
   // and scales sphT[pair][comp][g] (ncs components); output the partial sums
@@ -191,8 +204,10 @@ struct UnitIter {
       long r = u;
       t = (int)(r % a.ntile_i);
       r /= a.ntile_i;
-      c = (int)(r % a.ncomp);
-      r /= a.ncomp;
+      if constexpr (MODE == TC_MODE_DENSITY) {
+        c = (int)(r % a.ncomp);
+        r /= a.ncomp;
+      }
       h = (int)(r % 2);
       r /= 2;
       s = (int)(r % a.nspin);
@@ -205,6 +220,8 @@ struct Group {
   int nsteps;   // K steps of 64 bytes
   long qa, qb;  // V: chunk-relative pairs of the row / column blocks
   int blk;      // density: function block (-1: empty batch)
+  int c;        // rho: component
+  bool last;    // rho: last block of the component
 };
 
 __device__ __forceinline__ int blk_pos(const uint32_t *m, int I) {
@@ -259,6 +276,29 @@ __device__ __forceinline__ void for_each_group(const TcArgs &a, const UnitIter &
       yB = yb;
       zB = zb;
     });
+  } else if constexpr (MODE == TC_MODE_RHO) {
+    const long b = a.b0 + it.bl;
+    const int q0 = a.pair_off[b], q1 = a.pair_off[b + 1];
+    for (int c = 0; c < a.ncomp; ++c)
+      for (int q = q0; q < q1; ++q) {
+        Group g;
+        g.nsteps = 2;
+        g.qa = q - a.p0;
+        g.qb = 0;
+        g.blk = a.pair_blk[q];
+        g.c = c;
+        g.last = q + 1 == q1;
+        const int za = (int)((g.qa * a.ncs + c) * 4), ya = 128 * it.h;
+        const int xb0 = g.blk * 128, yb = a.nt * it.t, zb = it.s * 4;
+        fn(g, [=](int k, int &xa, int &yA, int &zA, int &xb, int &yB, int &zB) {
+          xa = 64 * k;
+          yA = ya;
+          zA = za;
+          xb = xb0 + 64 * k;
+          yB = yb;
+          zB = zb;
+        });
+      }
   } else {
     const long b = a.b0 + it.bl;
     const int q0 = a.pair_off[b], q1 = a.pair_off[b + 1];
@@ -293,14 +333,17 @@ template <int MODE, int NW, int EW = NW / 8>
 __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
     tc_i8_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, TcArgs a) {
   using Sh = TcShape<NW, EW>;
-  constexpr int N = Sh::N, NBUF = Sh::NBUF, kStages = Sh::kStages, kStageBytes = Sh::kStageBytes, CW = Sh::CW;
+  constexpr int N = Sh::N, NBUF = Sh::NBUF, kStageBytes = Sh::kStageBytes, CW = Sh::CW;
+  constexpr int kStages = MODE == TC_MODE_RHO ? kRhoStages : Sh::kStages;
+  // modes that accumulate a run of groups in registers
+  constexpr bool kRun = MODE == TC_MODE_V || MODE == TC_MODE_DENSITY || MODE == TC_MODE_RHO;
   static_assert(MODE == TC_MODE_V || CW == 32, "the density, Y and X epilogues take 32 columns a warp");
   extern __shared__ __align__(1024) uint8_t dsmem[];
   __shared__ uint64_t full_bar[kStages], empty_bar[kStages], tfull_bar[NBUF], tempty_bar[NBUF], drain_bar, stall_bar;
   __shared__ uint32_t tmem_base_sh;
   __shared__ volatile int abort_flag;
   // V and density: the column scales of each epilogue warp's current group
-  __shared__ __align__(16) int colscale[MODE == TC_MODE_V || MODE == TC_MODE_DENSITY ? Sh::EW * CW : 4];
+  __shared__ __align__(16) int colscale[kRun ? Sh::EW * CW : 4];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -418,6 +461,7 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
 #pragma unroll
       for (int j = 0; j < CW; ++j) acc[j] = 0.0;
       bool any = false;
+      double rs[4] = {0.0, 0.0, 0.0, 0.0};  // rho: the thread's sums over its columns
       for_each_group<MODE>(a, it, [&](const Group &g, auto) {
         if (abort_flag) return;
         const uint32_t buf = grp % NBUF, use = grp / NBUF;
@@ -572,7 +616,7 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
 #pragma unroll
             for (int k = 0; k < CW / 32; ++k) sb_g[k] = sbp[32 * k + lane];
           } else {
-            sa_g = a.sA[(g.qa * a.ncs + it.c) * 256 + 128 * it.h + row];
+            sa_g = a.sA[(g.qa * a.ncs + (MODE == TC_MODE_RHO ? g.c : it.c)) * 256 + 128 * it.h + row];
             sb_g[0] = a.sB[((size_t)it.s * a.nocc_pad + N * it.t + 32 * cq + lane) * a.nblk + g.blk];
           }
         }
@@ -582,7 +626,7 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
         // exact combine of the four levels, S = sum_L 2^(8 (3 - L)) Acc_L
         // (quad_sum); the product is s_a s_b 2^-36 S (one rounding per group
         // and element)
-        if constexpr (MODE == TC_MODE_V || MODE == TC_MODE_DENSITY) {
+        if constexpr (kRun) {
           // the high words of the warp's CW column scales are staged in
           // shared memory once per group and read back as broadcasts, four
           // per 16-byte load.  Slices of four columns are software-pipelined:
@@ -638,6 +682,26 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
           }
           ++grp;
           any = any || live;
+          if constexpr (MODE == TC_MODE_RHO) {
+            // the component is complete: T_0 stays in the thread's column of
+            // shared memory, and occ T_0 T_c is summed over its 32 orbitals
+            if (g.last) {
+              double *t0 = reinterpret_cast<double *>(smem + kStages * kStageBytes) + (threadIdx.x - 64);
+              const int i0 = N * it.t + 32 * cq;
+              const double *oc = a.occ + (size_t)it.s * a.nocc + i0;
+              const int n = a.nocc - i0;
+              double r = 0.0;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const double o = j < n ? oc[j] : 0.0;
+                if (g.c == 0) t0[j * Sh::kEpiThreads] = acc[j];
+                r += o * t0[j * Sh::kEpiThreads] * acc[j];
+                acc[j] = 0.0;
+              }
+#pragma unroll
+              for (int c = 0; c < 4; ++c) rs[c] = g.c == c ? r : rs[c];
+            }
+          }
           return;
         }
       });
@@ -654,6 +718,10 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
             for (int j = 0; j < CW; ++j) Vz[r + (c0 + j) * a.nbf_pad] += acc[j];
           }
         }
+      } else if constexpr (MODE == TC_MODE_RHO) {
+        double *out = a.Rp + (((size_t)(it.t * (N / 32) + cq) * a.nspin + it.s) * a.ncomp) * a.rstride +
+                      it.bl * kBatch + 128 * it.h + row;
+        for (int c = 0; c < a.ncomp; ++c) out[c * a.rstride] = c == 0 ? rs[0] : c == 1 ? rs[1] : c == 2 ? rs[2] : rs[3];
       } else if constexpr (MODE == TC_MODE_GRAD || MODE == TC_MODE_X) {
         // the partial sums (grad) or X (x) are written per group above
       } else {
@@ -1105,6 +1173,24 @@ __global__ void __launch_bounds__(256) ygrad_sum_kernel(const double *__restrict
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) grad[((size_t)s * 3 + c) * npad + b * kBatch + g] = gs[c];
+}
+
+// rho and grad rho = 2 sum_i occ_i T_0 T_c of the chunk's points (spin =
+// block y) from the column groups' shares Rp[part][spin][comp][point], in order
+__global__ void __launch_bounds__(256) rho_sum_kernel(const double *__restrict__ Rp, int nparts, int nspin, int nc,
+                                                      long n, long g0, long npad, double *__restrict__ rho,
+                                                      double *__restrict__ grad) {
+  const long p = blockIdx.x * 256L + threadIdx.x;
+  const int s = blockIdx.y;
+  if (p >= n) return;
+  for (int c = 0; c < nc; ++c) {
+    double v = 0.0;
+    for (int k = 0; k < nparts; ++k) v += Rp[(((size_t)k * nspin + s) * nc + c) * n + p];
+    if (c == 0)
+      rho[(size_t)s * npad + g0 + p] = v;
+    else
+      grad[((size_t)s * 3 + c - 1) * npad + g0 + p] = 2.0 * v;
+  }
 }
 
 // Pass A, fused: collocation of one (batch, block) pair straight into the
@@ -1764,6 +1850,7 @@ static MixedState &mixed_state(Plan &P, int nocc) {
                                   TcShape<64>::kSmem));
     NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_DENSITY, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   TcShape<64>::kSmem));
+    NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_RHO, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRhoSmem));
     NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_DENSITY, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   TcShape<128>::kSmem));
     NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_GRAD, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1800,7 +1887,8 @@ static MixedState &mixed_state(Plan &P, int nocc) {
 template <int MODE, int NW, int EW = NW / 8>
 static void launch_i8_shape(const CUtensorMap &mA, const CUtensorMap &mB, const TcArgs &a, unsigned grid,
                             cudaStream_t s) {
-  tc_i8_kernel<MODE, NW, EW><<<grid, TcShape<NW, EW>::kThreads, TcShape<NW, EW>::kSmem, s>>>(mA, mB, a);
+  constexpr int smem = MODE == TC_MODE_RHO ? kRhoSmem : TcShape<NW, EW>::kSmem;
+  tc_i8_kernel<MODE, NW, EW><<<grid, TcShape<NW, EW>::kThreads, smem, s>>>(mA, mB, a);
 }
 
 // The CTA-pair V contraction: one persistent cluster of two per pair of
@@ -1821,7 +1909,8 @@ static void launch_i8(MixedState &M, const CUtensorMap &mA, const CUtensorMap &m
   if (a.nunits <= 0) return;
   const unsigned grid = (unsigned)std::min<long>(a.nunits, M.nsm);
   NKX_REQUIRE(a.nt == 64 || a.nt == 128, NKX_ERR_ARG, "tensor-core width must be 64 or 128");
-  NKX_REQUIRE(a.mode != TC_MODE_X || a.nt == 64, NKX_ERR_ARG, "the X pass runs N = 64");
+  NKX_REQUIRE((a.mode != TC_MODE_X && a.mode != TC_MODE_RHO) || a.nt == 64, NKX_ERR_ARG,
+              "the X pass and the fused density run N = 64");
   NKX_REQUIRE(a.ew == a.nt / 8 || (a.mode == TC_MODE_V && a.nt == 128 && a.ew == 8), NKX_ERR_ARG,
               "epilogue warps: N / 8, or 8 for the N = 128 V contraction");
   if (a.mode == TC_MODE_V) {
@@ -1837,6 +1926,8 @@ static void launch_i8(MixedState &M, const CUtensorMap &mA, const CUtensorMap &m
                 : launch_i8_shape<TC_MODE_GRAD, 64>(mA, mB, a, grid, s);
   else if (a.mode == TC_MODE_X)
     launch_i8_shape<TC_MODE_X, 64>(mA, mB, a, grid, s);
+  else if (a.mode == TC_MODE_RHO)
+    launch_i8_shape<TC_MODE_RHO, 64>(mA, mB, a, grid, s);
   else
     a.nt == 128 ? launch_i8_shape<TC_MODE_DENSITY, 128>(mA, mB, a, grid, s)
                 : launch_i8_shape<TC_MODE_DENSITY, 64>(mA, mB, a, grid, s);
@@ -1993,8 +2084,15 @@ void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool 
   // by default from 256 orbitals on
   const bool y_ok = P.gga && M.nocc_pad <= 8192;
   const bool grad_mode = y_ok && (P.tune.ypath >= 0 ? P.tune.ypath != 0 : M.nocc_pad >= 256);
+  // Without the Y path, and at N = 64, the density contraction sums over the
+  // orbitals in its own epilogue: no T is written and read back ((H2O)_8 PBE,
+  // 40 orbitals: 999 us for both kernels, 809 now).  The Y path needs T_0
+  // itself, and N = 128 has no registers or shared memory left for it.
+  const bool fused_rho = !grad_mode && density_width(P, nocc) == 64;
+  const int rho_parts = 2 * ((nocc + 63) / 64);
   if (phase != 2) {
-    M.ensure_T((size_t)M.nbatch_chunk * nspin * (grad_mode ? 1 : nc) * M.nocc_pad * 256);
+    M.ensure_T(fused_rho ? (size_t)M.nbatch_chunk * kBatch * nspin * nc * rho_parts
+                         : (size_t)M.nbatch_chunk * nspin * (grad_mode ? 1 : nc) * M.nocc_pad * 256);
     if (grad_mode)
       M.ensure_qt0((size_t)M.nbatch_chunk * nspin * 2 * 4 * 128 * M.nocc_pad, (long)M.nbatch_chunk * nspin * 2 * 4,
                    M.nocc_pad);
@@ -2059,9 +2157,20 @@ void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool 
     a.wait_ns = P.wait_ns;
     a.stall = P.stall_test;
     a.nunits = nb * nspin * 2 * a.ncomp * a.ntile_i;
+    if (fused_rho) {
+      a.mode = TC_MODE_RHO;
+      a.nunits = nb * nspin * 2 * a.ntile_i;
+      a.occ = P.d_occ;
+      a.nocc = nocc;
+      a.Rp = M.T;
+      a.rstride = nb * kBatch;
+    }
     launch_i8(M, M.m_phT, a.nt == 128 ? M.m_ct128 : M.m_ct, a, s);
     ++P.launches;
-    if (P.gga && !grad_mode)
+    if (fused_rho)
+      rho_sum_kernel<<<dim3((unsigned)nb, nspin), 256, 0, s>>>(M.T, rho_parts, nspin, nc, nb * kBatch, c.b0 * kBatch,
+                                                               P.npad, P.d_rho, P.d_grad);
+    else if (P.gga && !grad_mode)
       density_contract_kernel<true><<<dim3((unsigned)nb, nspin), 256, 0, s>>>(M.T, P.d_occ, nocc, M.nocc_pad, nspin,
                                                                               c.b0, P.d_rho, P.d_grad, P.npad);
     else
