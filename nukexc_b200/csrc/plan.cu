@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(256) colloc_fp64_kernel(const StoFunc *__restr
   __syncthreads();
   const size_t tile = (size_t)kBatch * kBlockF;
   double *o = out + (size_t)blockIdx.x * (GRAD ? 4 : 1) * tile;
-  for (int g = warp; g < kBatch; g += 8) {
+  const int npt = kBatch / gridDim.y, g0 = blockIdx.y * npt;  // this CTA's points
+  for (int g = g0 + warp; g < g0 + npt; g += 8) {
     const double x = sx[g], y = sy[g], z = sz[g];
     double v[4][4];
     __syncwarp();
@@ -356,7 +357,8 @@ __global__ void zbuild_fp64_kernel(const double *__restrict__ phiT, const double
   const int b = pair_batch[p0 + q];
   const size_t tile = (size_t)kBatch * kBlockF;
   const double *P = phiT + q * NC * tile;
-  for (int e = threadIdx.x; e < kBatch * kBlockF; e += blockDim.x) {
+  const int ne = kBatch * kBlockF / gridDim.y, e0 = blockIdx.y * ne;  // this CTA's elements
+  for (int e = e0 + threadIdx.x; e < e0 + ne; e += blockDim.x) {
     const int g = e / kBlockF;
     const long gg = (long)b * kBatch + g;
     const double v = P[e];
@@ -1563,8 +1565,9 @@ void launch_colloc(Plan &P, const Chunk &c, cudaStream_t s) {
   const long np = c.p1 - c.p0;
   if (np <= 0) return;
   auto *kernel = P.gga ? colloc_fp64_kernel<true> : colloc_fp64_kernel<false>;
-  kernel<<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_px, P.d_py, P.d_pz,
-                                      P.d_pair_batch, P.d_pair_blk, c.p0, P.ws_phi);
+  kernel<<<dim3((unsigned)np, point_split(np, P.nsm)), 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell,
+                                                                    P.d_px, P.d_py, P.d_pz, P.d_pair_batch,
+                                                                    P.d_pair_blk, c.p0, P.ws_phi);
   NKX_LAUNCH_CHECK();
   ++P.launches;
 }
@@ -1829,11 +1832,12 @@ void fock_build_fp64(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool s
       T.end(s);
     }
     T.begin(ST_ZBUILD, s);
+    const dim3 zgrid((unsigned)np, point_split(np, P.nsm));
     if (P.gga)
-      zbuild_fp64_kernel<true><<<(unsigned)np, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs,
+      zbuild_fp64_kernel<true><<<zgrid, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs,
                                                             nspin, P.npad, P.ws_z);
     else
-      zbuild_fp64_kernel<false><<<(unsigned)np, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs,
+      zbuild_fp64_kernel<false><<<zgrid, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs,
                                                              nspin, P.npad, P.ws_z);
     NKX_LAUNCH_CHECK();
     ++P.launches;

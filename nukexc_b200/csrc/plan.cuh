@@ -213,6 +213,16 @@ inline int density_width(const Plan &P, int nocc) {
   if (P.tune.dens_n) return P.tune.dens_n;
   return ((nocc + 127) / 128) * 128 >= 1024 ? 128 : 64;
 }
+// CTAs a pair's points are split over (1 to 8) in the kernels that take a CTA
+// of eight warps per (batch, block) pair: while there are fewer than eight an
+// SM, the pairs alone leave SMs with a few warps whose latencies show (one
+// water, 261 pairs: FP64 collocation 59 -> 42 us, Z operands 95 -> 42, pass A
+// 67 -> 45)
+inline unsigned point_split(long pairs, int nsm) {
+  unsigned k = 1;
+  while (k < 8 && pairs * k < 8L * nsm) k *= 2;
+  return k;
+}
 // Units a V output tile's batches are dealt to: the fewest that fill nine
 // tenths of the last wave of `nsm` CTAs, up to four waves (else the best
 // found).  `parts` tiles alone leave SMs idle where a basis has few blocks

@@ -1224,7 +1224,8 @@ __global__ void __launch_bounds__(256) colloc_quantT_kernel(const StoFunc *__res
   load_block_funcs(B, sto, fshell, bshell, bnshell, I, threadIdx.x, blockDim.x);
   __syncthreads();
   const long qrel = blockIdx.x;
-  for (int g = warp; g < kBatch; g += 8) {
+  const int npt = kBatch / gridDim.y, g0 = blockIdx.y * npt;
+  for (int g = g0 + warp; g < g0 + npt; g += 8) {
     double v[4][4];
     __syncwarp();
     block_radials<GRAD>(B, lane, sx[g], sy[g], sz[g], wR[warp], wC[warp]);
@@ -1232,11 +1233,13 @@ __global__ void __launch_bounds__(256) colloc_quantT_kernel(const StoFunc *__res
     block_funcs_eval4<GRAD>(B, lane, sx[g], sy[g], sz[g], wR[warp], wC[warp], v[0], v[1], v[2], v[3]);
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      const unsigned el = max(max(exp_field(v[k][0]), exp_field(v[k][1])), max(exp_field(v[k][2]), exp_field(v[k][3])));
-      report_nonfinite(el == 0x7ffu, nonfinite);
+      // the largest high word of the row (sign cleared); its exponent field
+      // gives the scale, and a non-finite one is reported
+      const unsigned hi = __reduce_max_sync(0xffffffffu, max(max(abs_word(v[k][0]), abs_word(v[k][1])),
+                                                             max(abs_word(v[k][2]), abs_word(v[k][3]))));
       double s;
-      const double inv = warp_inv_pow2_scale(
-          el, fmax(fmax(fabs(v[k][0]), fabs(v[k][1])), fmax(fabs(v[k][2]), fabs(v[k][3]))), s);
+      const double inv = pow2_scale_of_word(hi, s);
+      if (hi >= 0x7fd00000u && lane == 0) atomicOr(nonfinite, 1);
       uint32_t w[4];
       quant4(v[k], inv, w);
       const long pc = qrel * NC + k;
@@ -1935,6 +1938,15 @@ static void launch_i8(MixedState &M, const CUtensorMap &mA, const CUtensorMap &m
 }
 
 
+// pass A of one chunk
+static void launch_colloc_quantT(Plan &P, MixedState &M, const Chunk &c, cudaStream_t s) {
+  const long np = c.p1 - c.p0;
+  auto *kernel = P.gga ? colloc_quantT_kernel<true> : colloc_quantT_kernel<false>;
+  kernel<<<dim3((unsigned)np, point_split(np, M.nsm)), 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell,
+                                                                    P.d_px, P.d_py, P.d_pz, P.d_pair_batch,
+                                                                    P.d_pair_blk, c.p0, M.qphT, M.sphT, P.d_status + 1);
+}
+
 template <bool GRAD>
 static void launch_colloc_z_g(Plan &P, MixedState &M, const Chunk &c, int nzs, int nspin, cudaStream_t s) {
   const unsigned np = (unsigned)(c.p1 - c.p0);
@@ -1987,14 +1999,7 @@ const double *mixed_gradient_chunk(Plan &P, const Chunk &c, int nspin, int nocc,
   const int nc = P.gga ? 4 : 1;
   const long np = c.p1 - c.p0, nb = c.b1 - c.b0;
   if (np > 0) {
-    if (P.gga)
-      colloc_quantT_kernel<true><<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_px,
-                                                              P.d_py, P.d_pz, P.d_pair_batch, P.d_pair_blk, c.p0,
-                                                              M.qphT, M.sphT, P.d_status + 1);
-    else
-      colloc_quantT_kernel<false><<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_px,
-                                                               P.d_py, P.d_pz, P.d_pair_batch, P.d_pair_blk, c.p0,
-                                                               M.qphT, M.sphT, P.d_status + 1);
+    launch_colloc_quantT(P, M, c, s);
     NKX_LAUNCH_CHECK();
     ++P.launches;
   }
@@ -2122,12 +2127,7 @@ void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool 
     const long np = c.p1 - c.p0, nb = c.b1 - c.b0;
     if (np > 0) {
       Tm.begin(ST_COLLOC, s);
-      if (P.gga)
-        colloc_quantT_kernel<true><<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_px, P.d_py, P.d_pz, P.d_pair_batch,
-                                                                P.d_pair_blk, c.p0, M.qphT, M.sphT, P.d_status + 1);
-      else
-        colloc_quantT_kernel<false><<<(unsigned)np, 256, 0, s>>>(P.d_sto, P.d_fshell, P.d_bshell, P.d_bnshell, P.d_px, P.d_py, P.d_pz, P.d_pair_batch,
-                                                                 P.d_pair_blk, c.p0, M.qphT, M.sphT, P.d_status + 1);
+      launch_colloc_quantT(P, M, c, s);
       NKX_LAUNCH_CHECK();
       ++P.launches;
       Tm.end(s);

@@ -327,22 +327,19 @@ __device__ __forceinline__ double inv_pow2_scale(double m, double &scale) {
   return ldexp(1.0, -e);
 }
 
-// The same scale for the largest |v| of a warp, from the biased exponents
-// alone: a normal m with exponent field E has frexp exponent E - 1022, so
-// scale = 2^(E - 1022) and its inverse are built from their bits.  Each lane
-// passes the largest exponent field of its values; all-zero or subnormal
-// (E = 0) and huge (E >= 2045) rows take the general path through `m`.
-__device__ __forceinline__ double warp_inv_pow2_scale(unsigned e_lane, double m_lane, double &scale) {
-  const unsigned e = __reduce_max_sync(0xffffffffu, e_lane);
-  if (e == 0u || e >= 2045u) {
-    double m = m_lane;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    return inv_pow2_scale(m, scale);
-  }
-  scale = __hiloint2double((int)((e + 1u) << 20), 0);
-  return __hiloint2double((int)((2045u - e) << 20), 0);
+// The same scale from the largest high word (sign cleared) of a row's values:
+// a normal m with exponent field E has frexp exponent E - 1022, so the scale
+// 2^(E - 1022) and its inverse are built from their bits.  A row below 2^-958
+// counts as zero and keeps scale 1 (its values become zero digits); one of
+// 2^1022 and more is the caller's to report.
+__device__ __forceinline__ double pow2_scale_of_word(unsigned hi, double &scale) {
+  const unsigned E = hi >> 20;
+  const bool zero = E < 64u;
+  scale = __hiloint2double((int)(zero ? 1023u << 20 : (E + 1u) << 20), 0);
+  return __hiloint2double((int)(zero ? 1023u << 20 : (2045u - E) << 20), 0);
 }
+// high word of |x|
+__device__ __forceinline__ unsigned abs_word(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
 // exponent field of x (sign ignored)
 __device__ __forceinline__ unsigned exp_field(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
 
