@@ -1378,25 +1378,35 @@ __global__ void __launch_bounds__(256, 2) colloc_z_kernel(const StoFunc *__restr
 // this moves about half the bytes (the pass-A digits in, the V digits
 // out).  (Clusters of eight CTAs of 32 points, phi staged in FP64, ran
 // 111 ms per (H2O)64 build against 97.)  Planes s >= nspin (a J build's
-// separate Coulomb plane) are Z = 1/2 vJ phi.  A row field of 0x7fd or more
-// (values of 2^1022 and up, Inf, NaN) is reported in *nonfinite.
+// separate Coulomb plane) are Z = 1/2 vJ phi.  Only planes with a gradient
+// part are staged (ZdShape::NS): the Coulomb plane, and every plane of an LDA
+// build, is one factor per point times phi and is formed again from phi's
+// digits when it is written, which lets two CTAs share an SM where two staged
+// planes allowed one ((H2O)_8 PBE + J: 2.71 -> 2.29 ms; one water LDA: 57 -> 43
+// us).  A row field of 0x7fd or more (values of 2^1022 and up, Inf, NaN)
+// is reported in *nonfinite.
 constexpr int kZdRanks = 4;
-constexpr size_t zdigits_smem(int nz) {
-  return ((size_t)nz * 8 + 4) * (kBatch / kZdRanks) * kBlockF + 8 * (kBatch / kZdRanks);
-}
-template <bool GRAD, int NZ>
-__global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, 2)
+template <bool GRAD, int NZ, bool JP>
+struct ZdShape {
+  static constexpr int NS = GRAD ? NZ - JP : 0;  // staged planes
+  static constexpr size_t kSmem = ((size_t)NS * 8 + 4) * (kBatch / kZdRanks) * kBlockF + 8 * (1 + NZ) * (kBatch / kZdRanks);
+};
+// JP: the last plane is the Coulomb one
+template <bool GRAD, int NZ, bool JP>
+__global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, GRAD || NZ > 1 ? 2 : 3)
     zdigits_kernel(const uint8_t *__restrict__ qphT, const double *__restrict__ sphT,
                    const int *__restrict__ pair_batch, long p0, const double *__restrict__ coef,
-                   const double *__restrict__ vj, int nspin, long npad, uint8_t *__restrict__ qph,
+                   const double *__restrict__ vj, long npad, uint8_t *__restrict__ qph,
                    double *__restrict__ sph, uint8_t *__restrict__ qz, double *__restrict__ szs, int *nonfinite) {
-  constexpr int NC = GRAD ? 4 : 1, nop = 1 + NZ, kPts = kBatch / kZdRanks;
+  constexpr int NC = GRAD ? 4 : 1, nop = 1 + NZ, kPts = kBatch / kZdRanks, NS = ZdShape<GRAD, NZ, JP>::NS;
+  constexpr int nspin = NZ - JP;
   constexpr size_t kPlane = (size_t)kBatch * kBlockF;  // one digit plane of a pair, bytes
-  // dynamic shared memory: Z_s [NZ][kPts][128] FP64, then phi as packed
-  // pass-A digits [kPts][128] and its point scales s_g 2^-30 [kPts]
+  // dynamic shared memory: the staged Z_s [NS][kPts][128] FP64, then phi as
+  // packed pass-A digits [kPts][128], its point scales s_g 2^-30 [kPts] and
+  // the planes' phi coefficients [NZ][kPts]
   extern __shared__ __align__(16) double zst[];
-  uint32_t(*phid)[128] = reinterpret_cast<uint32_t(*)[128]>(zst + (size_t)NZ * kPts * kBlockF);
-  double *phis = reinterpret_cast<double *>(phid + kPts);
+  uint32_t(*phid)[128] = reinterpret_cast<uint32_t(*)[128]>(zst + (size_t)NS * kPts * kBlockF);
+  double *phis = reinterpret_cast<double *>(phid + kPts), *zc = phis + kPts;
   __shared__ uint32_t red[8][nop][128];
   __shared__ uint32_t part[kZdRanks][nop][128];  // every CTA's row fields, pushed by their owners
   __shared__ double inv_s[nop][128];
@@ -1450,7 +1460,9 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, 2)
       }
 #pragma unroll
       for (int s = 0; s < NZ; ++s) {
-        const double cc = s < nspin ? coef[((size_t)s * 4 + c) * npad + gg] : (c == 0 ? 0.5 * vj[gg] : 0.0);
+        if (s >= NS && c > 0) continue;  // a multiple of phi
+        const double cc = s < nspin ? coef[((size_t)s * 4 + c) * npad + gg] : 0.5 * vj[gg];
+        if (s >= NS && (lane & 15) == 0) zc[s * kPts + gl] = cc;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           // Z = c0 phi + ((c1 dx phi + c2 dy phi) + c3 dz phi)
@@ -1467,12 +1479,14 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, 2)
     for (int s = 0; s < NZ; ++s) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        if (GRAD) z[s][k] += t[s][k];
+        if (s < NS) z[s][k] += t[s][k];
         e[1 + s][k] = max(e[1 + s][k], exp_field(z[s][k]));
       }
-      double2 *dst = reinterpret_cast<double2 *>(zst + ((size_t)s * kPts + gl) * kBlockF + f8);
+      if (s < NS) {
+        double2 *dst = reinterpret_cast<double2 *>(zst + ((size_t)s * kPts + gl) * kBlockF + f8);
 #pragma unroll
-      for (int k = 0; k < 8; k += 2) dst[k / 2] = make_double2(z[s][k], z[s][k + 1]);
+        for (int k = 0; k < 8; k += 2) dst[k / 2] = make_double2(z[s][k], z[s][k + 1]);
+      }
     }
   }
   unsigned ez = 0;
@@ -1539,9 +1553,14 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, 2)
           const int gl = 32 * gh + 16 * h + 4 * k4;
           double v[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            v[i] = (o == 0) ? int_to_double(digits_value(phid[gl + i][f])) * phis[gl + i]
-                            : zst[((size_t)(o - 1) * kPts + gl + i) * kBlockF + f];
+          for (int i = 0; i < 4; ++i) {
+            if (o >= 1 && o <= NS) {
+              v[i] = zst[((size_t)(o - 1) * kPts + gl + i) * kBlockF + f];
+            } else {
+              v[i] = int_to_double(digits_value(phid[gl + i][f])) * phis[gl + i];
+              if (o > 0) v[i] *= zc[(o - 1) * kPts + gl + i];
+            }
+          }
           uint32_t ww[4];
           quant4(v, inv, ww);
 #pragma unroll
@@ -1807,6 +1826,12 @@ bool mixed_available(const Plan &) {
   return major == 10 && minor == 0;
 }
 
+template <bool GRAD, int NZ, bool JP>
+static void zdigits_attributes() {
+  NKX_CUDA(cudaFuncSetAttribute(zdigits_kernel<GRAD, NZ, JP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)ZdShape<GRAD, NZ, JP>::kSmem));
+}
+
 static MixedState &mixed_state(Plan &P, int nocc) {
   if (!P.mx_state) {
     MixedState *M = new MixedState();
@@ -1863,10 +1888,12 @@ static MixedState &mixed_state(Plan &P, int nocc) {
     NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_GRAD, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   TcShape<128>::kSmem));
     NKX_CUDA(cudaFuncSetAttribute(zquant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 4 * 128 * 36));
-    NKX_CUDA(cudaFuncSetAttribute(zdigits_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zdigits_smem(1)));
-    NKX_CUDA(cudaFuncSetAttribute(zdigits_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zdigits_smem(2)));
-    NKX_CUDA(cudaFuncSetAttribute(zdigits_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zdigits_smem(1)));
-    NKX_CUDA(cudaFuncSetAttribute(zdigits_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zdigits_smem(2)));
+    zdigits_attributes<true, 1, false>();
+    zdigits_attributes<true, 2, false>();
+    zdigits_attributes<true, 2, true>();
+    zdigits_attributes<false, 1, false>();
+    zdigits_attributes<false, 2, false>();
+    zdigits_attributes<false, 2, true>();
   }
   MixedState &M = *static_cast<MixedState *>(P.mx_state);
   // orbitals pad to 128 so that either density tile width divides them
@@ -2284,20 +2311,23 @@ void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool 
   // (one cluster of four CTAs per pair); nzs <= 2
   auto launch_zdigits = [&](const Chunk &c) {
     const long np = c.p1 - c.p0;
-#define NKX_ZD(G, NZ)                                                                                            \
-  zdigits_kernel<G, NZ><<<(unsigned)np * kZdRanks, 256, zdigits_smem(NZ), s>>>(                               \
-      M.qphT, M.sphT, P.d_pair_batch, c.p0, P.d_coef, P.d_vj, nspin, P.npad, M.qph, M.sph, M.qz, M.sz,         \
-      P.d_status + 1)
+#define NKX_ZD(G, NZ, JP)                                                                                        \
+  zdigits_kernel<G, NZ, JP><<<(unsigned)np * kZdRanks, 256, ZdShape<G, NZ, JP>::kSmem, s>>>(                  \
+      M.qphT, M.sphT, P.d_pair_batch, c.p0, P.d_coef, P.d_vj, P.npad, M.qph, M.sph, M.qz, M.sz, P.d_status + 1)
     if (P.gga) {
       if (nzs == 1)
-        NKX_ZD(true, 1);
+        NKX_ZD(true, 1, false);
+      else if (separateJ)
+        NKX_ZD(true, 2, true);
       else
-        NKX_ZD(true, 2);
+        NKX_ZD(true, 2, false);
     } else {
       if (nzs == 1)
-        NKX_ZD(false, 1);
+        NKX_ZD(false, 1, false);
+      else if (separateJ)
+        NKX_ZD(false, 2, true);
       else
-        NKX_ZD(false, 2);
+        NKX_ZD(false, 2, false);
     }
 #undef NKX_ZD
     NKX_LAUNCH_CHECK();
