@@ -651,15 +651,15 @@ __global__ void aux_rtab_kernel(const AuxShell *__restrict__ shells, int nshell,
 }
 
 // TAB: C R from the mixed build's table (no distance powers or radial
-// factors evaluated here)
-template <int L, bool TAB>
-__global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const AuxGroup *__restrict__ groups, const AuxShell *__restrict__ shells,
+// factors evaluated here); QM: the most shells the group may have
+template <int L, int QM, bool TAB>
+__device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *__restrict__ shells,
                                    const double *__restrict__ px, const double *__restrict__ py,
                                    const double *__restrict__ pz, const double *__restrict__ w,
                                    const double *__restrict__ rho, int nspin, long npad, long slice,
-                                   const float *__restrict__ rtab, int naux, double *__restrict__ y) {
-  constexpr int NM = 2 * L + 1, QM = aux_group_max(L);
-  const AuxGroup G = groups[blockIdx.x];
+                                   const float *__restrict__ rtab, int naux, double *__restrict__ y,
+                                   double (*red)[36]) {
+  constexpr int NM = 2 * L + 1;
   const long g0 = blockIdx.y * slice, g1 = min(npad, g0 + slice);
   double acc[QM][NM];
 #pragma unroll
@@ -718,7 +718,6 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const Aux
   }
   // every sum over its warp first, then all of them over the warps behind
   // one barrier (two barriers a sum took most of a short slice's time)
-  __shared__ double red[8][QM * NM];
 #pragma unroll
   for (int q = 0; q < QM; ++q) {
     if (q >= G.n) break;
@@ -734,6 +733,38 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1) aux_y_group_kernel(const Aux
     double s = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][e];
     y[(size_t)blockIdx.y * naux + shells[G.first + e / NM].first + e % NM] = s;
+  }
+}
+
+// every group of every l in one launch (block x = group): with few centres
+// the launches of single l leave most SMs idle (one water, FP64: 149 us in
+// four launches, 107 in one; (H2O)_8, tables: 790 and 707).  The fixed-count shell loops come in quarters
+// of the l's largest group, so that a group of 6 s shells does not pay for 16.
+template <bool TAB>
+__global__ void __launch_bounds__(256, TAB ? 2 : 1)
+    aux_y_groups_kernel(const AuxGroup *__restrict__ groups, const AuxShell *__restrict__ shells,
+                        const double *__restrict__ px, const double *__restrict__ py, const double *__restrict__ pz,
+                        const double *__restrict__ w, const double *__restrict__ rho, int nspin, long npad, long slice,
+                        const float *__restrict__ rtab, int naux, double *__restrict__ y) {
+  __shared__ double red[8][36];
+  const AuxGroup G = groups[blockIdx.x];
+  auto go = [&](auto l) {
+    constexpr int L = decltype(l)::value, QM = aux_group_max(L);
+    const int quarter = (4 * G.n + QM - 1) / QM;
+    if (quarter <= 1)
+      aux_y_group<L, (QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+    else if (quarter == 2)
+      aux_y_group<L, (2 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+    else if (quarter == 3)
+      aux_y_group<L, (3 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+    else
+      aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+  };
+  switch (G.l) {
+    case 0: return go(std::integral_constant<int, 0>{});
+    case 1: return go(std::integral_constant<int, 1>{});
+    case 2: return go(std::integral_constant<int, 2>{});
+    default: return go(std::integral_constant<int, 3>{});
   }
 }
 
@@ -768,14 +799,16 @@ __device__ __forceinline__ double aux_group_v(const AuxGroup &G, const AuxShell 
   return s;
 }
 
-// y_a = the sum of its slices' shares, in slice order (the fit amplifies
-// rounding differences of y, so the sum does not depend on scheduling)
-__global__ void aux_y_reduce_kernel(const double *__restrict__ part, int nsl, int naux, double *__restrict__ y) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+// y_a = the sum of its slices' shares, in a fixed order (the fit amplifies
+// rounding differences of y, so the sum must not depend on scheduling)
+__global__ void __launch_bounds__(256) aux_y_reduce_kernel(const double *__restrict__ part, int nsl, int naux,
+                                                           double *__restrict__ y) {
+  const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;  // a warp per function
   if (a >= naux) return;
   double s = 0.0;
-  for (int k = 0; k < nsl; ++k) s += part[(size_t)k * naux + a];
-  y[a] = s;
+  for (int k = lane; k < nsl; k += 32) s += part[(size_t)k * naux + a];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) y[a] = s;
 }
 
 // v_g = w_g sum_a c_a V_a(g) over the groups, then the loose shells
@@ -1606,47 +1639,20 @@ static const float *coulomb_table(Plan &P, bool mixed, cudaStream_t s) {
 void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
     const float *rtab = coulomb_table(P, mixed, s);
     // point slices: 64 or one per 4096 points, and more (down to 1024 points
-    // each) where an l has few groups, so that four blocks an SM are in flight
-    // (one water has 3 groups an l: 17 slices kept 51 of 148 SMs busy)
+    // each) where there are few groups, so that four blocks an SM are in flight
     long nsl = std::max<long>(1, std::min<long>(64, (P.npad + 4095) / 4096));
     auto more_slices = [&](int groups) {
       if (groups > 0) nsl = std::max(nsl, std::min((4L * P.nsm + groups - 1) / groups, P.npad / 1024));
     };
-    for (int L = 0; L <= 3; ++L) more_slices(P.h_group_off[L + 1] - P.h_group_off[L]);
+    more_slices(P.nagroup);
     more_slices(P.nloose);
     const long slice = (P.npad + nsl - 1) / nsl;
     if (!P.d_ypart) P.d_ypart = P.alloc<double>((size_t)nsl * P.naux);
-    for (int L = 0; L <= 3; ++L) {
-      const int n = P.h_group_off[L + 1] - P.h_group_off[L];
-      if (n == 0) continue;
-      const AuxGroup *gp = P.d_agroup + P.h_group_off[L];
-      const dim3 gy((unsigned)n, (unsigned)nsl);
-      switch (L) {
-        case 0:
-          if (rtab)
-            aux_y_group_kernel<0, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          else
-            aux_y_group_kernel<0, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          break;
-        case 1:
-          if (rtab)
-            aux_y_group_kernel<1, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          else
-            aux_y_group_kernel<1, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          break;
-        case 2:
-          if (rtab)
-            aux_y_group_kernel<2, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          else
-            aux_y_group_kernel<2, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          break;
-        default:
-          if (rtab)
-            aux_y_group_kernel<3, true><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          else
-            aux_y_group_kernel<3, false><<<gy, 256, 0, s>>>(gp, P.d_ashell, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, P.d_ypart);
-          break;
-      }
+    if (P.nagroup > 0) {
+      auto *kernel = rtab ? aux_y_groups_kernel<true> : aux_y_groups_kernel<false>;
+      kernel<<<dim3((unsigned)P.nagroup, (unsigned)nsl), 256, 0, s>>>(P.d_agroup, P.d_ashell, P.d_px, P.d_py, P.d_pz,
+                                                                      P.d_w, P.d_rho, nspin, P.npad, slice, rtab,
+                                                                      P.naux, P.d_ypart);
       NKX_LAUNCH_CHECK();
       ++P.launches;
     }
@@ -1657,7 +1663,7 @@ void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
       NKX_LAUNCH_CHECK();
       ++P.launches;
     }
-    aux_y_reduce_kernel<<<nblk(P.naux, 128), 128, 0, s>>>(P.d_ypart, (int)nsl, P.naux, P.d_y);
+    aux_y_reduce_kernel<<<nblk(P.naux * 32L, 256), 256, 0, s>>>(P.d_ypart, (int)nsl, P.naux, P.d_y);
     NKX_LAUNCH_CHECK();
     ++P.launches;
 }
