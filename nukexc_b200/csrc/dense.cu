@@ -11,6 +11,7 @@
 #include <functional>
 #include <vector>
 
+#include "dmma.cuh"
 #include "functionals.cuh"
 #include "host_setup.hpp"
 
@@ -31,6 +32,9 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
 };
 
+// fill_collocation / fill_grad_collocation, a thread per element (one water,
+// 68k points: 50 us with gradients; a thread per point and run of functions
+// sharing the radial factor, through a shared tile, took 64)
 __global__ void colloc_dense_kernel(const StoFunc *__restrict__ f, int nbf, const double *__restrict__ pts,
                                     long npts, double *phi, double *gx, double *gy, double *gz) {
   const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -50,48 +54,153 @@ __global__ void colloc_dense_kernel(const StoFunc *__restrict__ f, int nbf, cons
   }
 }
 
-// One warp per point: T_i = sum_mu C(mu,i) phi(mu,g); rho = sum occ_i T_i^2,
-// grad rho = 2 sum occ_i T_i grad T_i (density.hpp:188-255).
-__global__ void density_dense_kernel(int nbf, long npts, const double *__restrict__ phi,
-                                     const double *__restrict__ gx, const double *__restrict__ gy,
-                                     const double *__restrict__ gz, int nocc, const double *__restrict__ C,
-                                     const double *__restrict__ occ, double *rho, double *grad, double *sigma) {
-  const long g = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (g >= npts) return;
-  const double *ph = phi + g * (long)nbf;
-  double r = 0, sx = 0, sy = 0, sz = 0;
-  for (int i = 0; i < nocc; ++i) {
-    const double *ci = C + (long)i * nbf;
-    double t = 0, tx = 0, ty = 0, tz = 0;
-    for (int mu = lane; mu < nbf; mu += 32) {
-      t += ci[mu] * ph[mu];
-      if (gx) {
-        tx += ci[mu] * gx[g * (long)nbf + mu];
-        ty += ci[mu] * gy[g * (long)nbf + mu];
-        tz += ci[mu] * gz[g * (long)nbf + mu];
+// T_i = sum_mu C(mu,i) phi(mu,g); rho = sum occ_i T_i^2, grad rho =
+// 2 sum occ_i T_i grad T_i, sigma = |grad rho|^2 (density.hpp:188-255).  One
+// CTA per 64 points with gradients or 256 without: its 256 (component, point)
+// rows go 32 to a warp as four 8-row DMMA tiles against 8 NN orbitals, 16
+// functions a step through a ring of shared stages (rows padded by four
+// doubles: conflict-free fragments); orbital tiles follow one another and the
+// sums stay in registers.  VEC: every row starts on a 16-byte boundary (even
+// nbf, aligned matrices) and is copied 16 bytes at a time, else 8.
+// Bound: the collocation's HBM reads up to about 16 orbitals, then FP64 (one
+// water with gradients, 5 orbitals: 103 us with a warp per point, 36 now).
+constexpr int kDdK = 16, kDdLd = kDdK + 4, kDdStages = 3;
+template <int NN>
+constexpr int kDdSmem = kDdStages * (256 + 8 * NN) * kDdLd * 8;
+template <bool GRAD, int NN, bool VEC>
+__global__ void __launch_bounds__(256)
+    density_dense_kernel(int nbf, long npts, const double *__restrict__ phi, const double *__restrict__ gx,
+                         const double *__restrict__ gy, const double *__restrict__ gz, int nocc,
+                         const double *__restrict__ C, const double *__restrict__ occ, double *__restrict__ rho,
+                         double *__restrict__ grad, double *__restrict__ sigma) {
+  constexpr int NT = 8 * NN, kStage = (256 + NT) * kDdLd, PTS = GRAD ? 64 : 256;
+  constexpr int W = VEC ? 2 : 1, PARTS = kDdK / W;  // doubles a copy, copies a row
+  extern __shared__ __align__(16) double dsm[];
+  const long g0 = blockIdx.x * (long)PTS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  const int ksteps = (nbf + kDdK - 1) / kDdK, total = ksteps * ((nocc + NT - 1) / NT);
+  auto copy = [&](double *dst, const double *src, bool in) {
+    if constexpr (VEC)
+      cp_async16_fill(dst, src, in);
+    else
+      cp_async8_fill(dst, src, in);
+  };
+  auto issue = [&](int t, int st) {
+    if (t < total) {
+      const int f0 = (t % ksteps) * kDdK, i0 = (t / ksteps) * NT;
+      double *Ps = dsm + st * kStage, *Cs = Ps + 256 * kDdLd;
+#pragma unroll
+      for (int e = threadIdx.x; e < 256 * PARTS; e += 256) {
+        const int row = e / PARTS, part = W * (e % PARTS);
+        // GRAD: row = 32 (point / 8) + 8 comp + point % 8
+        const int c = GRAD ? (row / 8) % 4 : 0;
+        const long g = g0 + (GRAD ? 8 * (row / 32) + row % 8 : row);
+        const double *src = c == 0 ? phi : c == 1 ? gx : c == 2 ? gy : gz;
+        const bool in = g < npts && f0 + part < nbf;
+        copy(Ps + row * kDdLd + part, in ? src + (size_t)g * nbf + f0 + part : src, in);
+      }
+      for (int e = threadIdx.x; e < NT * PARTS; e += 256) {
+        const int row = e / PARTS, part = W * (e % PARTS);
+        const bool in = i0 + row < nocc && f0 + part < nbf;
+        copy(Cs + row * kDdLd + part, in ? C + (size_t)(i0 + row) * nbf + f0 + part : C, in);
       }
     }
-    for (int o = 16; o; o >>= 1) {
-      t += __shfl_xor_sync(0xffffffffu, t, o);
-      tx += __shfl_xor_sync(0xffffffffu, tx, o);
-      ty += __shfl_xor_sync(0xffffffffu, ty, o);
-      tz += __shfl_xor_sync(0xffffffffu, tz, o);
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int st = 0; st < kDdStages - 1; ++st) issue(st, st);
+  double sm[4] = {0.0, 0.0, 0.0, 0.0}, acc[4][NN][2];
+  for (int t = 0; t < total; ++t) {
+    if (t % ksteps == 0) {
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int n = 0; n < NN; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
     }
-    r += occ[i] * t * t;
-    sx += occ[i] * tx * t;
-    sy += occ[i] * ty * t;
-    sz += occ[i] * tz * t;
+    cp_async_wait<kDdStages - 2>();
+    __syncthreads();  // step t is visible; the stage refilled below was read in step t - 1
+    issue(t + kDdStages - 1, (t + kDdStages - 1) % kDdStages);
+    const double *Ps = dsm + (t % kDdStages) * kStage, *Cs = Ps + 256 * kDdLd;
+#pragma unroll
+    for (int k = 0; k < kDdK; k += 4) {
+      double av[4], bv[NN];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) av[m] = Ps[(32 * warp + 8 * m + fr) * kDdLd + k + fk];
+#pragma unroll
+      for (int n = 0; n < NN; ++n) bv[n] = Cs[(8 * n + fr) * kDdLd + k + fk];
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int n = 0; n < NN; ++n) dmma884(acc[m][n], av[m], bv[n]);
+    }
+    if (t % ksteps == ksteps - 1) {
+#pragma unroll
+      for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = (t / ksteps) * NT + 8 * n + 2 * fk + h;
+          const double o = i < nocc ? occ[i] : 0.0;
+#pragma unroll
+          for (int m = 0; m < 4; ++m) sm[m] += o * acc[GRAD ? 0 : m][n][h] * acc[m][n][h];
+        }
+    }
   }
-  if (lane == 0) {
-    rho[g] = r;
+  cp_async_wait<0>();
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    sm[m] += __shfl_xor_sync(0xffffffffu, sm[m], 1);
+    sm[m] += __shfl_xor_sync(0xffffffffu, sm[m], 2);
+  }
+  if (fk != 0) return;
+  if constexpr (GRAD) {
+    const long g = g0 + 8 * warp + fr;
+    if (g >= npts) return;
+    rho[g] = sm[0];
     if (grad) {
-      grad[g] = 2 * sx;
-      grad[npts + g] = 2 * sy;
-      grad[2 * npts + g] = 2 * sz;
+      grad[g] = 2 * sm[1];
+      grad[npts + g] = 2 * sm[2];
+      grad[2 * npts + g] = 2 * sm[3];
     }
-    if (sigma) sigma[g] = 4.0 * (sx * sx + sy * sy + sz * sz);
+    if (sigma) sigma[g] = 4.0 * (sm[1] * sm[1] + sm[2] * sm[2] + sm[3] * sm[3]);
+  } else {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const long g = g0 + 32 * warp + 8 * m + fr;
+      if (g < npts) rho[g] = sm[m];
+    }
   }
+}
+
+template <bool GRAD, int NN, bool VEC>
+static void launch_density_dense_nn(int nbf, long npts, const double *phi, const double *gx, const double *gy,
+                                    const double *gz, int nocc, const double *C, const double *occ, double *rho,
+                                    double *grad, double *sigma, cudaStream_t s) {
+  NKX_CUDA(cudaFuncSetAttribute(density_dense_kernel<GRAD, NN, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kDdSmem<NN>));
+  const int pts = GRAD ? 64 : 256;
+  density_dense_kernel<GRAD, NN, VEC><<<(unsigned)((npts + pts - 1) / pts), 256, kDdSmem<NN>, s>>>(
+      nbf, npts, phi, gx, gy, gz, nocc, C, occ, rho, grad, sigma);
+}
+
+// rho (and, with gx given, grad / sigma where not null) of one spin
+static void launch_density_dense(int nbf, long npts, const double *phi, const double *gx, const double *gy,
+                                 const double *gz, int nocc, const double *C, const double *occ, double *rho,
+                                 double *grad, double *sigma, cudaStream_t s) {
+  bool vec = nbf % 2 == 0;
+  for (const double *q : {phi, gx, gy, gz, C}) vec = vec && ((uintptr_t)q & 15) == 0;
+  auto go = [&](auto g, auto v) {
+    constexpr bool G = decltype(g)::value, V = decltype(v)::value;
+    auto f = nocc <= 8    ? launch_density_dense_nn<G, 1, V>
+             : nocc <= 16 ? launch_density_dense_nn<G, 2, V>
+             : nocc <= 32 ? launch_density_dense_nn<G, 4, V>
+                          : launch_density_dense_nn<G, 8, V>;
+    f(nbf, npts, phi, gx, gy, gz, nocc, C, occ, rho, grad, sigma, s);
+  };
+  if (gx)
+    vec ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+  else
+    vec ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
+  NKX_LAUNCH_CHECK();
 }
 
 // libxc-layout functional evaluation (thread per point)
@@ -122,12 +231,12 @@ __global__ void xc_eval_kernel(XcSpec s, int nspin, long n, const double *rho, c
   }
 }
 
-// Per point: functional of the (spin) densities, energy, and the Z matrix
-// Z(mu, g) = w (1/2 phi vrho + vec . grad phi) (xc_integrals.hpp:486-515,
-// :655-697).  Z holds nspin blocks of nbf x npts.
-__global__ void xc_z_dense_kernel(XcSpec s, bool gga, int nbf, long npts, int nspin, const double *phi,
-                                  const double *gx, const double *gy, const double *gz, const double *w,
-                                  const double *rho, const double *grad, double *Z, double *Eacc) {
+// Per point: functional of the (spin) densities, energy, and the coefficients
+// of Z(mu, g) = w (1/2 phi vrho + vec . grad phi) (xc_integrals.hpp:486-515,
+// :655-697), which take the place of rho (w vrho / 2) and grad rho (w vec).
+__global__ void __launch_bounds__(128) xc_coef_dense_kernel(XcSpec s, bool gga, long npts, int nspin,
+                                                            const double *__restrict__ w, double *rho, double *grad,
+                                                            double *Eacc) {
   const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
   double e = 0.0;
   if (g < npts) {
@@ -160,91 +269,245 @@ __global__ void xc_z_dense_kernel(XcSpec s, bool gga, int nbf, long npts, int ns
       }
     }
     for (int sp = 0; sp < nspin; ++sp) {
-      double *Zs = Z + (size_t)sp * nbf * npts;
-      for (int mu = 0; mu < nbf; ++mu) {
-        const size_t i = (size_t)mu + (size_t)g * nbf;
-        double z = 0.5 * phi[i] * vr[sp];
-        if (gga) z += vec[sp][0] * gx[i] + vec[sp][1] * gy[i] + vec[sp][2] * gz[i];
-        Zs[i] = w[g] * z;
-      }
+      rho[(size_t)sp * npts + g] = 0.5 * w[g] * vr[sp];
+      if (gga)
+        for (int k = 0; k < 3; ++k) grad[(size_t)sp * 3 * npts + k * npts + g] = w[g] * vec[sp][k];
     }
   }
   for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(Eacc, e);
 }
 
+// Z holds nspin blocks of nbf x npts: block (x, spin) walks the rows of
+// kZPts points with the functions contiguous.  Bound: HBM (one water: 164 us
+// with a thread per point walking its row, 13 + 27 now).
+constexpr int kZPts = 64;
+template <bool GGA>
+__global__ void __launch_bounds__(256) xc_z_dense_kernel(int nbf, long npts, const double *__restrict__ phi,
+                                                         const double *__restrict__ gx, const double *__restrict__ gy,
+                                                         const double *__restrict__ gz, const double *__restrict__ c0,
+                                                         const double *__restrict__ ck, double *__restrict__ Z) {
+  __shared__ double cf[GGA ? 4 : 1][kZPts];
+  const long g0 = blockIdx.x * (long)kZPts;
+  const int sp = blockIdx.y, np = (int)min((long)kZPts, npts - g0);
+  for (int e = threadIdx.x; e < (GGA ? 4 : 1) * kZPts; e += 256) {
+    const int k = e / kZPts, p = e % kZPts;
+    if (p < np)
+      cf[k][p] = k == 0 ? c0[(size_t)sp * npts + g0 + p] : ck[((size_t)sp * 3 + k - 1) * npts + g0 + p];
+  }
+  __syncthreads();
+  const int n = np * nbf;
+  const size_t base = (size_t)g0 * nbf;
+  double *Zs = Z + (size_t)sp * nbf * npts;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < n; t += 256) {
+    const int p = t / nbf;
+    double r = cf[0][p] * phi[base + t];
+    if (GGA) r += cf[GGA ? 1 : 0][p] * gx[base + t] + cf[GGA ? 2 : 0][p] * gy[base + t] + cf[GGA ? 3 : 0][p] * gz[base + t];
+    Zs[base + t] = r;
+  }
+}
+
+// the functional and Z of the dense build, from rho and grad in place
+static void launch_xc_z_dense(const XcSpec &sp, bool gga, int nbf, long npts, int nspin, const double *phi,
+                              const double *gx, const double *gy, const double *gz, const double *w, double *rho,
+                              double *grad, double *Z, double *E, cudaStream_t s) {
+  xc_coef_dense_kernel<<<(unsigned)((npts + 127) / 128), 128, 0, s>>>(sp, gga, npts, nspin, w, rho, grad, E);
+  auto *kernel = gga ? xc_z_dense_kernel<true> : xc_z_dense_kernel<false>;
+  kernel<<<dim3((unsigned)((npts + kZPts - 1) / kZPts), nspin), 256, 0, s>>>(nbf, npts, phi, gx, gy, gz, rho, grad, Z);
+  NKX_LAUNCH_CHECK();
+}
+
 // V += Vbar + Vbar^T with Vbar(i,j) = sum_g A(i,g) B(j,g); A, B column-major
 // n x npts (xc_integrals.hpp:148-153 forms Vbar by DGEMM and then adds its
 // transpose).  n is small (the basis) and npts large, so the point range is
 // split over blockIdx.z: each block forms a 64 x 64 tile over its slice of
-// points in registers (4 x 4 per thread, 16-point steps through shared
-// memory) and adds it to V(i,j) and V(j,i) atomically.  V must be zero on
-// entry.
-constexpr int kGemmTile = 64, kGemmK = 16;
-__global__ void __launch_bounds__(256) nt_gemm_sym_kernel(int n, long npts, long kslice, const double *__restrict__ A,
-                                                          const double *__restrict__ B, double *V) {
-  __shared__ double As[kGemmK][kGemmTile + 1], Bs[kGemmK][kGemmTile + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+// points, eight warps of 32 x 16 on DMMA tiles, 32 points a step through a
+// ring of shared stages (rows padded by four doubles), and adds it to V(i,j)
+// and V(j,i) atomically.  V must be zero on entry.  VEC as in
+// density_dense_kernel (one water: 50 us on CUDA-core tiles, 31 now).  With v, B(j,g) is taken times v(g) / 2 (J = Phi
+// diag(v) Phi^T, whose Vbar is symmetric).
+constexpr int kGemmTile = 64, kGemmK = 32, kGemmLd = kGemmTile + 4, kGemmStages = 3;
+constexpr int kGemmStage = 2 * kGemmK * kGemmLd, kGemmSmem = kGemmStages * kGemmStage * 8;
+template <bool VEC, bool SCALE>
+__global__ void __launch_bounds__(256, 2) nt_gemm_sym_kernel(int n, long npts, long kslice, const double *__restrict__ A,
+                                                             const double *__restrict__ B,
+                                                             const double *__restrict__ v, double *V) {
+  extern __shared__ __align__(16) double gsm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
   const int i0 = blockIdx.y * kGemmTile, j0 = blockIdx.x * kGemmTile;
   const long g_lo = blockIdx.z * kslice, g_hi = min(npts, g_lo + kslice);
-  double acc[4][4] = {};
-  for (long g0 = g_lo; g0 < g_hi; g0 += kGemmK) {
-    // 64 rows x 16 points of A and of B: thread t loads rows t % 64, points
-    // t / 64 + 4 e (coalesced along the rows)
-    for (int e = 0; e < 4; ++e) {
-      const int r = threadIdx.x & 63, k = (threadIdx.x >> 6) + 4 * e;
-      const long g = g0 + k;
-      const bool gin = g < g_hi;
-      As[k][r] = (gin && i0 + r < n) ? A[(size_t)(i0 + r) + (size_t)g * n] : 0.0;
-      Bs[k][r] = (gin && j0 + r < n) ? B[(size_t)(j0 + r) + (size_t)g * n] : 0.0;
+  const int total = (int)((g_hi - g_lo + kGemmK - 1) / kGemmK);
+  constexpr int W = VEC ? 2 : 1, PARTS = kGemmTile / W;
+  auto issue = [&](int t, int st) {
+    if (t < total) {
+      double *As = gsm + st * kGemmStage, *Bs = As + kGemmK * kGemmLd;
+#pragma unroll
+      for (int r = 0; r < kGemmK * PARTS / 256; ++r) {
+        const int e = threadIdx.x + 256 * r, k = e / PARTS, part = W * (e % PARTS);
+        const long g = g_lo + (long)t * kGemmK + k;
+        const bool ia = g < g_hi && i0 + part < n, ib = g < g_hi && j0 + part < n;
+        const double *a = ia ? A + (size_t)g * n + i0 + part : A, *b = ib ? B + (size_t)g * n + j0 + part : B;
+        if constexpr (VEC) {
+          cp_async16_fill(As + k * kGemmLd + part, a, ia);
+          cp_async16_fill(Bs + k * kGemmLd + part, b, ib);
+        } else {
+          cp_async8_fill(As + k * kGemmLd + part, a, ia);
+          cp_async8_fill(Bs + k * kGemmLd + part, b, ib);
+        }
+      }
     }
-    __syncthreads();
+    cp_async_commit();
+  };
 #pragma unroll
-    for (int k = 0; k < kGemmK; ++k) {
-      double a[4], b[4];
+  for (int st = 0; st < kGemmStages - 1; ++st) issue(st, st);
+  double acc[4][2][2];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        a[r] = As[k][tx + 16 * r];
-        b[r] = Bs[k][ty + 16 * r];
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  const int r0 = 32 * (warp & 1) + fr, c0 = 16 * (warp >> 1) + fr;
+  for (int t = 0; t < total; ++t) {
+    cp_async_wait<kGemmStages - 2>();
+    __syncthreads();  // step t is visible; the stage refilled below was read in step t - 1
+    issue(t + kGemmStages - 1, (t + kGemmStages - 1) % kGemmStages);
+    const double *As = gsm + (t % kGemmStages) * kGemmStage, *Bs = As + kGemmK * kGemmLd;
+#pragma unroll
+    for (int k = 0; k < kGemmK; k += 4) {
+      double av[4], bv[2];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) av[a] = As[(k + fk) * kGemmLd + r0 + 8 * a];
+#pragma unroll
+      for (int b = 0; b < 2; ++b) bv[b] = Bs[(k + fk) * kGemmLd + c0 + 8 * b];
+      if constexpr (SCALE) {
+        const double h = 0.5 * v[min(g_lo + (long)t * kGemmK + k + fk, npts - 1)];  // rows past g_hi are zero
+#pragma unroll
+        for (int b = 0; b < 2; ++b) bv[b] *= h;
       }
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+        for (int b = 0; b < 2; ++b) dmma884(acc[a][b], av[a], bv[b]);
     }
-    __syncthreads();
   }
+  cp_async_wait<0>();
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * c;
-      if (i < n && j < n) {
-        atomicAdd(&V[(size_t)i + (size_t)j * n], acc[r][c]);
-        atomicAdd(&V[(size_t)j + (size_t)i * n], acc[r][c]);
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = i0 + r0 + 8 * a, j = j0 + 16 * (warp >> 1) + 8 * b + 2 * fk + h;
+        if (i < n && j < n) {
+          atomicAdd(&V[(size_t)i + (size_t)j * n], acc[a][b][h]);
+          atomicAdd(&V[(size_t)j + (size_t)i * n], acc[a][b][h]);
+        }
       }
-    }
 }
 
 // Launch of nt_gemm_sym_kernel for one n x n output (zeroed here): enough
 // point slices to give every SM a couple of blocks.
-static void launch_nt_gemm_sym(int n, long npts, const double *A, const double *B, double *V, cudaStream_t s) {
+static void launch_nt_gemm_sym(int n, long npts, const double *A, const double *B, double *V, cudaStream_t s,
+                               const double *v = nullptr) {
   NKX_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * n * n, s));
   const int nt = (n + kGemmTile - 1) / kGemmTile;
   const long want = std::max<long>(1, (2L * 148 + (long)nt * nt - 1) / ((long)nt * nt));
   const long nsl = std::max<long>(1, std::min<long>(want, (npts + 255) / 256));
   const long kslice = ((npts + nsl - 1) / nsl + kGemmK - 1) / kGemmK * kGemmK;
   const long nz = (npts + kslice - 1) / kslice;
-  nt_gemm_sym_kernel<<<dim3(nt, nt, (unsigned)nz), 256, 0, s>>>(n, npts, kslice, A, B, V);
+  const bool vec = n % 2 == 0 && (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
+  auto *kernel = v ? (vec ? nt_gemm_sym_kernel<true, true> : nt_gemm_sym_kernel<false, true>)
+                   : (vec ? nt_gemm_sym_kernel<true, false> : nt_gemm_sym_kernel<false, false>);
+  NKX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  kernel<<<dim3(nt, nt, (unsigned)nz), 256, kGemmSmem, s>>>(n, npts, kslice, A, B, v, V);
 }
 
-__global__ void potential_dense_kernel(const AuxFunc *__restrict__ f, int naux, const double *__restrict__ pts,
-                                       const double *__restrict__ w, long npts, double *Vw) {
-  const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (idx >= (long)naux * npts) return;
-  const int a = (int)(idx % naux);
-  const long g = idx / naux;
-  Vw[idx] = aux_potential(f[a], pts[3 * g], pts[3 * g + 1], pts[3 * g + 2]) * w[g];
+// The dense table Vw(a, g), functions a contiguous, one CTA per 128
+// points and chunk of at most kDenseF functions.  A thread owns a point and
+// walks every kDenseG-th run of the chunk's functions, so the basis data, the harmonic's branch and
+// the loop bounds are the same for the whole warp, and the functions of a run
+// (one centre, exponent, n and l) share the radial factor; the chunk leaves
+// through a shared tile with the functions contiguous.
+constexpr int kDenseP = 128, kDenseF = 16, kDenseG = 4, kDenseT = kDenseP * kDenseG;
+struct DenseRun {
+  int first, nm;  // functions [first, first + nm)
+};
+struct DenseChunk {
+  int run0, run1, f0, nf;
+};
+
+// Runs of consecutive functions for which same(i, i + 1) holds (at most 15
+// long), and chunks of whole runs
+template <class Same>
+static void dense_runs(int n, Same &&same, std::vector<DenseRun> &runs, std::vector<DenseChunk> &chunks) {
+  for (int i = 0; i < n;) {
+    int e = i + 1;
+    while (e < n && e - i < 15 && same(e - 1, e)) ++e;
+    if (chunks.empty() || chunks.back().nf + (e - i) > kDenseF)
+      chunks.push_back(DenseChunk{(int)runs.size(), (int)runs.size(), i, 0});
+    DenseChunk &c = chunks.back();
+    runs.push_back(DenseRun{i, e - i});
+    c.run1 = (int)runs.size();
+    c.nf += e - i;
+    i = e;
+  }
+}
+
+// the chunk's runs and functions into shared memory
+template <class F>
+__device__ __forceinline__ void dense_load(const F *__restrict__ fn, const DenseRun *__restrict__ runs,
+                                           const DenseChunk &ch, F *sfn, DenseRun *srun) {
+  for (int e = threadIdx.x; e < ch.nf; e += kDenseT) sfn[e] = fn[ch.f0 + e];
+  for (int e = threadIdx.x; e < ch.run1 - ch.run0; e += kDenseT) srun[e] = runs[ch.run0 + e];
+  __syncthreads();
+}
+
+// keeps the compiler from hoisting the products of all harmonics out of a
+// loop over a run's functions (it spilled a few hundred of them)
+__device__ __forceinline__ void opaque(double &x, double &y, double &z) {
+  asm volatile("" : "+d"(x), "+d"(y), "+d"(z));
+}
+
+// one chunk's tile [f][point] to its place in the output
+__device__ __forceinline__ void dense_store(const double *tile, int nf, int f0, int nfun, long g0, int np,
+                                            double *__restrict__ out) {
+  for (int e = threadIdx.x; e < np * nf; e += kDenseT) {
+    const int pt = e / nf, f = e - pt * nf;
+    out[(size_t)(g0 + pt) * nfun + f0 + f] = tile[f * (kDenseP + 1) + pt];
+  }
+}
+
+// Vw(a, g) = V_a(r_g) w_g.  Bound: FP64 issue of the incomplete gamma functions,
+// evaluated once per run and point (one water, 143 functions, 68k points:
+// 311 us with a thread per element, 111 us now).
+__global__ void __launch_bounds__(kDenseT) potential_dense_kernel(const AuxFunc *__restrict__ fn,
+                                                                  const DenseRun *__restrict__ runs,
+                                                                  const DenseChunk *__restrict__ chunks, int naux,
+                                                                  const double *__restrict__ pts,
+                                                                  const double *__restrict__ w, long npts,
+                                                                  double *__restrict__ Vw) {
+  extern __shared__ double dtile[];  // [kDenseF][kDenseP + 1]
+  __shared__ AuxFunc sfn[kDenseF];
+  __shared__ DenseRun srun[kDenseF];
+  const DenseChunk ch = chunks[blockIdx.y];
+  const long g0 = blockIdx.x * (long)kDenseP, g = min(g0 + threadIdx.x % kDenseP, npts - 1);
+  const int np = (int)min((long)kDenseP, npts - g0);
+  const double px = pts[3 * g], py = pts[3 * g + 1], pz = pts[3 * g + 2], wg = w[g];
+  dense_load(fn, runs, ch, sfn, srun);
+  for (int r = threadIdx.x / kDenseP; r < ch.run1 - ch.run0; r += kDenseG) {
+    const int k0 = srun[r].first - ch.f0, nm = srun[r].nm;
+    const AuxFunc &f = sfn[k0];
+    const double dx = px - f.cx, dy = py - f.cy, dz = pz - f.cz;
+    const double R = aux_radial(f, sqrt(dx * dx + dy * dy + dz * dz));
+#pragma unroll 1
+    for (int k = k0; k < k0 + nm; ++k) {
+      double x = dx, y = dy, z = dz;
+      opaque(x, y, z);
+      dtile[k * (kDenseP + 1) + threadIdx.x % kDenseP] = f.C * solid_harmonic(f.l, sfn[k].m, x, y, z) * R * wg;
+    }
+  }
+  __syncthreads();
+  dense_store(dtile, ch.nf, ch.f0, naux, g0, np, Vw);
 }
 
 __global__ void precondition_kernel(int N, const double *S, double *A, double *D) {
@@ -277,6 +540,28 @@ using namespace nkx;
 
 static unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// the runs and chunks of an aux function table, on the device
+struct DenseTable {
+  std::vector<DenseChunk> hchunks;  // filled while hruns is made
+  std::vector<DenseRun> hruns;
+  int nchunk;
+  DevBuf<DenseRun> runs;
+  DevBuf<DenseChunk> chunks;
+  static std::vector<DenseRun> split(const std::vector<AuxFunc> &t, std::vector<DenseChunk> &c) {
+    std::vector<DenseRun> r;
+    dense_runs((int)t.size(), [&](int i, int j) {
+      const AuxFunc &x = t[i], &y = t[j];
+      return x.cx == y.cx && x.cy == y.cy && x.cz == y.cz && x.zeta == y.zeta && x.l == y.l && x.a == y.a;
+    }, r, c);
+    return r;
+  }
+  DenseTable(const std::vector<AuxFunc> &t, cudaStream_t s)
+      : hruns(split(t, hchunks)), nchunk((int)hchunks.size()), runs(hruns.size()), chunks(hchunks.size()) {
+    NKX_CUDA(cudaMemcpyAsync(runs.p, hruns.data(), sizeof(DenseRun) * hruns.size(), cudaMemcpyHostToDevice, s));
+    NKX_CUDA(cudaMemcpyAsync(chunks.p, hchunks.data(), sizeof(DenseChunk) * hchunks.size(), cudaMemcpyHostToDevice, s));
+  }
+};
+
 extern "C" nkx_status nkx_fill_collocation(const nkx_basis *basis, const double *d_points, long npts, double *d_phi,
                                            double *d_gx, double *d_gy, double *d_gz, void *stream) {
   return run_guarded("nkx_fill_collocation", [&] {
@@ -307,9 +592,8 @@ extern "C" nkx_status nkx_density_dense(int nbf, long npts, const double *d_phi,
     NKX_REQUIRE(!(d_grad || d_sigma) || (d_gx && d_gy && d_gz), NKX_ERR_ARG, "gradient output needs grad inputs");
     cudaStream_t s = (cudaStream_t)stream;
     if (npts > 0)
-      density_dense_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(nbf, npts, d_phi, (d_grad || d_sigma) ? d_gx : nullptr,
-                                                                d_gy, d_gz, nocc, d_C, d_occ, d_rho, d_grad, d_sigma);
-    NKX_LAUNCH_CHECK();
+      launch_density_dense(nbf, npts, d_phi, (d_grad || d_sigma) ? d_gx : nullptr, d_gy, d_gz, nocc, d_C, d_occ, d_rho,
+                           d_grad, d_sigma, s);
     NKX_CUDA(cudaStreamSynchronize(s));
   });
 }
@@ -347,15 +631,11 @@ extern "C" nkx_status nkx_xc_dense(int nbf, long npts, const double *d_phi, cons
     cudaStream_t s = (cudaStream_t)stream;
     DevBuf<double> rho((size_t)nspin * npts), grad((size_t)nspin * 3 * npts), Z((size_t)nspin * nbf * npts), Ed(1);
     for (int sp_i = 0; sp_i < nspin; ++sp_i)
-      density_dense_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(
-          nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
-          d_occ + (size_t)sp_i * nocc, rho.p + (size_t)sp_i * npts, gga ? grad.p + (size_t)sp_i * 3 * npts : nullptr,
-          nullptr);
-    NKX_LAUNCH_CHECK();
+      launch_density_dense(nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
+                           d_occ + (size_t)sp_i * nocc, rho.p + (size_t)sp_i * npts,
+                           gga ? grad.p + (size_t)sp_i * 3 * npts : nullptr, nullptr, s);
     NKX_CUDA(cudaMemsetAsync(Ed.p, 0, sizeof(double), s));
-    xc_z_dense_kernel<<<nblk(npts, 128), 128, 0, s>>>(sp, gga, nbf, npts, nspin, d_phi, d_gx, d_gy, d_gz, d_w,
-                                                     rho.p, grad.p, Z.p, Ed.p);
-    NKX_LAUNCH_CHECK();
+    launch_xc_z_dense(sp, gga, nbf, npts, nspin, d_phi, d_gx, d_gy, d_gz, d_w, rho.p, grad.p, Z.p, Ed.p, s);
     for (int sp_i = 0; sp_i < nspin; ++sp_i)
       launch_nt_gemm_sym(nbf, npts, d_phi, Z.p + (size_t)sp_i * nbf * npts, d_V + (size_t)sp_i * nbf * nbf, s);
     NKX_LAUNCH_CHECK();
@@ -372,8 +652,10 @@ extern "C" nkx_status nkx_potential_collocation(const nkx_basis *aux, const doub
     DevBuf<AuxFunc> df(tab.size());
     cudaStream_t s = (cudaStream_t)stream;
     NKX_CUDA(cudaMemcpyAsync(df.p, tab.data(), tab.size() * sizeof(AuxFunc), cudaMemcpyHostToDevice, s));
-    const long tot = (long)aux->nbf * npts;
-    if (tot > 0) potential_dense_kernel<<<nblk(tot, 128), 128, 0, s>>>(df.p, aux->nbf, d_points, d_w, npts, d_Vw);
+    const DenseTable dt(tab, s);
+    if (npts > 0)
+      potential_dense_kernel<<<dim3(nblk(npts, kDenseP), dt.nchunk), kDenseT, kDenseF * (kDenseP + 1) * 8, s>>>(
+          df.p, dt.runs.p, dt.chunks.p, aux->nbf, d_points, d_w, npts, d_Vw);
     NKX_LAUNCH_CHECK();
     NKX_CUDA(cudaStreamSynchronize(s));
   });
@@ -386,6 +668,54 @@ __global__ void scale_columns_kernel(int nbf, long npts, const double *__restric
   if (e < (long)nbf * npts) S[e] = phi[e] * v[e / nbf];
 }
 
+// part[slice][a] = sum over a slice of points of Vw(a, g) rho(g): warp w of a
+// block takes points w, w + 8, .. of the slice, lane l function a0 + l
+// (coulomb.hpp:84-85).  Bound: Vw from HBM (78 MB in 20 us).
+__global__ void __launch_bounds__(256) vw_rho_kernel(int naux, long npts, long slice, const double *__restrict__ Vw,
+                                                     const double *__restrict__ rho, double *__restrict__ part) {
+  __shared__ double red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, a = blockIdx.x * 32 + lane;
+  const long g1 = min(npts, (blockIdx.y + 1) * slice);
+  double s = 0.0;
+  if (a < naux) {
+#pragma unroll 8
+    for (long g = blockIdx.y * slice + warp; g < g1; g += 8) s += Vw[(size_t)g * naux + a] * rho[g];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && a < naux) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += red[w][lane];
+    part[(size_t)blockIdx.y * naux + a] = s;
+  }
+}
+// out(a) = sum_k M(a, k) x(k) over the n columns of M (m x n, column-major;
+// x == nullptr: ones), a warp per row: y from its slices' shares, c = X t
+__global__ void __launch_bounds__(256) rows_dot_kernel(int m, int n, const double *__restrict__ M,
+                                                       const double *__restrict__ x, double *__restrict__ out) {
+  const int a = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (a >= m) return;
+  double s = 0.0;
+#pragma unroll 4
+  for (int k = lane; k < n; k += 32) s += M[(size_t)k * m + a] * (x ? x[k] : 1.0);
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[a] = s;
+}
+// out(j) = sum_a M(a, j) x(a) for the n columns of M (m x n, column-major),
+// a warp per column: t = X^T y, and v = Vw^T c with one column per point
+// (coulomb.hpp:86-95)
+__global__ void __launch_bounds__(256) columns_dot_kernel(int m, long n, const double *__restrict__ M,
+                                                          const double *__restrict__ x, double *__restrict__ out) {
+  const long j = (blockIdx.x * 256L + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (j >= n) return;
+  double s = 0.0;
+#pragma unroll 4
+  for (int a = lane; a < m; a += 32) s += M[(size_t)j * m + a] * x[a];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[j] = s;
+}
+
 extern "C" nkx_status nkx_coulomb_dense(int nbf, int naux, long npts, const double *d_phi, const double *d_Vw,
                                         const double *d_X, int K, int nocc, const double *d_C, const double *d_occ,
                                         double *d_J, void *stream) {
@@ -394,29 +724,20 @@ extern "C" nkx_status nkx_coulomb_dense(int nbf, int naux, long npts, const doub
                     d_occ && d_J,
                 NKX_ERR_ARG, "invalid arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf<double> rho(npts), y(naux), t(K), c(naux), v(npts), S((size_t)nbf * npts);
-    density_dense_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(nbf, npts, d_phi, nullptr, nullptr, nullptr, nocc, d_C,
-                                                              d_occ, rho.p, nullptr, nullptr);
+    // about eight blocks an SM over (32-function tiles) x (slices of 128 points and more)
+    const long na = (naux + 31) / 32, nsl = std::max<long>(1, std::min<long>((8 * 148 + na - 1) / na, npts / 128));
+    const long slice = (npts + nsl - 1) / nsl;
+    DevBuf<double> rho(npts), y(naux), t(K), c(naux), v(npts), part((size_t)nsl * naux);
+    launch_density_dense(nbf, npts, d_phi, nullptr, nullptr, nullptr, nocc, d_C, d_occ, rho.p, nullptr, nullptr, s);
+    vw_rho_kernel<<<dim3((unsigned)na, (unsigned)nsl), 256, 0, s>>>(naux, npts, slice, d_Vw, rho.p, part.p);
+    rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, (int)nsl, part.p, nullptr, y.p);
+    columns_dot_kernel<<<nblk(K * 32L, 256), 256, 0, s>>>(naux, K, d_X, y.p, t.p);
+    rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, K, d_X, t.p, c.p);
+    columns_dot_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(naux, npts, d_Vw, c.p, v.p);
     NKX_LAUNCH_CHECK();
-    cublasHandle_t h;
-    NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
-    cublasSetStream(h, s);
-    const double one = 1.0, zero = 0.0;
-    bool ok = cublasDgemv(h, CUBLAS_OP_N, naux, (int)npts, &one, d_Vw, naux, rho.p, 1, &zero, y.p, 1) ==
-              CUBLAS_STATUS_SUCCESS;
-    ok = ok && cublasDgemv(h, CUBLAS_OP_T, naux, K, &one, d_X, naux, y.p, 1, &zero, t.p, 1) == CUBLAS_STATUS_SUCCESS;
-    ok = ok && cublasDgemv(h, CUBLAS_OP_N, naux, K, &one, d_X, naux, t.p, 1, &zero, c.p, 1) == CUBLAS_STATUS_SUCCESS;
-    ok = ok && cublasDgemv(h, CUBLAS_OP_T, naux, (int)npts, &one, d_Vw, naux, c.p, 1, &zero, v.p, 1) ==
-                   CUBLAS_STATUS_SUCCESS;
-    if (ok) {
-      scale_columns_kernel<<<nblk((long)nbf * npts, 256), 256, 0, s>>>(nbf, npts, d_phi, v.p, S.p);
-      ok = cudaGetLastError() == cudaSuccess;
-    }
-    ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)npts, &one, d_phi, nbf, S.p, nbf, &zero, d_J,
-                           nbf) == CUBLAS_STATUS_SUCCESS;
+    launch_nt_gemm_sym(nbf, npts, d_phi, d_phi, d_J, s, v.p);
+    NKX_LAUNCH_CHECK();
     NKX_CUDA(cudaStreamSynchronize(s));
-    cublasDestroy(h);
-    NKX_REQUIRE(ok, NKX_ERR_CUDA, "cuBLAS call in nkx_coulomb_dense failed");
   });
 }
 
@@ -660,15 +981,11 @@ extern "C" nkx_status nkx_xc_dense_noalloc(int nbf, long npts, const double *d_p
     double *Ed = base, *rho = base + nE, *grad = rho + nrho, *Z = grad + ngrad;
     cudaStream_t s = (cudaStream_t)stream;
     for (int sp_i = 0; sp_i < nspin; ++sp_i)
-      density_dense_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(
-          nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
-          d_occ + (size_t)sp_i * nocc, rho + (size_t)sp_i * npts, gga ? grad + (size_t)sp_i * 3 * npts : nullptr,
-          nullptr);
-    NKX_LAUNCH_CHECK();
+      launch_density_dense(nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
+                           d_occ + (size_t)sp_i * nocc, rho + (size_t)sp_i * npts,
+                           gga ? grad + (size_t)sp_i * 3 * npts : nullptr, nullptr, s);
     NKX_CUDA(cudaMemsetAsync(Ed, 0, sizeof(double), s));  // the array keeps the previous call's sum
-    xc_z_dense_kernel<<<nblk(npts, 128), 128, 0, s>>>(sp, gga, nbf, npts, nspin, d_phi, d_gx, d_gy, d_gz, d_w,
-                                                     rho, grad, Z, Ed);
-    NKX_LAUNCH_CHECK();
+    launch_xc_z_dense(sp, gga, nbf, npts, nspin, d_phi, d_gx, d_gy, d_gz, d_w, rho, grad, Z, Ed, s);
     for (int sp_i = 0; sp_i < nspin; ++sp_i)
       launch_nt_gemm_sym(nbf, npts, d_phi, Z + (size_t)sp_i * nbf * npts, d_V + (size_t)sp_i * nbf * nbf, s);
     NKX_LAUNCH_CHECK();

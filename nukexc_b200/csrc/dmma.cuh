@@ -11,10 +11,15 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
-// the same, or 16 zero bytes when !in (src is then not read)
+// 16 (8) bytes, or zeros when !in (src is then not read)
 __device__ __forceinline__ void cp_async16_fill(void *dst, const void *src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
                "r"(in ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async8_fill(void *dst, const void *src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 8 : 0)
                : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
