@@ -139,7 +139,11 @@ def fill_grad_collocation(basis, points):
 
 
 def _flat_lmat(M):
-    """tensor M[i, j] -> column-major contiguous flat buffer"""
+    """tensor M[i, j] -> column-major contiguous flat buffer (M's own memory
+    where it is one already, as the matrices returned by this module are)"""
+    if isinstance(M, torch.Tensor) and M.dtype == torch.float64 and M.is_cuda \
+            and M.device.index == torch.cuda.current_device() and M.dim() == 2 and M.t().is_contiguous():
+        return M.t().reshape(-1)
     return _dev(M).t().contiguous().reshape(-1)
 
 
@@ -451,9 +455,9 @@ class FockBuilder:
         n = self.info()["npoints"]
         Cc = np.concatenate([np.ascontiguousarray(np.asarray(c, np.float64).T).reshape(-1) for c in C_list])
         oc = np.concatenate([_np(o, np.float64) for o in occ_list])
-        rho = np.zeros(nspin * n)
-        g = np.zeros(3 * nspin * n) if grad else None
-        sg = np.zeros(nspin * n) if grad else None
+        rho = np.empty(nspin * n)
+        g = np.empty(3 * nspin * n) if grad else None
+        sg = np.empty(nspin * n) if grad else None
         s = C.c_void_p(stream) if stream else None
         ptr = lambda a: a.ctypes.data_as(C.c_void_p) if a is not None else None  # noqa: E731
         check(L.lib().nkx_plan_density(self._h, nspin, nocc, ptr(Cc), ptr(oc), L.MEM_HOST, 0, ptr(rho), ptr(g),

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <functional>
+#include <mutex>
 #include <vector>
 
 #include "dmma.cuh"
@@ -19,14 +20,49 @@ namespace nkx {
 
 nkx_status run_guarded(const char *where, const std::function<void()> &fn);
 
+// Workspaces of the dense entry points come from a memory pool of the
+// library's own, one per device, allocated and freed in stream order: a call
+// allocates and frees up to a few hundred megabytes, which took cudaMalloc /
+// cudaFree 1 to 3 ms (and a device-wide synchronisation) against 0.1 to 0.5 ms
+// of kernels.  The pool keeps at most kPoolKeep bytes between calls and gives
+// them back when a plan's allocation fails.
+constexpr uint64_t kPoolKeep = (uint64_t)256 << 20;
+static cudaMemPool_t workspace_pool(int dev, bool create) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[128] = {};
+  NKX_REQUIRE(dev >= 0 && dev < 128, NKX_ERR_ARG, "device ordinal out of range");
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev] && create) {
+    cudaMemPoolProps p{};
+    p.allocType = cudaMemAllocationTypePinned;
+    p.location.type = cudaMemLocationTypeDevice;
+    p.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    NKX_CUDA(cudaMemPoolCreate(&pool, &p));
+    uint64_t keep = kPoolKeep;
+    NKX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    pools[dev] = pool;
+  }
+  return pools[dev];
+}
+void trim_workspace_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  if (cudaMemPool_t pool = workspace_pool(dev, false)) cudaMemPoolTrimTo(pool, 0);
+}
+
 template <class T>
 struct DevBuf {
   T *p = nullptr;
-  explicit DevBuf(size_t n) {
-    if (n) NKX_CUDA(cudaMalloc(&p, n * sizeof(T)));
+  cudaStream_t s;
+  DevBuf(size_t n, cudaStream_t stream) : s(stream) {
+    if (!n) return;
+    int dev = 0;
+    NKX_CUDA(cudaGetDevice(&dev));
+    NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev, true), s));
   }
   ~DevBuf() {
-    if (p) cudaFree(p);
+    if (p) cudaFreeAsync(p, s);
   }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
@@ -556,7 +592,7 @@ struct DenseTable {
     return r;
   }
   DenseTable(const std::vector<AuxFunc> &t, cudaStream_t s)
-      : hruns(split(t, hchunks)), nchunk((int)hchunks.size()), runs(hruns.size()), chunks(hchunks.size()) {
+      : hruns(split(t, hchunks)), nchunk((int)hchunks.size()), runs(hruns.size(), s), chunks(hchunks.size(), s) {
     NKX_CUDA(cudaMemcpyAsync(runs.p, hruns.data(), sizeof(DenseRun) * hruns.size(), cudaMemcpyHostToDevice, s));
     NKX_CUDA(cudaMemcpyAsync(chunks.p, hchunks.data(), sizeof(DenseChunk) * hchunks.size(), cudaMemcpyHostToDevice, s));
   }
@@ -572,8 +608,8 @@ extern "C" nkx_status nkx_fill_collocation(const nkx_basis *basis, const double 
                       abs(basis->m[i]) <= basis->l[i] && basis->zeta[i] > 0,
                   NKX_ERR_UNSUPPORTED, "basis function outside n > l, |m| <= l <= 7, zeta > 0");
     auto tab = make_sto_table(*basis);
-    DevBuf<StoFunc> df(tab.size());
     cudaStream_t s = (cudaStream_t)stream;
+    DevBuf<StoFunc> df(tab.size(), s);
     NKX_CUDA(cudaMemcpyAsync(df.p, tab.data(), tab.size() * sizeof(StoFunc), cudaMemcpyHostToDevice, s));
     const long tot = (long)basis->nbf * npts;
     if (tot > 0) colloc_dense_kernel<<<nblk(tot, 128), 128, 0, s>>>(df.p, basis->nbf, d_points, npts, d_phi, d_gx, d_gy, d_gz);
@@ -629,7 +665,7 @@ extern "C" nkx_status nkx_xc_dense(int nbf, long npts, const double *d_phi, cons
     const bool gga = spec_is_gga(sp);
     NKX_REQUIRE(!gga || (d_gx && d_gy && d_gz), NKX_ERR_ARG, "GGA needs collocation gradients");
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf<double> rho((size_t)nspin * npts), grad((size_t)nspin * 3 * npts), Z((size_t)nspin * nbf * npts), Ed(1);
+    DevBuf<double> rho((size_t)nspin * npts, s), grad((size_t)nspin * 3 * npts, s), Z((size_t)nspin * nbf * npts, s), Ed(1, s);
     for (int sp_i = 0; sp_i < nspin; ++sp_i)
       launch_density_dense(nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
                            d_occ + (size_t)sp_i * nocc, rho.p + (size_t)sp_i * npts,
@@ -649,8 +685,8 @@ extern "C" nkx_status nkx_potential_collocation(const nkx_basis *aux, const doub
   return run_guarded("nkx_potential_collocation", [&] {
     NKX_REQUIRE(aux && aux->nbf > 0 && npts >= 0 && d_points && d_w && d_Vw, NKX_ERR_ARG, "invalid arguments");
     auto tab = make_aux_table(*aux);
-    DevBuf<AuxFunc> df(tab.size());
     cudaStream_t s = (cudaStream_t)stream;
+    DevBuf<AuxFunc> df(tab.size(), s);
     NKX_CUDA(cudaMemcpyAsync(df.p, tab.data(), tab.size() * sizeof(AuxFunc), cudaMemcpyHostToDevice, s));
     const DenseTable dt(tab, s);
     if (npts > 0)
@@ -727,7 +763,7 @@ extern "C" nkx_status nkx_coulomb_dense(int nbf, int naux, long npts, const doub
     // about eight blocks an SM over (32-function tiles) x (slices of 128 points and more)
     const long na = (naux + 31) / 32, nsl = std::max<long>(1, std::min<long>((8 * 148 + na - 1) / na, npts / 128));
     const long slice = (npts + nsl - 1) / nsl;
-    DevBuf<double> rho(npts), y(naux), t(K), c(naux), v(npts), part((size_t)nsl * naux);
+    DevBuf<double> rho(npts, s), y(naux, s), t(K, s), c(naux, s), v(npts, s), part((size_t)nsl * naux, s);
     launch_density_dense(nbf, npts, d_phi, nullptr, nullptr, nullptr, nocc, d_C, d_occ, rho.p, nullptr, nullptr, s);
     vw_rho_kernel<<<dim3((unsigned)na, (unsigned)nsl), 256, 0, s>>>(naux, npts, slice, d_Vw, rho.p, part.p);
     rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, (int)nsl, part.p, nullptr, y.p);
@@ -757,7 +793,7 @@ extern "C" nkx_status nkx_exchange_dense(int nbf, int naux, long npts, const dou
     std::vector<double> occ(nocc);
     NKX_CUDA(cudaMemcpyAsync(occ.data(), d_occ, sizeof(double) * nocc, cudaMemcpyDeviceToHost, s));
     NKX_CUDA(cudaStreamSynchronize(s));
-    DevBuf<double> T((size_t)npts * nocc), B((size_t)nbf * npts), P3((size_t)naux * nbf), Y((size_t)nbf * K);
+    DevBuf<double> T((size_t)npts * nocc, s), B((size_t)nbf * npts, s), P3((size_t)naux * nbf, s), Y((size_t)nbf * K, s);
     cublasHandle_t h;
     NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
     cublasSetStream(h, s);
@@ -814,17 +850,17 @@ extern "C" nkx_status nkx_core_hamiltonian_dense(const nkx_basis *basis, const n
     cudaStream_t s = (cudaStream_t)stream;
     const int nbf = basis->nbf;
     auto tab = make_sto_table(*basis);
-    DevBuf<StoFunc> df(tab.size());
+    DevBuf<StoFunc> df(tab.size(), s);
     NKX_CUDA(cudaMemcpyAsync(df.p, tab.data(), sizeof(StoFunc) * tab.size(), cudaMemcpyHostToDevice, s));
     std::vector<double> zc(mol->natoms);
     for (int a = 0; a < mol->natoms; ++a) zc[a] = mol->Z[a];
-    DevBuf<double> dc(3 * (size_t)mol->natoms), dz(mol->natoms);
+    DevBuf<double> dc(3 * (size_t)mol->natoms, s), dz(mol->natoms, s);
     NKX_CUDA(cudaMemcpyAsync(dc.p, mol->xyz, sizeof(double) * 3 * mol->natoms, cudaMemcpyHostToDevice, s));
     NKX_CUDA(cudaMemcpyAsync(dz.p, zc.data(), sizeof(double) * mol->natoms, cudaMemcpyHostToDevice, s));
     // points in chunks holding 6 nbf x chunk matrices in about 1 GiB
     const long chunk = std::max<long>(256, std::min<long>(npts, ((long)1 << 27) / (6L * nbf)));
-    DevBuf<double> phi((size_t)nbf * chunk), gx((size_t)nbf * chunk), gy((size_t)nbf * chunk),
-        gz((size_t)nbf * chunk), sc((size_t)nbf * chunk), wv(chunk);
+    DevBuf<double> phi((size_t)nbf * chunk, s), gx((size_t)nbf * chunk, s), gy((size_t)nbf * chunk, s),
+        gz((size_t)nbf * chunk, s), sc((size_t)nbf * chunk, s), wv(chunk, s);
     NKX_CUDA(cudaMemsetAsync(d_S, 0, sizeof(double) * nbf * nbf, s));
     NKX_CUDA(cudaMemsetAsync(d_T, 0, sizeof(double) * nbf * nbf, s));
     NKX_CUDA(cudaMemsetAsync(d_V, 0, sizeof(double) * nbf * nbf, s));
@@ -864,8 +900,8 @@ extern "C" nkx_status nkx_half_inverse(int N, const double *d_S, double thr, dou
   return run_guarded("nkx_half_inverse", [&] {
     NKX_REQUIRE(N > 0 && d_S && d_X && K, NKX_ERR_ARG, "invalid arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf<double> A((size_t)N * N), D(N), lam(N);
-    DevBuf<int> info(1);
+    DevBuf<double> A((size_t)N * N, s), D(N, s), lam(N, s);
+    DevBuf<int> info(1, s);
     dim3 tb(16, 16), gb(nblk(N, 16), nblk(N, 16));
     precondition_kernel<<<gb, tb, 0, s>>>(N, d_S, A.p, D.p);
     NKX_LAUNCH_CHECK();
@@ -874,7 +910,7 @@ extern "C" nkx_status nkx_half_inverse(int N, const double *d_S, double thr, dou
     cusolverDnSetStream(h, s);
     int lwork = 0;
     cusolverDnDsyevd_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N, lam.p, &lwork);
-    DevBuf<double> work(lwork > 0 ? lwork : 1);
+    DevBuf<double> work(lwork > 0 ? lwork : 1, s);
     const cusolverStatus_t st =
         cusolverDnDsyevd(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N, lam.p, work.p, lwork, info.p);
     cusolverDnDestroy(h);

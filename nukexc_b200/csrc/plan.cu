@@ -59,6 +59,7 @@ nkx_status run_guarded(const char *where, const std::function<void()> &fn) {
   }
 }
 
+void trim_workspace_pool();  // dense.cu
 XcSpec make_spec(const nkx_plan_options *o);
 bool spec_is_gga(const XcSpec &s);
 
@@ -66,7 +67,12 @@ template <class T>
 static T *dalloc(size_t n) {
   T *p = nullptr;
   if (n == 0) return nullptr;
-  const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    trim_workspace_pool();  // give back what the dense entry points keep
+    e = cudaMalloc(&p, n * sizeof(T));
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     throw Error{NKX_ERR_ALLOC, "cudaMalloc of " + std::to_string(n * sizeof(T)) + " bytes failed"};
@@ -1021,6 +1027,8 @@ Plan::~Plan() {
   if (cublas) cublasDestroy((cublasHandle_t)cublas);
   if (cusolver) cusolverDnDestroy((cusolverDnHandle_t)cusolver);
   for (auto &e : ev) cudaEventDestroy(e);
+  for (auto &e : ev_pool) cudaEventDestroy(e);
+  cudaFreeHost(h_result);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -1485,8 +1493,9 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
   P.d_coef = P.alloc<double>(8 * P.npad);
   P.d_vj = P.alloc<double>(P.npad);
   P.d_V = P.alloc<double>(3 * (size_t)P.nbf_pad * P.nbf_pad);
-  P.d_E = P.alloc<double>(1);
-  P.d_status = P.alloc<int>(2);
+  P.d_E = P.alloc<double>(2);
+  P.d_status = reinterpret_cast<int *>(P.d_E + 1);
+  NKX_CUDA(cudaMallocHost(&P.h_result, sizeof(Plan::Result)));
   NKX_CUDA(cudaMemset(P.d_status, 0, sizeof(int) * 2));
   NKX_CUDA(cudaMemset(P.d_rho, 0, sizeof(double) * 2 * P.npad));
   NKX_CUDA(cudaMemset(P.d_grad, 0, sizeof(double) * 6 * P.npad));
@@ -1911,14 +1920,9 @@ static void fock_build_once(Plan &P, int precision, int nspin, int nocc, const d
   const bool separateJ = needJ && !fuse_j && J;
   cudaStream_t s = user ? user : P.stream;
   P.launches = 0;
-  StageTimer T;
+  StageTimer T(P);
   T.on = !capture_only;
-  cudaEvent_t t0 = nullptr, t1 = nullptr;
-  if (!capture_only) {
-    NKX_CUDA(cudaEventCreate(&t0));
-    NKX_CUDA(cudaEventCreate(&t1));
-    NKX_CUDA(cudaEventRecord(t0, s));
-  }
+  if (!capture_only) NKX_CUDA(cudaEventRecord(P.ev[0], s));
   P.phase1_done = false;
   if (phase == 2) {
     NKX_CUDA(cudaMemcpyAsync(P.d_y, y, sizeof(double) * P.naux,
@@ -1938,12 +1942,9 @@ static void fock_build_once(Plan &P, int precision, int nspin, int nocc, const d
   if (phase == 1) {
     NKX_CUDA(cudaMemcpyAsync(y, P.d_y, sizeof(double) * P.naux,
                              mem == NKX_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, s));
-    int status[2] = {0, 0};
-    NKX_CUDA(cudaMemcpyAsync(status, P.d_status, sizeof(status), cudaMemcpyDeviceToHost, s));
-    NKX_CUDA(cudaEventRecord(t1, s));
+    NKX_CUDA(cudaMemcpyAsync(P.h_result, P.d_E, sizeof(Plan::Result), cudaMemcpyDeviceToHost, s));
     NKX_CUDA(cudaStreamSynchronize(s));
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
+    const int *status = P.h_result->status;
     NKX_REQUIRE(status[0] == 0, NKX_ERR_TIMEOUT, "a tensor-core kernel wait gave up in phase 1");
     NKX_REQUIRE(status[1] == 0, NKX_ERR_NUMERIC, "non-finite value in the orbitals, occupations or an operand");
     P.phase1_done = true;
@@ -1977,11 +1978,11 @@ static void fock_build_once(Plan &P, int precision, int nspin, int nocc, const d
     if (V) NKX_CUDA(cudaMemcpyAsync(V, dst, sizeof(double) * nspin * nn, cudaMemcpyDeviceToHost, s));
     if (separateJ) NKX_CUDA(cudaMemcpyAsync(J, dst + nspin * nn, sizeof(double) * nn, cudaMemcpyDeviceToHost, s));
   }
-  NKX_CUDA(cudaMemcpyAsync(E, P.d_E, sizeof(double), cudaMemcpyDeviceToHost, s));
-  int status[2] = {0, 0};
-  NKX_CUDA(cudaMemcpyAsync(status, P.d_status, sizeof(status), cudaMemcpyDeviceToHost, s));
-  NKX_CUDA(cudaEventRecord(t1, s));
+  NKX_CUDA(cudaMemcpyAsync(P.h_result, P.d_E, sizeof(Plan::Result), cudaMemcpyDeviceToHost, s));
+  NKX_CUDA(cudaEventRecord(P.ev[1], s));
   NKX_CUDA(cudaStreamSynchronize(s));
+  *E = P.h_result->E;
+  const int *status = P.h_result->status;
   float st[6];
   T.collect(st);
   P.last.colloc_ms = st[ST_COLLOC];
@@ -1990,10 +1991,8 @@ static void fock_build_once(Plan &P, int precision, int nspin, int nocc, const d
   P.last.coulomb_ms = st[ST_COULOMB];
   P.last.zbuild_ms = st[ST_ZBUILD];
   P.last.vgemm_ms = st[ST_VGEMM];
-  cudaEventElapsedTime(&P.last.total_ms, t0, t1);
+  cudaEventElapsedTime(&P.last.total_ms, P.ev[0], P.ev[1]);
   P.last.launches = P.launches;
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
   P.last_nspin = nspin;
   NKX_REQUIRE(status[0] == 0, NKX_ERR_TIMEOUT,
               "a tensor-core kernel wait gave up (wait code " + std::to_string(status[0]) + "); outputs are invalid");
@@ -2080,26 +2079,21 @@ static void fock_build_graph(Plan &P, int precision, int nspin, int nocc, const 
   // replay
   cudaStream_t s = user ? user : P.stream;
   const size_t nn = (size_t)P.nbf * P.nbf;
-  cudaEvent_t t0, t1;
-  NKX_CUDA(cudaEventCreate(&t0));
-  NKX_CUDA(cudaEventCreate(&t1));
-  NKX_CUDA(cudaEventRecord(t0, s));
+  NKX_CUDA(cudaEventRecord(P.ev[0], s));
   NKX_CUDA(cudaMemcpyAsync(g->C, C, sizeof(double) * nspin * nocc * P.nbf, cudaMemcpyDeviceToDevice, s));
   NKX_CUDA(cudaMemcpyAsync(g->occ, occ, sizeof(double) * nspin * nocc, cudaMemcpyDeviceToDevice, s));
   NKX_CUDA(cudaGraphLaunch(g->exec, s));
   if (V) NKX_CUDA(cudaMemcpyAsync(V, g->V, sizeof(double) * nspin * nn, cudaMemcpyDeviceToDevice, s));
   if (J) NKX_CUDA(cudaMemcpyAsync(J, g->J, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
-  NKX_CUDA(cudaMemcpyAsync(E, P.d_E, sizeof(double), cudaMemcpyDeviceToHost, s));
-  int status[2] = {0, 0};
-  NKX_CUDA(cudaMemcpyAsync(status, P.d_status, sizeof(status), cudaMemcpyDeviceToHost, s));
-  NKX_CUDA(cudaEventRecord(t1, s));
+  NKX_CUDA(cudaMemcpyAsync(P.h_result, P.d_E, sizeof(Plan::Result), cudaMemcpyDeviceToHost, s));
+  NKX_CUDA(cudaEventRecord(P.ev[1], s));
   NKX_CUDA(cudaStreamSynchronize(s));
+  *E = P.h_result->E;
+  const int *status = P.h_result->status;
   P.last = nkx_build_timing{};
-  cudaEventElapsedTime(&P.last.total_ms, t0, t1);
+  cudaEventElapsedTime(&P.last.total_ms, P.ev[0], P.ev[1]);
   P.last.launches = g->launches;
   P.last_nspin = nspin;
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
   ++P.graph_replays;
   NKX_REQUIRE(status[0] == 0, NKX_ERR_TIMEOUT, "a tensor-core kernel wait gave up; outputs are invalid");
   NKX_REQUIRE(status[1] == 0 && std::isfinite(*E), NKX_ERR_NUMERIC,
@@ -2320,7 +2314,7 @@ NKX_API nkx_status nkx_plan_density(nkx_plan *plan, int nspin, int nocc, const d
     // the gradient needs the gradient collocation whatever the functional
     const bool gga = P.gga;
     P.gga = grad || sigma;
-    StageTimer T;
+    StageTimer T(P);
     try {
       fp64_density_pass(P, nspin, nocc, s, T);
     } catch (...) {

@@ -42,6 +42,8 @@ struct Plan {
   int device = 0, nsm = 148;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
+  std::vector<cudaEvent_t> ev_pool;  // stage events, made on first use and kept
+  size_t ev_used = 0;
   std::vector<void *> allocs;
   void *cublas = nullptr, *cusolver = nullptr;
 
@@ -125,6 +127,12 @@ struct Plan {
   // build status words, zeroed by every build: [0] code of the first
   // tensor-core wait that gave up, [1] non-finite input or operand seen
   int *d_status = nullptr;
+  // E_xc and the status words lie together on the device and come back in
+  // one copy to pinned memory
+  struct Result {
+    double E;
+    int status[2];
+  } *h_result = nullptr;
   // limit of the device waits that may be abandoned (nkx_plan_set_wait_limit)
   unsigned long long wait_ns = 2000000000ull;
   int stall_test = 0;  // tests of the error path: tensor-core kernels wait on a barrier nothing completes
@@ -154,30 +162,31 @@ void fock_build(Plan &P, int precision, int nspin, int nocc, const double *C, co
                 double *E, double *V, double *J, cudaStream_t user, int phase = 0, double *y = nullptr);
 void destroy_mixed_state(void *p);
 
-// Accumulates CUDA-event time per build stage.
+// Accumulates CUDA-event time per build stage, with the plan's events.
 struct StageTimer {
+  Plan &P;
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
   cudaEvent_t begin_ev = nullptr;
   int cur = -1;
   bool on = true;  // off while a build is recorded into a CUDA graph
-  ~StageTimer() {
-    for (auto &m : marks) {
-      cudaEventDestroy(m.second.first);
-      cudaEventDestroy(m.second.second);
+  explicit StageTimer(Plan &plan) : P(plan) { P.ev_used = 0; }
+  cudaEvent_t next() {
+    if (P.ev_used == P.ev_pool.size()) {
+      cudaEvent_t e;
+      NKX_CUDA(cudaEventCreate(&e));
+      P.ev_pool.push_back(e);
     }
+    return P.ev_pool[P.ev_used++];
   }
   void begin(int stage, cudaStream_t s) {
     if (!on) return;
-    cudaEvent_t e;
-    NKX_CUDA(cudaEventCreate(&e));
-    NKX_CUDA(cudaEventRecord(e, s));
-    begin_ev = e;
+    begin_ev = next();
+    NKX_CUDA(cudaEventRecord(begin_ev, s));
     cur = stage;
   }
   void end(cudaStream_t s) {
     if (!on) return;
-    cudaEvent_t e;
-    NKX_CUDA(cudaEventCreate(&e));
+    const cudaEvent_t e = next();
     NKX_CUDA(cudaEventRecord(e, s));
     marks.push_back({cur, {begin_ev, e}});
   }
