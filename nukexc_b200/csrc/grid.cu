@@ -29,8 +29,8 @@ __device__ __forceinline__ double dist3(const double *a, const double *b) {
 
 constexpr int kBeckeList = 128;
 
-// The weight of one point by its thread alone, for points with more candidate
-// atoms than becke_kernel's list holds.  With the Laqua clamp R_ij = min(|A_i-A_j|, Rc)
+// One thread per point, for molecules of more than kBeckeCap atoms.  With the
+// Laqua clamp R_ij = min(|A_i-A_j|, Rc)
 // (partitioning.hpp:134-148) the cell functions are exactly 0 or 1 far from
 // the point: every atom with r_i >= r_min + Rc has P_i = 0 (its factor
 // against the nearest atom is s(1) = 0), and in P_i of the others every atom
@@ -39,9 +39,12 @@ constexpr int kBeckeList = 128;
 // same products and sums as the full O(N_atoms^2) loop of
 // partition_becke_team (partitioning.hpp:166-212).  Rc <= 0 selects the
 // unclamped original (partition_becke, partitioning.hpp:63-120) without
-// screening.  Returns P_owner / sum_i P_i.
-__device__ __noinline__ double becke_point(const double *__restrict__ centers, int natoms, const double *p, int own,
-                                           double Rc) {
+// screening.
+__global__ void becke_thread_kernel(const double *__restrict__ centers, int natoms, const double *__restrict__ pts,
+                                    const int *__restrict__ owner, long npts, double *__restrict__ w, double Rc) {
+  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (g >= npts) return;
+  const double *p = pts + 3 * g;
   const bool clamp = Rc > 0.0;
   double rmin = 1e300;
   for (int i = 0; i < natoms; ++i) rmin = fmin(rmin, dist3(p, centers + 3 * i));
@@ -60,6 +63,7 @@ __device__ __noinline__ double becke_point(const double *__restrict__ centers, i
       }
     }
   }
+  const int own = owner[g];
   double norm = 0.0, pown = 0.0;
   if (full) {
     // with the clamp, factors of atoms j with r_j >= r_i + Rc are 1 (mu <= -1
@@ -96,7 +100,7 @@ __device__ __noinline__ double becke_point(const double *__restrict__ centers, i
       norm += P;
     }
   }
-  return pown / norm;
+  w[g] *= pown / norm;
 }
 
 // Becke weights, one warp per 32 points (a point per lane).  The same exact
@@ -111,15 +115,16 @@ __device__ __noinline__ double becke_point(const double *__restrict__ centers, i
 // Bound: FP64 issue of the pair loop (about 20 instructions a pair).
 // (H2O)_16, 1.09 M points: 5.05 ms with a thread per point (distances and
 // R_ij recomputed per pair, lists in local memory), 1.63 ms now.  The list
-// holds `cap` atoms, chosen at launch: all of them up to kBeckeCap (36 KB a
-// warp, six warps an SM), beyond which a warp that overflows falls back to
-// becke_point.
+// has room for every atom, up to kBeckeCap (37 KB a warp, six warps an SM):
+// 144 atoms, 1.35 M points: 12.6 ms against 20.7; at 192 the points of a warp,
+// all round their owner, share few of their candidates, and with lists of 144
+// (the others by a thread each) 1.80 M points took 40.8 ms against 33.3.
 constexpr int kBeckeCap = 144;
 __global__ void __launch_bounds__(32) becke_kernel(const double *__restrict__ centers, int natoms,
                                                    const double *__restrict__ pts, const int *__restrict__ owner,
-                                                   long npts, double *__restrict__ w, double clamp, int cap) {
-  extern __shared__ double rsm[];  // [cap][32] distances, then the atoms' indices [cap]
-  int *list = reinterpret_cast<int *>(rsm + (size_t)cap * 32);
+                                                   long npts, double *__restrict__ w, double clamp) {
+  extern __shared__ double rsm[];  // [natoms][32] distances, then the atoms' indices [natoms]
+  int *list = reinterpret_cast<int *>(rsm + (size_t)natoms * 32);
   const int lane = threadIdx.x;
   const long g = blockIdx.x * 32L + lane;
   const bool in = g < npts;
@@ -141,15 +146,9 @@ __global__ void __launch_bounds__(32) becke_kernel(const double *__restrict__ ce
   for (int j = 0; j < natoms; ++j) {
     const double r = dist3(pt, centers + 3 * j);
     if (!__any_sync(0xffffffffu, live && r < lim)) continue;
-    if (nl < cap) {
-      rsm[nl * 32 + lane] = r;
-      if (lane == 0) list[nl] = j;
-    }
+    rsm[nl * 32 + lane] = r;
+    if (lane == 0) list[nl] = j;
     ++nl;
-  }
-  if (nl > cap) {
-    if (live) w[g] *= becke_point(centers, natoms, pt, own, clamp);
-    return;
   }
   __syncwarp();
   double norm = 0.0, pown = 0.0;
@@ -182,9 +181,14 @@ __global__ void __launch_bounds__(32) becke_kernel(const double *__restrict__ ce
 void launch_becke(const double *d_centers, int natoms, const double *d_pts, const int *d_owner, long npts,
                   double *d_w, double clamp, cudaStream_t s) {
   if (npts <= 0) return;
-  const int cap = std::min(natoms, kBeckeCap);
-  const size_t smem = (size_t)cap * (32 * sizeof(double) + sizeof(int));
-  becke_kernel<<<(unsigned)((npts + 31) / 32), 32, smem, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w, clamp, cap);
+  if (natoms <= kBeckeCap) {
+    const size_t smem = (size_t)natoms * (32 * sizeof(double) + sizeof(int));
+    becke_kernel<<<(unsigned)((npts + 31) / 32), 32, smem, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w, clamp);
+  } else {
+    const int T = 128;
+    becke_thread_kernel<<<(unsigned)((npts + T - 1) / T), T, 0, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w,
+                                                                    clamp);
+  }
   NKX_LAUNCH_CHECK();
 }
 

@@ -1,5 +1,5 @@
 """Becke weights where the warp's atom list can go wrong: one atom, lists of
-exactly and just over 32 atoms, more candidates than the list holds (the
+exactly and just over 32 atoms, more atoms than the list holds (the
 per-thread path), the unclamped original, points far outside, and owners that
 change inside a warp -- against the oracle's full loops (1e-13 absolute on
 weights of at most 1)."""
