@@ -1220,6 +1220,81 @@ void plan_chunks(Plan &P, long maxp) {
   P.ws_phi = P.alloc<double>(std::max<long>(1, P.max_chunk_pairs) * 4 * tile);
 }
 
+static double box_distance2(const double *c, const double *lo, const double *hi) {
+  double d2 = 0.0;
+  for (int d = 0; d < 3; ++d) {
+    const double e = c[d] < lo[d] ? lo[d] - c[d] : (c[d] > hi[d] ? c[d] - hi[d] : 0.0);
+    d2 += e * e;
+  }
+  return d2;
+}
+
+// Functions of one atom reach very differently far (zeta 0.5 to 26: 46 to 1
+// bohr at 1e-10), and a 128-function block is significant where any of its
+// functions is, so blocks cut along the Morton order of the centres are
+// significant almost everywhere.  This splits the order at a cutoff radius --
+// the far-reaching functions first, then the others, each in the given
+// order -- or sorts it by radius, if the blocks significant in a sample of
+// batches then cost less: V takes n^2 tile products of a batch with n blocks,
+// the other passes about kLinear times n ((H2O)_64 PBE: 37 ns a product, 0.87
+// us a pair).  Blocks of like reach are screened with radii of a tolerance
+// 1e-6 times the caller's, so that no term above FP64 rounding is dropped that
+// the mixed blocks would have kept; the gain of three per cent asked for
+// counts that.  On a change `order` and the radii `cut` are replaced.
+// ((H2O)_64: 24 -> 22.2 blocks a batch, 576 -> 493 products; 624 -> 567 ms per
+// build.)
+static void group_by_reach(const nkx_basis &prim, double tol, long nbatch, const std::vector<double> &blo,
+                           const std::vector<double> &bhi, std::vector<int> &order, std::vector<double> &cut) {
+  if (tol < 1e-280) return;
+  constexpr double kLinear = 23.0;
+  const int nbf = prim.nbf, nblk = (nbf + kBlockF - 1) / kBlockF;
+  const auto far = make_cutoffs(prim, 1e-6 * tol);
+  const long ns = std::min<long>(nbatch, 256);
+  std::vector<char> sig((size_t)ns * nbf), sig0((size_t)ns * nbf);
+#pragma omp parallel for schedule(static)
+  for (long k = 0; k < ns; ++k) {
+    const long b = ns > 1 ? k * (nbatch - 1) / (ns - 1) : 0;
+    for (int f = 0; f < nbf; ++f) {
+      const double d2 = box_distance2(&prim.center[3 * f], &blo[3 * b], &bhi[3 * b]);
+      sig[k * nbf + f] = d2 <= far[f] * far[f];
+      sig0[k * nbf + f] = d2 <= cut[f] * cut[f];
+    }
+  }
+  auto cost = [&](const std::vector<int> &o, const std::vector<char> &s) {
+    double c = 0.0;
+    for (long k = 0; k < ns; ++k) {
+      long n = 0;
+      for (int I = 0; I < nblk; ++I) {
+        bool any = false;
+        for (int p = I * kBlockF; p < std::min(nbf, (I + 1) * kBlockF) && !any; ++p) any = s[k * nbf + o[p]];
+        n += any;
+      }
+      c += (double)n * n + kLinear * n;
+    }
+    return c;
+  };
+  // the radii that occur, at most 24 of them
+  std::vector<double> radii(far);
+  std::sort(radii.begin(), radii.end());
+  radii.erase(std::unique(radii.begin(), radii.end(), [](double x, double y) { return y - x < 1e-9 * y; }),
+              radii.end());
+  const long nr = (long)radii.size(), nc = std::min<long>(nr - 1, 24);
+  std::vector<std::vector<int>> cand(nc + 1, order);
+  for (long i = 0; i < nc; ++i) {
+    const double r = radii[i * (nr - 1) / nc] * (1.0 + 1e-8);
+    std::stable_partition(cand[i].begin(), cand[i].end(), [&](int f) { return far[f] > r; });
+  }
+  std::stable_sort(cand[nc].begin(), cand[nc].end(), [&](int x, int y) { return far[x] > far[y]; });
+  std::vector<double> costs(nc + 1);
+#pragma omp parallel for schedule(dynamic)
+  for (long i = 0; i <= nc; ++i) costs[i] = cost(cand[i], sig);
+  const long best = std::min_element(costs.begin(), costs.end()) - costs.begin();
+  if (costs[best] < 0.97 * cost(order, sig0)) {
+    order = cand[best];
+    cut = far;
+  }
+}
+
 static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, const nkx_basis *aux, long npoints,
                        const double *xyz, const double *w, const int *owner, const nkx_plan_options *opts) {
   NKX_REQUIRE(prim && prim->nbf > 0 && npoints > 0 && xyz && w && opts, NKX_ERR_ARG, "invalid arguments");
@@ -1303,6 +1378,19 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
     for (const Run &r : runs)
       for (int i = 0; i < r.n; ++i) order[k++] = r.first + i;
   }
+  const double tol = opts->screen_tol > 0 ? opts->screen_tol : 1e-10;
+  auto cut = make_cutoffs(*prim, tol);
+  // bounding boxes of the batches
+  std::vector<double> blo(3 * (size_t)P.nbatch), bhi(3 * (size_t)P.nbatch);
+#pragma omp parallel for schedule(static)
+  for (long b = 0; b < P.nbatch; ++b)
+    for (int d = 0; d < 3; ++d) {
+      const std::vector<double> &h = d == 0 ? hx : d == 1 ? hy : hz;
+      const auto mm = std::minmax_element(h.begin() + b * kBatch, h.begin() + (b + 1) * kBatch);
+      blo[3 * b + d] = *mm.first;
+      bhi[3 * b + d] = *mm.second;
+    }
+  if (P.nblk > 1) group_by_reach(*prim, tol, P.nbatch, blo, bhi, order, cut);
   std::vector<StoFunc> tab(P.nbf_pad);
   P.h_fperm.assign(P.nbf_pad, -1);
   std::vector<int> finv(std::max(1, P.nbf), 0);
@@ -1397,8 +1485,6 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
   NKX_CUDA(cudaMemcpy(P.d_fperm, P.h_fperm.data(), sizeof(int) * P.nbf_pad, cudaMemcpyHostToDevice));
   P.d_finv = P.alloc<int>(finv.size());
   NKX_CUDA(cudaMemcpy(P.d_finv, finv.data(), sizeof(int) * finv.size(), cudaMemcpyHostToDevice));
-  const double tol = opts->screen_tol > 0 ? opts->screen_tol : 1e-10;
-  auto cut = make_cutoffs(*prim, tol);
 
   // --- screening: block I is significant for batch b if any function's
   // cutoff sphere meets the batch bounding box (octree.hpp:331-366)
@@ -1406,41 +1492,27 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
   P.h_pair_off.assign(P.nbatch + 1, 0);
   // per block, the box holding every function's cutoff sphere: a block whose
   // box misses the batch box has no significant function there
-  std::vector<double> blo(3 * (size_t)P.nblk, 1e300), bhi(3 * (size_t)P.nblk, -1e300);
+  std::vector<double> flo(3 * (size_t)P.nblk, 1e300), fhi(3 * (size_t)P.nblk, -1e300);
   for (int q = 0; q < P.nbf_pad; ++q) {
     const int f = P.h_fperm[q], I = q / kBlockF;
     if (f < 0) continue;
     for (int d = 0; d < 3; ++d) {
-      blo[3 * I + d] = std::min(blo[3 * I + d], prim->center[3 * f + d] - cut[f]);
-      bhi[3 * I + d] = std::max(bhi[3 * I + d], prim->center[3 * f + d] + cut[f]);
+      flo[3 * I + d] = std::min(flo[3 * I + d], prim->center[3 * f + d] - cut[f]);
+      fhi[3 * I + d] = std::max(fhi[3 * I + d], prim->center[3 * f + d] + cut[f]);
     }
   }
 #pragma omp parallel for schedule(dynamic, 64)
   for (long b = 0; b < P.nbatch; ++b) {
-    double bl[3] = {1e300, 1e300, 1e300}, bh[3] = {-1e300, -1e300, -1e300};
-    for (int g = 0; g < kBatch; ++g) {
-      const long p = b * kBatch + g;
-      const double v[3] = {hx[p], hy[p], hz[p]};
-      for (int d = 0; d < 3; ++d) {
-        bl[d] = std::min(bl[d], v[d]);
-        bh[d] = std::max(bh[d], v[d]);
-      }
-    }
+    const double *bl = &blo[3 * b], *bh = &bhi[3 * b];
     for (int I = 0; I < P.nblk; ++I) {
       bool near = true;
-      for (int d = 0; d < 3; ++d) near = near && blo[3 * I + d] <= bh[d] && bhi[3 * I + d] >= bl[d];
+      for (int d = 0; d < 3; ++d) near = near && flo[3 * I + d] <= bh[d] && fhi[3 * I + d] >= bl[d];
       if (!near) continue;
       bool sig = false;
       for (int q = I * kBlockF; q < (I + 1) * kBlockF && !sig; ++q) {
         const int f = P.h_fperm[q];
         if (f < 0) continue;
-        double d2 = 0.0;
-        for (int d = 0; d < 3; ++d) {
-          const double c = prim->center[3 * f + d];
-          const double e = c < bl[d] ? bl[d] - c : (c > bh[d] ? c - bh[d] : 0.0);
-          d2 += e * e;
-        }
-        sig = d2 <= cut[f] * cut[f];
+        sig = box_distance2(&prim->center[3 * f], bl, bh) <= cut[f] * cut[f];
       }
       if (sig) P.h_mask[b * P.mask_words + I / 32] |= 1u << (I % 32);
     }
