@@ -430,13 +430,25 @@ __device__ __forceinline__ void vstep_next(const uint32_t *__restrict__ mask, in
   }
 }
 
-// element e of thread t of a tile: rows and columns of warp (t / 32)'s 64 x 32 part
+// Output tiles: SL slots of each lane of both blocks (positions 4 lane + c,
+// c < SL), 32 SL rows and columns.  A block of at most 64 functions has them all
+// in two slots, so a basis of one such block multiplies a quarter of the tile
+// (SL = 2; one water, 48 functions, FP64 V of two planes: 176 us with SL = 4,
+// 78 us).  Row or column r of the tile is position vtile_pos<SL>(r) of its block.
+template <int SL>
+__device__ __forceinline__ int vtile_pos(int r) {
+  return SL == 4 ? r : 4 * (r / SL) + r % SL;
+}
+// element e of thread t of a tile: rows and columns of warp (t / 32)'s
+// 16 SL x 8 SL part
+template <int SL>
 __device__ __forceinline__ void vtile_element(int t, int e, int &r, int &c) {
   const int lane = t & 31, warp = t >> 5;
-  r = 64 * (warp & 1) + 8 * (e >> 3) + (lane >> 2);
-  c = 32 * (warp >> 1) + 8 * ((e >> 1) & 3) + 2 * (lane & 3) + (e & 1);
+  r = vtile_pos<SL>(16 * SL * (warp & 1) + 8 * (e / (2 * SL)) + (lane >> 2));
+  c = vtile_pos<SL>(8 * SL * (warp >> 1) + 8 * ((e >> 1) % SL) + 2 * (lane & 3) + (e & 1));
 }
 
+template <int SL>
 __global__ void __launch_bounds__(256, 1)
     vgemm_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ zT, int phi_stride_tiles,
                       int z_stride, const int *__restrict__ pair_off, const uint32_t *__restrict__ mask,
@@ -472,12 +484,16 @@ __global__ void __launch_bounds__(256, 1)
   };
 #pragma unroll
   for (int st = 0; st < kVStages - 1; ++st) issue(st);
-  double acc[8][4][2];
+  constexpr int NI = 2 * SL, NJ = SL;
+  double acc[NI][NJ][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int fr = lane >> 2, fk = lane & 3, r0 = 64 * (warp & 1) + fr, c0 = 32 * (warp >> 1) + fr;
+    for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  // fragment rows 8 i + fr of the warp's part; eight rows are 32 / SL positions
+  const int fr = lane >> 2, fk = lane & 3, r0 = vtile_pos<SL>(16 * SL * (warp & 1) + fr),
+            c0 = vtile_pos<SL>(8 * SL * (warp >> 1) + fr);
+  constexpr int kStep = SL == 4 ? 8 : 32 / SL;
   for (int it = 0; cb < b1; ++it) {
     cp_async_wait<kVStages - 2>();
     __syncthreads();  // step it is visible; the stage refilled below was read in step it - 1
@@ -485,47 +501,48 @@ __global__ void __launch_bounds__(256, 1)
     const double *As = vsm + (it % kVStages) * kVStageDoubles, *Bs = As + kVKs * kVLd;
 #pragma unroll
     for (int k = 0; k < kVKs; k += 4) {
-      double a[8], bb[4];
+      double a[NI], bb[NJ];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = As[(k + fk) * kVLd + r0 + 8 * i];
+      for (int i = 0; i < NI; ++i) a[i] = As[(k + fk) * kVLd + r0 + kStep * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bb[j] = Bs[(k + fk) * kVLd + c0 + 8 * j];
+      for (int j = 0; j < NJ; ++j) bb[j] = Bs[(k + fk) * kVLd + c0 + kStep * j];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma884(acc[i][j], a[i], bb[j]);
+        for (int j = 0; j < NJ; ++j) dmma884(acc[i][j], a[i], bb[j]);
     }
     vstep_next(mask, mask_words, b1, nsplit, I, J, cb, ck);
   }
   cp_async_wait<0>();
   if (nsplit > 1) {
-    double *o = part + ((((size_t)zi * gridDim.y + I) * gridDim.x + J) * nsplit + sp) * kBlockF * kBlockF + threadIdx.x;
+    double *o = part + ((((size_t)zi * gridDim.y + I) * gridDim.x + J) * nsplit + sp) * 4 * SL * SL * 256 + threadIdx.x;
 #pragma unroll
-    for (int e = 0; e < 64; ++e) o[e * 256] = acc[e >> 3][(e >> 1) & 3][e & 1];
+    for (int e = 0; e < 4 * SL * SL; ++e) o[e * 256] = acc[e / (2 * SL)][(e >> 1) % SL][e & 1];
     return;
   }
   double *Vz = V + (size_t)zi * nbf_pad * nbf_pad;
 #pragma unroll
-  for (int e = 0; e < 64; ++e) {
+  for (int e = 0; e < 4 * SL * SL; ++e) {
     int r, c;
-    vtile_element(threadIdx.x, e, r, c);
-    Vz[(size_t)I * 128 + r + ((size_t)J * 128 + c) * nbf_pad] += acc[e >> 3][(e >> 1) & 3][e & 1];
+    vtile_element<SL>(threadIdx.x, e, r, c);
+    Vz[(size_t)I * 128 + r + ((size_t)J * 128 + c) * nbf_pad] += acc[e / (2 * SL)][(e >> 1) % SL][e & 1];
   }
 }
 
 // Vbar += the parts of a split vgemm_fp64_kernel, in split order: block
 // (tile, element e of every thread), one output element per thread
+template <int SL>
 __global__ void __launch_bounds__(256) vpart_reduce_kernel(const double *__restrict__ part, int nsplit, int nblk,
                                                            int nbf_pad, double *__restrict__ V) {
   const int t = blockIdx.x, J = t % nblk, I = (t / nblk) % nblk, zi = t / (nblk * nblk);
-  const double *p = part + (size_t)t * nsplit * kBlockF * kBlockF + threadIdx.x;
+  const double *p = part + (size_t)t * nsplit * 4 * SL * SL * 256 + threadIdx.x;
   double *Vz = V + (size_t)zi * nbf_pad * nbf_pad;
   const int e = blockIdx.y;
   double s = 0.0;
 #pragma unroll 8
-  for (int k = 0; k < nsplit; ++k) s += p[((size_t)k * 64 + e) * 256];
+  for (int k = 0; k < nsplit; ++k) s += p[((size_t)k * 4 * SL * SL + e) * 256];
   int r, c;
-  vtile_element(threadIdx.x, e, r, c);
+  vtile_element<SL>(threadIdx.x, e, r, c);
   Vz[(size_t)I * 128 + r + ((size_t)J * 128 + c) * nbf_pad] += s;
 }
 
@@ -1834,15 +1851,21 @@ static void launch_vgemm_fp64(Plan &P, const Chunk &c, const double *phiT, const
   const long parts = (long)nz * P.nblk * P.nblk;
   const int nsplit = batch_split(parts, c.b1 - c.b0, P.nsm);
   if (nsplit > 1 && !P.d_vpart) P.d_vpart = P.alloc<double>((size_t)4 * P.nsm * kBlockF * kBlockF);
-  NKX_CUDA(cudaFuncSetAttribute(vgemm_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVSmemBytes));
-  vgemm_fp64_kernel<<<dim3(P.nblk, P.nblk, nz * nsplit), 256, kVSmemBytes, s>>>(
-      phiT, zT, phi_stride, z_stride, P.d_pair_off, P.d_mask, P.mask_words, c.b0, c.b1, c.p0, nsplit, P.nbf_pad, V,
-      P.d_vpart);
-  ++P.launches;
-  if (nsplit > 1) {
-    vpart_reduce_kernel<<<dim3((unsigned)parts, 64), 256, 0, s>>>(P.d_vpart, nsplit, P.nblk, P.nbf_pad, V);
+  auto go = [&](auto slots) {
+    constexpr int SL = decltype(slots)::value;
+    NKX_CUDA(cudaFuncSetAttribute(vgemm_fp64_kernel<SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVSmemBytes));
+    vgemm_fp64_kernel<SL><<<dim3(P.nblk, P.nblk, nz * nsplit), 256, kVSmemBytes, s>>>(
+        phiT, zT, phi_stride, z_stride, P.d_pair_off, P.d_mask, P.mask_words, c.b0, c.b1, c.p0, nsplit, P.nbf_pad, V,
+        P.d_vpart);
     ++P.launches;
-  }
+    if (nsplit > 1) {
+      vpart_reduce_kernel<SL><<<dim3((unsigned)parts, 4 * SL * SL), 256, 0, s>>>(P.d_vpart, nsplit, P.nblk, P.nbf_pad,
+                                                                               V);
+      ++P.launches;
+    }
+  };
+  // a block's functions fill slot after slot (build_plan)
+  P.nbf <= 64 ? go(std::integral_constant<int, 2>{}) : go(std::integral_constant<int, 4>{});
   NKX_LAUNCH_CHECK();
 }
 
