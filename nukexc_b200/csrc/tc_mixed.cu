@@ -88,7 +88,10 @@ struct TcShape {
 };
 // TC_MODE_RHO: N = 64 with one stage fewer and T_0 of the epilogue threads,
 // [32 columns][thread]
-constexpr int kRhoStages = 3;
+// TC_MODE_X: the same with each epilogue warp's 32 x 32 tile of X, rows padded
+// to 34 doubles
+constexpr int kRhoStages = 3, kXPitch = 34;
+constexpr int kXSmemTc = kRhoStages * TcShape<64>::kStageBytes + TcShape<64>::EW * 32 * kXPitch * 8 + 1024;
 constexpr int kRhoSmem = kRhoStages * TcShape<64>::kStageBytes + 32 * TcShape<64>::kEpiThreads * 8 + 1024;
 
 struct TcArgs {
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
     tc_i8_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, TcArgs a) {
   using Sh = TcShape<NW, EW>;
   constexpr int N = Sh::N, NBUF = Sh::NBUF, kStageBytes = Sh::kStageBytes, CW = Sh::CW;
-  constexpr int kStages = MODE == TC_MODE_RHO ? kRhoStages : Sh::kStages;
+  constexpr int kStages = MODE == TC_MODE_RHO || MODE == TC_MODE_X ? kRhoStages : Sh::kStages;
   // modes that accumulate a run of groups in registers
   constexpr bool kRun = MODE == TC_MODE_V || MODE == TC_MODE_DENSITY || MODE == TC_MODE_RHO;
   static_assert(MODE == TC_MODE_V || CW == 32, "the density, Y and X epilogues take 32 columns a warp");
@@ -466,17 +469,15 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
         if (abort_flag) return;
         const uint32_t buf = grp % NBUF, use = grp / NBUF;
         if constexpr (MODE == TC_MODE_X) {
-          // X_c(g, mu) of the thread's point and 32 functions, written in
-          // FP64 slice by slice (8 consecutive doubles a slice)
-          const int gpt = 128 * it.h + row;
+          // X_c(g, mu) of the thread's point and 32 functions in FP64, by
+          // slices of 8 into the warp's shared tile
           const double sa =
               a.sA[((((it.bl * a.nspin + it.s) * a.ncomp + it.c) * 2 + it.h)) * 128 + row] * kTwoM36;
           const double sbl = a.sB[(size_t)it.s * a.nbf_pad + 128 * g.blk + 64 * it.t + 32 * cq + lane];
           if (!mbar_wait(&tfull_bar[buf], use & 1, a.err, 6, &abort_flag, a.wait_ns)) return;
           tc_fence_after();
           __syncwarp();
-          double *Xp = a.X + ((((size_t)it.q * a.nspin + it.s) * a.ncomp + it.c) * kBatch + gpt) * kBlockF +
-                       64 * it.t + 32 * cq;
+          double *xs = reinterpret_cast<double *>(smem + kStages * kStageBytes) + (warp - 2) * 32 * kXPitch;
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
             uint32_t v0[8], v1[8], v2[8], v3[8];
@@ -498,8 +499,21 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
             for (int j = 0; j < 8; ++j)
               x[j] = level_sum(v0[j], v1[j], v2[j], v3[j]) * (sa * __shfl_sync(0xffffffffu, sbl, 8 * h + j));
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) reinterpret_cast<double2 *>(Xp + 8 * h + j)[0] = make_double2(x[j], x[j + 1]);
+            for (int j = 0; j < 8; j += 2)
+              *reinterpret_cast<double2 *>(xs + lane * kXPitch + 8 * h + j) = make_double2(x[j], x[j + 1]);
           }
+          // the warp's 32 points x 32 functions leave as two 256-byte rows an
+          // instruction (each lane writing its own point's row made every
+          // store touch 32 lines: (H2O)_8 PBE 2.78 ms, 2.05 ms now)
+          __syncwarp();
+          double *Xp = a.X + ((((size_t)it.q * a.nspin + it.s) * a.ncomp + it.c) * kBatch + 128 * it.h + 32 * q) * kBlockF +
+                       64 * it.t + 32 * cq;
+          const int r2 = lane >> 4, c2 = 2 * (lane & 15);
+#pragma unroll
+          for (int r = 0; r < 32; r += 2)
+            *reinterpret_cast<double2 *>(Xp + (size_t)(r + r2) * kBlockF + c2) =
+                *reinterpret_cast<const double2 *>(xs + (r + r2) * kXPitch + c2);
+          __syncwarp();
           ++grp;
           return;
         }
@@ -1883,8 +1897,7 @@ static MixedState &mixed_state(Plan &P, int nocc) {
                                   TcShape<128>::kSmem));
     NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_GRAD, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   TcShape<64>::kSmem));
-    NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_X, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  TcShape<64>::kSmem));
+    NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_X, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmemTc));
     NKX_CUDA(cudaFuncSetAttribute(tc_i8_kernel<TC_MODE_GRAD, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   TcShape<128>::kSmem));
     NKX_CUDA(cudaFuncSetAttribute(zquant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 4 * 128 * 36));
@@ -1917,7 +1930,7 @@ static MixedState &mixed_state(Plan &P, int nocc) {
 template <int MODE, int NW, int EW = NW / 8>
 static void launch_i8_shape(const CUtensorMap &mA, const CUtensorMap &mB, const TcArgs &a, unsigned grid,
                             cudaStream_t s) {
-  constexpr int smem = MODE == TC_MODE_RHO ? kRhoSmem : TcShape<NW, EW>::kSmem;
+  constexpr int smem = MODE == TC_MODE_RHO ? kRhoSmem : MODE == TC_MODE_X ? kXSmemTc : TcShape<NW, EW>::kSmem;
   tc_i8_kernel<MODE, NW, EW><<<grid, TcShape<NW, EW>::kThreads, smem, s>>>(mA, mB, a);
 }
 
