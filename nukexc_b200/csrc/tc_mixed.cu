@@ -1403,7 +1403,15 @@ constexpr int kZdRanks = 4;
 template <bool GRAD, int NZ, bool JP>
 struct ZdShape {
   static constexpr int NS = GRAD ? NZ - JP : 0;  // staged planes
-  static constexpr size_t kSmem = ((size_t)NS * 8 + 4) * (kBatch / kZdRanks) * kBlockF + 8 * (1 + NZ) * (kBatch / kZdRanks);
+  // rows of the staged planes and of phi's digits, and the per-point numbers, are
+  // skewed by 64 and 32 bytes and by one number for each 16 points
+  static constexpr int kPts = kBatch / kZdRanks, kTile = kPts * kBlockF + 8 * (kPts / 16), kNums = kPts + kPts / 16;
+  static constexpr size_t kSmem = ((size_t)NS * 8 + 4) * kTile + 8 * (1 + NZ) * kNums;
+  // element (point, function) of a staged plane and of phi's digits: 16-byte
+  // pieces of a row change places so that both phases meet no bank twice
+  static __device__ __forceinline__ int z_at(int gl, int f) { return gl * kBlockF + 8 * (gl >> 4) + (f ^ ((f >> 3) & 6)); }
+  static __device__ __forceinline__ int phi_at(int gl, int f) { return gl * kBlockF + 8 * (gl >> 4) + (f ^ ((f >> 3) & 4)); }
+  static __device__ __forceinline__ int num_at(int gl) { return gl + (gl >> 4); }
 };
 // JP: the last plane is the Coulomb one
 template <bool GRAD, int NZ, bool JP>
@@ -1412,15 +1420,16 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, GRAD || 
                    const int *__restrict__ pair_batch, long p0, const double *__restrict__ coef,
                    const double *__restrict__ vj, long npad, uint8_t *__restrict__ qph,
                    double *__restrict__ sph, uint8_t *__restrict__ qz, double *__restrict__ szs, int *nonfinite) {
-  constexpr int NC = GRAD ? 4 : 1, nop = 1 + NZ, kPts = kBatch / kZdRanks, NS = ZdShape<GRAD, NZ, JP>::NS;
+  using Sh = ZdShape<GRAD, NZ, JP>;
+  constexpr int NC = GRAD ? 4 : 1, nop = 1 + NZ, kPts = Sh::kPts, NS = Sh::NS;
   constexpr int nspin = NZ - JP;
   constexpr size_t kPlane = (size_t)kBatch * kBlockF;  // one digit plane of a pair, bytes
   // dynamic shared memory: the staged Z_s [NS][kPts][128] FP64, then phi as
   // packed pass-A digits [kPts][128], its point scales s_g 2^-30 [kPts] and
-  // the planes' phi coefficients [NZ][kPts]
+  // the planes' phi coefficients [NZ][kPts], all skewed
   extern __shared__ __align__(16) double zst[];
-  uint32_t(*phid)[128] = reinterpret_cast<uint32_t(*)[128]>(zst + (size_t)NS * kPts * kBlockF);
-  double *phis = reinterpret_cast<double *>(phid + kPts), *zc = phis + kPts;
+  uint32_t *phid = reinterpret_cast<uint32_t *>(zst + (size_t)NS * Sh::kTile);
+  double *phis = reinterpret_cast<double *>(phid + Sh::kTile), *zc = phis + Sh::kNums;
   __shared__ uint32_t red[8][nop][128];
   __shared__ uint32_t part[kZdRanks][nop][128];  // every CTA's row fields, pushed by their owners
   __shared__ double inv_s[nop][128];
@@ -1465,10 +1474,9 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, GRAD || 
 #pragma unroll
       for (int k = 0; k < 8; ++k) v[k] = int_to_double(digits_value(bw[k])) * sc;
       if (c == 0) {
-        uint4 *pd = reinterpret_cast<uint4 *>(&phid[gl][f8]);
-        pd[0] = make_uint4(bw[0], bw[1], bw[2], bw[3]);
-        pd[1] = make_uint4(bw[4], bw[5], bw[6], bw[7]);
-        if ((lane & 15) == 0) phis[gl] = sc;
+        *reinterpret_cast<uint4 *>(&phid[Sh::phi_at(gl, f8)]) = make_uint4(bw[0], bw[1], bw[2], bw[3]);
+        *reinterpret_cast<uint4 *>(&phid[Sh::phi_at(gl, f8 + 4)]) = make_uint4(bw[4], bw[5], bw[6], bw[7]);
+        if ((lane & 15) == 0) phis[Sh::num_at(gl)] = sc;
 #pragma unroll
         for (int k = 0; k < 8; ++k) e[0][k] = max(e[0][k], exp_field(v[k]));
       }
@@ -1476,7 +1484,7 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, GRAD || 
       for (int s = 0; s < NZ; ++s) {
         if (s >= NS && c > 0) continue;  // a multiple of phi
         const double cc = s < nspin ? coef[((size_t)s * 4 + c) * npad + gg] : 0.5 * vj[gg];
-        if (s >= NS && (lane & 15) == 0) zc[s * kPts + gl] = cc;
+        if (s >= NS && (lane & 15) == 0) zc[s * Sh::kNums + Sh::num_at(gl)] = cc;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           // Z = c0 phi + ((c1 dx phi + c2 dy phi) + c3 dz phi)
@@ -1497,9 +1505,9 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, GRAD || 
         e[1 + s][k] = max(e[1 + s][k], exp_field(z[s][k]));
       }
       if (s < NS) {
-        double2 *dst = reinterpret_cast<double2 *>(zst + ((size_t)s * kPts + gl) * kBlockF + f8);
 #pragma unroll
-        for (int k = 0; k < 8; k += 2) dst[k / 2] = make_double2(z[s][k], z[s][k + 1]);
+        for (int k = 0; k < 8; k += 2)
+          *reinterpret_cast<double2 *>(&zst[s * Sh::kTile + Sh::z_at(gl, f8 + k)]) = make_double2(z[s][k], z[s][k + 1]);
       }
     }
   }
@@ -1552,41 +1560,43 @@ __global__ void __cluster_dims__(kZdRanks, 1, 1) __launch_bounds__(256, GRAD || 
     }
   }
   __syncthreads();
-  // ---- phase 2: thread (f, gh) writes points gbase + 32 gh .. + 31 of row f
-  static_assert(kPts == 64, "two threads a row, 32 points each");
-  {
-    const int f = threadIdx.x & 127, gh = threadIdx.x >> 7;
+  // ---- phase 2: lane 4 r + c of warp w writes points 16 c .. 16 c + 15 of rows
+  // 8 w + r and 64 + 8 w + r: a store instruction fills the CTA's 64 bytes of
+  // eight rows.  (With 32 rows of 16 bytes a store and unskewed tiles the L1 data
+  // pipe was busy 58 % of the time: 12285 pairs of the 149-atom aggregate 3.05
+  // ms, 2.37 now; (H2O)_8 PBE + J 2.28 -> 1.92; one water LDA 43 -> 31 us.)
+  static_assert(kPts == 64 && kBlockF == 128, "four lanes a row, two rows a thread");
+  const int gl0 = 16 * (lane & 3);
 #pragma unroll
-    for (int o = 0; o < nop; ++o) {
+  for (int o = 0; o < nop; ++o) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int f = 64 * h + 8 * warp + (lane >> 2);
       const double inv = inv_s[o][f];
+      uint32_t w[4][4];  // [digit plane][group of four points]
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t w[4][4];  // [digit plane][group of four points]
+      for (int k4 = 0; k4 < 4; ++k4) {
+        double v[4];
 #pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) {
-          const int gl = 32 * gh + 16 * h + 4 * k4;
-          double v[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if (o >= 1 && o <= NS) {
-              v[i] = zst[((size_t)(o - 1) * kPts + gl + i) * kBlockF + f];
-            } else {
-              v[i] = int_to_double(digits_value(phid[gl + i][f])) * phis[gl + i];
-              if (o > 0) v[i] *= zc[(o - 1) * kPts + gl + i];
-            }
+        for (int i = 0; i < 4; ++i) {
+          const int gl = gl0 + 4 * k4 + i;
+          if (o >= 1 && o <= NS) {
+            v[i] = zst[(o - 1) * Sh::kTile + Sh::z_at(gl, f)];
+          } else {
+            v[i] = int_to_double(digits_value(phid[Sh::phi_at(gl, f)])) * phis[Sh::num_at(gl)];
+            if (o > 0) v[i] *= zc[(o - 1) * Sh::kNums + Sh::num_at(gl)];
           }
-          uint32_t ww[4];
-          quant4(v, inv, ww);
-#pragma unroll
-          for (int d = 0; d < 4; ++d) w[d][k4] = ww[d];
         }
+        uint32_t ww[4];
+        quant4(v, inv, ww);
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-          uint8_t *row = (o == 0) ? qph + ((q * 4 + d) * 128 + f) * (size_t)kBatch
-                                  : qz + (((q * NZ + (o - 1)) * 4 + d) * 128 + f) * (size_t)kBatch;
-          *reinterpret_cast<uint4 *>(row + gbase + 32 * gh + 16 * h) =
-              make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
-        }
+        for (int d = 0; d < 4; ++d) w[d][k4] = ww[d];
+      }
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        uint8_t *row = (o == 0) ? qph + ((q * 4 + d) * 128 + f) * (size_t)kBatch
+                                : qz + (((q * NZ + (o - 1)) * 4 + d) * 128 + f) * (size_t)kBatch;
+        *reinterpret_cast<uint4 *>(row + gbase + gl0) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
       }
     }
   }
