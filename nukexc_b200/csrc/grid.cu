@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "host_setup.hpp"
@@ -103,87 +104,120 @@ __global__ void becke_thread_kernel(const double *__restrict__ centers, int nato
   w[g] *= pown / norm;
 }
 
-// Becke weights, one warp per 32 points (a point per lane).  The same exact
-// screening, shared by the warp: a point whose owner has r_own >= r_min + Rc
-// has weight exactly 0 and needs no cell at all; the other points' candidate
-// atoms (r_j < r_min + 2 Rc for any of them) are listed once with every
-// point's distance in shared memory [candidate][lane], so the pair loop reads
-// distances instead of taking square roots, and 1/R_ij, the same for all
-// points, is formed by one lane per j and broadcast.  Cells and factors that
-// are trivial for all 32 points are skipped by a warp vote.
+// Becke weights, a block of W warps per 32 points (a point per lane,
+// the same in every warp).  The same exact screening, shared by the block: a
+// point whose owner has r_own >= r_min + Rc has weight exactly 0 and needs no
+// cell at all; the other points' candidate atoms (r_j < r_min + 2 Rc for any of
+// them) are listed once with every point's distance in shared memory
+// [candidate][lane], warp w the atoms w, w + W, ..., so the pair loop
+// reads distances instead of taking square roots, and 1/R_ij, the same for all
+// points, is formed by one lane per j and broadcast.  A warp takes the cells of
+// its own list.  Cells and factors that are trivial for all 32 points are
+// skipped by a warp vote.
 //
 // Bound: FP64 issue of the pair loop (about 20 instructions a pair).
-// (H2O)_16, 1.09 M points: 5.05 ms with a thread per point (distances and
-// R_ij recomputed per pair, lists in local memory), 1.63 ms now.  The list
-// has room for every atom, up to kBeckeCap (37 KB a warp, six warps an SM):
-// 144 atoms, 1.35 M points: 12.6 ms against 20.7; at 192 the points of a warp,
-// all round their owner, share few of their candidates, and with lists of 144
-// (the others by a thread each) 1.80 M points took 40.8 ms against 33.3.
-constexpr int kBeckeCap = 144;
-__global__ void __launch_bounds__(32) becke_kernel(const double *__restrict__ centers, int natoms,
-                                                   const double *__restrict__ pts, const int *__restrict__ owner,
-                                                   long npts, double *__restrict__ w, double clamp) {
-  extern __shared__ double rsm[];  // [natoms][32] distances, then the atoms' indices [natoms]
-  int *list = reinterpret_cast<int *>(rsm + (size_t)natoms * 32);
-  const int lane = threadIdx.x;
+// By W, in ms (a thread per point, distances and R_ij recomputed per pair: 0):
+//   atoms  points    W = 0   W = 1   W = 4   W = 8   W = 16
+//     24   0.23 M     0.51    0.21    0.20    0.26    0.42
+//     48   0.47 M     2.60    0.90    0.73    0.90    1.24
+//     96   0.93 M     9.4     4.5     2.57    2.82    3.90
+//    192   1.86 M    33.3             14.0    10.1    11.9
+//    384   3.72 M                     60.7    38.4    34.1
+// so four up to 96 atoms and eight beyond.  The list has room for every atom, up
+// to kBeckeCap (104 KB, two CTAs an SM).
+constexpr int kBeckeCap = 400, kBeckeNarrow = 96;  // kBeckeCap a multiple of every W
+template <int W>
+__global__ void __launch_bounds__(32 * W)
+    becke_kernel(const double *__restrict__ centers, int natoms, const double *__restrict__ pts,
+                 const int *__restrict__ owner, long npts, double *__restrict__ w, double clamp) {
+  extern __shared__ double rsm[];  // [slots][32] distances, then the atoms' indices [slots]
+  __shared__ double red[2][W][32];
+  __shared__ int nw[W];
+  const int seg = (natoms + W - 1) / W;
+  int *list = reinterpret_cast<int *>(rsm + (size_t)seg * W * 32);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s0 = warp * seg;
   const long g = blockIdx.x * 32L + lane;
   const bool in = g < npts;
   const double *p = pts + 3 * (in ? g : npts - 1);
-  const double x = p[0], y = p[1], z = p[2];
+  const double pt[3] = {p[0], p[1], p[2]};
   const int own = owner[in ? g : npts - 1];
   const double Rc = clamp > 0.0 ? clamp : 1e300;  // unclamped: no atom is screened
   double r2min = 1e300;
-  for (int i = 0; i < natoms; ++i) {
-    const double dx = x - centers[3 * i], dy = y - centers[3 * i + 1], dz = z - centers[3 * i + 2];
+  for (int i = warp; i < natoms; i += W) {
+    const double dx = pt[0] - centers[3 * i], dy = pt[1] - centers[3 * i + 1], dz = pt[2] - centers[3 * i + 2];
     r2min = fmin(r2min, dx * dx + dy * dy + dz * dz);
   }
+  red[0][warp][lane] = r2min;
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < W; ++v) r2min = fmin(r2min, red[0][v][lane]);
   const double rmin = sqrt(r2min), lim = rmin + 2.0 * Rc;
-  const double pt[3] = {x, y, z};
   const bool live = in && dist3(pt, centers + 3 * own) < rmin + Rc;
-  if (in && !live) w[g] *= 0.0;  // P_owner == 0 exactly
-  if (!__any_sync(0xffffffffu, live)) return;
+  if (warp == 0 && in && !live) w[g] *= 0.0;  // P_owner == 0 exactly
+  if (!__any_sync(0xffffffffu, live)) return;  // alike in every warp
   int nl = 0;
-  for (int j = 0; j < natoms; ++j) {
+  for (int j = warp; j < natoms; j += W) {
     const double r = dist3(pt, centers + 3 * j);
     if (!__any_sync(0xffffffffu, live && r < lim)) continue;
-    rsm[nl * 32 + lane] = r;
-    if (lane == 0) list[nl] = j;
+    rsm[(s0 + nl) * 32 + lane] = r;
+    if (lane == 0) list[s0 + nl] = j;
     ++nl;
   }
-  __syncwarp();
+  if (lane == 0) nw[warp] = nl;
+  __syncthreads();  // also: every warp has read red[0]
   double norm = 0.0, pown = 0.0;
-  for (int a = 0; a < nl; ++a) {
+  for (int a = s0; a < s0 + nl; ++a) {
     const double ri = rsm[a * 32 + lane];
     const bool cell = live && ri < rmin + Rc;  // else P_i == 0 exactly
     if (!__any_sync(0xffffffffu, cell)) continue;
     const int i = list[a];
     const double reach = cell ? ri + Rc : -1.0;  // factors of atoms at reach and beyond are 1
     double P = 1.0;
-    for (int c0 = 0; c0 < nl; c0 += 32) {
-      double iR = 0.0;
-      if (c0 + lane < nl && c0 + lane != a)
-        iR = 1.0 / fmin(dist3(centers + 3 * i, centers + 3 * list[c0 + lane]), Rc);
-      const int n = min(32, nl - c0);
-      for (int t = 0; t < n; ++t) {
-        const double rj = rsm[(c0 + t) * 32 + lane];
-        if (!__any_sync(0xffffffffu, rj < reach) || c0 + t == a) continue;
-        P *= becke_s((ri - rj) * __shfl_sync(0xffffffffu, iR, t));
+    for (int v = 0; v < W; ++v)
+      for (int c0 = 0; c0 < nw[v]; c0 += 32) {
+        const int n = min(32, nw[v] - c0), cb = v * seg + c0;
+        double iR = 0.0;
+        if (lane < n && cb + lane != a) iR = 1.0 / fmin(dist3(centers + 3 * i, centers + 3 * list[cb + lane]), Rc);
+        for (int t = 0; t < n; ++t) {
+          const double rj = rsm[(cb + t) * 32 + lane];
+          if (!__any_sync(0xffffffffu, rj < reach) || cb + t == a) continue;
+          P *= becke_s((ri - rj) * __shfl_sync(0xffffffffu, iR, t));
+        }
       }
-    }
     if (cell) {
       if (i == own) pown = P;
       norm += P;
     }
   }
-  if (live) w[g] *= pown / norm;
+  red[0][warp][lane] = norm;
+  red[1][warp][lane] = pown;
+  __syncthreads();
+  if (warp == 0 && live) {
+    norm = pown = 0.0;
+#pragma unroll
+    for (int v = 0; v < W; ++v) {
+      norm += red[0][v][lane];
+      pown += red[1][v][lane];  // one of them, the others are zero
+    }
+    w[g] *= pown / norm;
+  }
 }
 
 void launch_becke(const double *d_centers, int natoms, const double *d_pts, const int *d_owner, long npts,
                   double *d_w, double clamp, cudaStream_t s) {
   if (npts <= 0) return;
   if (natoms <= kBeckeCap) {
-    const size_t smem = (size_t)natoms * (32 * sizeof(double) + sizeof(int));
-    becke_kernel<<<(unsigned)((npts + 31) / 32), 32, smem, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w, clamp);
+    auto go = [&](auto warps) {
+      constexpr int W = decltype(warps)::value;
+      constexpr size_t kAtomBytes = 32 * sizeof(double) + sizeof(int);
+      const size_t smem = (size_t)((natoms + W - 1) / W * W) * kAtomBytes;
+      // the limit is the same for every call, so that threads cannot lower it for one another
+      NKX_CUDA(cudaFuncSetAttribute(becke_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(kBeckeCap * kAtomBytes)));
+      becke_kernel<W><<<(unsigned)((npts + 31) / 32), 32 * W, smem, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w,
+                                                                        clamp);
+    };
+    natoms <= kBeckeNarrow ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 8>{});
   } else {
     const int T = 128;
     becke_thread_kernel<<<(unsigned)((npts + T - 1) / T), T, 0, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w,

@@ -1,6 +1,6 @@
-"""Becke weights where the warp's atom list can go wrong: one atom, lists of
-exactly and just over 32 atoms, more atoms than the list holds (the
-per-thread path), the unclamped original, points far outside, and owners that
+"""Becke weights where the warps' atom lists can go wrong: fewer atoms than warps,
+lists of about 32 atoms, the last size of four warps and of eight, more atoms
+than the lists hold (the per-thread path), the unclamped original, points far outside, and owners that
 change inside a warp -- against the oracle's full loops (1e-13 absolute on
 weights of at most 1)."""
 import numpy as np
@@ -18,7 +18,7 @@ from oracle import oracle as O  # noqa: E402
 
 @pytest.mark.parametrize("natoms,box,clamp", [(1, 3.0, 5.0), (2, 3.0, 0.0), (32, 9.0, 5.0), (33, 9.0, 0.0),
                                               (70, 30.0, 5.0), (144, 6.0, 5.0), (150, 6.0, 5.0), (150, 6.0, 0.0),
-                                              (200, 40.0, 2.0)])
+                                              (200, 40.0, 2.0), (96, 12.0, 5.0), (97, 12.0, 5.0), (400, 25.0, 5.0), (401, 25.0, 5.0)])
 def test_becke_matches_oracle(natoms, box, clamp):
     rng = np.random.default_rng(natoms)
     c = rng.uniform(0, box, size=(natoms, 3))
