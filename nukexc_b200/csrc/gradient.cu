@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <functional>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -486,137 +487,165 @@ __global__ void becke_grad_kernel(const double *__restrict__ C, int natoms, cons
   }
 }
 
-// The Becke-weight term of molecules of up to kGradCap atoms, one warp per 32
-// points, with the screening of becke_grad_kernel: atoms with
-// r < r_min + 2 Rc of any of the points are candidates.
-// The candidates are listed once; shared memory holds per candidate and point the distance, the cell function
-// P and the weight D.  With a_ij = f a kappa_i s'(mu_ij) / (s(mu_ij) R_ij) the
-// terms of all pairs collapse to
+// The Becke-weight term of molecules of up to kGradCap atoms, a block of
+// W warps per 32 points (a point per lane, the same in every warp),
+// with the screening of becke_grad_kernel: atoms with r < r_min + 2 Rc of any
+// of the points are candidates.  Warp w lists those among the atoms w,
+// w + W, ...; shared memory holds per candidate and point the
+// distance, the cell function P and the weight D.  With
+// a_ij = f a kappa_i s'(mu_ij) / (s(mu_ij) R_ij) the terms of all pairs collapse to
 //   F_k += -D_k u_k,  F_o += sum_k D_k u_k,   D_k = sum_j a_kj - sum_i a_ik,
 //   F_i -= G_ij e_ij, F_j += G_ij e_ij,       G_ij = sum_points a_ij mu_ij
 // (e_ij terms only where |R_i - R_j| is below the clamp), so a pair costs one
 // scalar per point, and one warp reduction when it is not clamped; vectors
-// appear once per atom.  Each warp strides over the points and adds its sums
-// to F once.
+// appear once per atom.  A warp takes the cells i of its own list for P and the
+// atoms j of its own list for D, so only the sums over j (Ss) meet between
+// warps.  Each block strides over the points and adds its sums to F once.
 //
-// Bound: FP64 issue.  (H2O)_8: 7.2 ms per gradient with a thread per point
-// (vector atomics in shared memory per pair), 1.91 ms now.
-constexpr int kGradCap = 64;
-__global__ void __launch_bounds__(32)
+// Bound: FP64 issue; the candidates' arrays in shared memory set how many
+// points an SM has in flight, which is why several warps share them.  By W, in ms
+// (a thread per point with vector atomics in shared memory per pair: 0):
+//   atoms  points    W = 0   W = 1   W = 4   W = 8   W = 16
+//     24   0.22 M     3.97    1.21    0.67    0.79    1.21
+//     48   0.43 M    15.3     5.84    2.60    2.57    3.05
+//     96   0.85 M    67.0             13.5    8.8     13.9
+//    192   1.68 M     250             68.6    42.9    38.3
+// so four up to 48 atoms and eight beyond, up to what shared memory holds.
+constexpr int kGradCap = 192, kGradNarrow = 48;  // kGradCap a multiple of every W
+constexpr size_t kGradAtomBytes = 4 * 32 * sizeof(double) + 3 * sizeof(double) + sizeof(int);
+template <int W>
+__global__ void __launch_bounds__(32 * W)
     becke_grad_warp_kernel(const double *__restrict__ C, int natoms, const double *__restrict__ px,
                            const double *__restrict__ py, const double *__restrict__ pz, const double *__restrict__ w,
                            const int *__restrict__ owner, const double *__restrict__ edens, long npad, double clamp,
                            double *__restrict__ F) {
-  extern __shared__ double gsm[];  // r, P, D [natoms][32], F [3 natoms], list [natoms]
-  double *rs = gsm, *Ps = rs + natoms * 32, *Ds = Ps + natoms * 32, *Fa = Ds + natoms * 32;
+  extern __shared__ double gsm[];  // r, P, D, S [slots][32], F [3 natoms], list [slots]
+  __shared__ double red[2][W][32], redP[W][32], redZ[W][32];
+  __shared__ int nw[W];
+  const int seg = (natoms + W - 1) / W, slots = seg * W;
+  double *rs = gsm, *Ps = rs + slots * 32, *Ds = Ps + slots * 32, *Ss = Ds + slots * 32, *Fa = Ss + slots * 32;
   int *list = reinterpret_cast<int *>(Fa + 3 * natoms);
-  const int lane = threadIdx.x;
-  for (int e = lane; e < 3 * natoms; e += 32) Fa[e] = 0.0;
-  __syncwarp();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s0 = warp * seg;
+  for (int e = threadIdx.x; e < 3 * natoms; e += blockDim.x) Fa[e] = 0.0;
   const double Rc = clamp > 0.0 ? clamp : 1e300;
-  for (long g0 = blockIdx.x * 32L; g0 < npad; g0 += gridDim.x * 32L) {  // npad is a multiple of 256
+  int turn = 0;
+  for (long g0 = blockIdx.x * 32L; g0 < npad; g0 += gridDim.x * 32L, turn ^= 1) {  // npad is a multiple of 256
     const long g = g0 + lane;
     const double r[3] = {px[g], py[g], pz[g]};
     const double wg = w[g], eg = edens[g];
     const int o = owner[g];
-    auto dist = [&](int a) {
+    auto dist2 = [&](int a) {
       const double dx = r[0] - C[3 * a], dy = r[1] - C[3 * a + 1], dz = r[2] - C[3 * a + 2];
-      return sqrt(dx * dx + dy * dy + dz * dz);
+      return dx * dx + dy * dy + dz * dz;
     };
     double r2min = 1e300;
-    for (int a = 0; a < natoms; ++a) {
-      const double dx = r[0] - C[3 * a], dy = r[1] - C[3 * a + 1], dz = r[2] - C[3 * a + 2];
-      r2min = fmin(r2min, dx * dx + dy * dy + dz * dz);
-    }
+    for (int a = warp; a < natoms; a += W) r2min = fmin(r2min, dist2(a));
+    red[turn][warp][lane] = r2min;
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < W; ++v) r2min = fmin(r2min, red[turn][v][lane]);
     const double rmin = sqrt(r2min), lim = rmin + 2.0 * Rc;
-    const bool live = wg != 0.0 && eg != 0.0 && dist(o) < rmin + Rc;  // else no term, or P_o == 0
-    if (!__any_sync(0xffffffffu, live)) continue;
+    const bool live = wg != 0.0 && eg != 0.0 && sqrt(dist2(o)) < rmin + Rc;  // else no term, or P_o == 0
+    if (!__any_sync(0xffffffffu, live)) continue;  // alike in every warp
     int nl = 0;
-    for (int a = 0; a < natoms; ++a) {
-      const double ra = dist(a);
+    for (int a = warp; a < natoms; a += W) {
+      const double ra = sqrt(dist2(a));
       if (!__any_sync(0xffffffffu, live && ra < lim)) continue;
-      rs[nl * 32 + lane] = ra;
-      Ds[nl * 32 + lane] = 0.0;
-      if (lane == 0) list[nl] = a;
+      rs[(s0 + nl) * 32 + lane] = ra;
+      Ds[(s0 + nl) * 32 + lane] = Ss[(s0 + nl) * 32 + lane] = 0.0;
+      if (lane == 0) list[s0 + nl] = a;
       ++nl;
     }
-    __syncwarp();
-    // |R_i - R_j| of candidates a and c0 + lane (inverse of the clamped one)
-    auto inverse = [&](int i, int c, double &dij) {
+    if (lane == 0) nw[warp] = nl;
+    __syncthreads();
+    // |R_i - R_j| of atom i and the candidate in slot c (inverse of the clamped one)
+    auto inverse = [&](int i, int c, bool in, double &dij) {
       dij = 0.0;
-      if (c >= nl || list[c] == i) return 0.0;
+      if (!in || list[c] == i) return 0.0;
       const int j = list[c];
       const double dx = C[3 * i] - C[3 * j], dy = C[3 * i + 1] - C[3 * j + 1], dz = C[3 * i + 2] - C[3 * j + 2];
       dij = sqrt(dx * dx + dy * dy + dz * dz);
       return 1.0 / fmin(dij, Rc);
     };
     double Z = 0.0, Po = 0.0;
-    for (int a = 0; a < nl; ++a) {
+    for (int a = s0; a < s0 + nl; ++a) {
       const double ri = rs[a * 32 + lane];
       const bool cell = live && ri < rmin + Rc;  // else P_i = 0 exactly
       double P = cell ? 1.0 : 0.0;
       const int i = list[a];
       if (__any_sync(0xffffffffu, cell)) {
         const double reach = cell ? ri + Rc : -1.0;
-        for (int c0 = 0; c0 < nl; c0 += 32) {
-          double dij;
-          const double iR = inverse(i, c0 + lane, dij);
-          const int n = min(32, nl - c0);
-          for (int t = 0; t < n; ++t) {
-            const double rj = rs[(c0 + t) * 32 + lane];
-            if (!__any_sync(0xffffffffu, rj < reach) || c0 + t == a) continue;
-            double mu = (ri - rj) * __shfl_sync(0xffffffffu, iR, t), sv, dsv;
-            mu = mu > 1.0 ? 1.0 : (mu < -1.0 ? -1.0 : mu);
-            becke_s_ds(mu, sv, dsv);
-            P *= sv;
+        for (int v = 0; v < W; ++v)
+          for (int c0 = 0; c0 < nw[v]; c0 += 32) {
+            double dij;
+            const int n = min(32, nw[v] - c0), cb = v * seg + c0;
+            const double iR = inverse(i, cb + lane, lane < n, dij);
+            for (int t = 0; t < n; ++t) {
+              const double rj = rs[(cb + t) * 32 + lane];
+              if (!__any_sync(0xffffffffu, rj < reach) || cb + t == a) continue;
+              double mu = (ri - rj) * __shfl_sync(0xffffffffu, iR, t), sv, dsv;
+              mu = mu > 1.0 ? 1.0 : (mu < -1.0 ? -1.0 : mu);
+              becke_s_ds(mu, sv, dsv);
+              P *= sv;
+            }
           }
-        }
       }
       Ps[a * 32 + lane] = P;
       Z += P;
       if (i == o) Po = P;
     }
+    redZ[warp][lane] = Z;
+    redP[warp][lane] = Po;
+    __syncthreads();
+    Z = Po = 0.0;
+#pragma unroll
+    for (int v = 0; v < W; ++v) {
+      Z += redZ[v][lane];
+      Po += redP[v][lane];  // one of them, the others are zero
+    }
     const bool on = live && Po > 0.0 && Z > 0.0;
     const double Q = on ? Po / Z : 0.0, fa = on ? eg * (wg / Q) : 0.0, iZ = on ? 1.0 / Z : 0.0;
-    for (int a = 0; a < nl; ++a) {
-      const double ri = rs[a * 32 + lane];
-      const int i = list[a];
-      const double kappa = Q * ((i == o ? 1.0 : 0.0) - Ps[a * 32 + lane] * iZ);
-      const bool cell = on && kappa != 0.0 && ri > 0.0;
-      if (!__any_sync(0xffffffffu, cell)) continue;
-      const double reach = cell ? ri + Rc : -1.0, fk = cell ? fa * kappa : 0.0;
-      double A = 0.0;
-      for (int c0 = 0; c0 < nl; c0 += 32) {
-        double dij;
-        const double iR = inverse(i, c0 + lane, dij);
-        const int n = min(32, nl - c0);
-        for (int t = 0; t < n; ++t) {
-          const double rj = rs[(c0 + t) * 32 + lane];
-          if (!__any_sync(0xffffffffu, rj < reach) || c0 + t == a) continue;
-          const double iRt = __shfl_sync(0xffffffffu, iR, t), dt = __shfl_sync(0xffffffffu, dij, t);
-          const double mu = (ri - rj) * iRt;
-          double sv, ds, lam = 0.0;
-          becke_s_ds(mu, sv, ds);
-          if (rj > 0.0 && mu > -1.0 && mu < 1.0 && sv > 0.0) lam = fk * ds / sv * iRt;
-          A += lam;
-          Ds[(c0 + t) * 32 + lane] -= lam;
-          if (dt < Rc) {
-            const double G = warp_sum(lam * mu);
-            if (lane < 3 && G != 0.0) {
-              const int j = list[c0 + t];
-              const double e = G * (C[3 * i + lane] - C[3 * j + lane]) / dt;
-              atomicAdd(&Fa[3 * i + lane], -e);
-              atomicAdd(&Fa[3 * j + lane], e);
+    for (int v = 0; v < W; ++v)
+      for (int a = v * seg; a < v * seg + nw[v]; ++a) {
+        const double ri = rs[a * 32 + lane];
+        const int i = list[a];
+        const double kappa = Q * ((i == o ? 1.0 : 0.0) - Ps[a * 32 + lane] * iZ);
+        const bool cell = on && kappa != 0.0 && ri > 0.0;
+        if (!__any_sync(0xffffffffu, cell)) continue;
+        const double reach = cell ? ri + Rc : -1.0, fk = cell ? fa * kappa : 0.0;
+        double S = 0.0;
+        for (int c0 = 0; c0 < nl; c0 += 32) {
+          double dij;
+          const int n = min(32, nl - c0), cb = s0 + c0;
+          const double iR = inverse(i, cb + lane, lane < n, dij);
+          for (int t = 0; t < n; ++t) {
+            const double rj = rs[(cb + t) * 32 + lane];
+            if (!__any_sync(0xffffffffu, rj < reach) || cb + t == a) continue;
+            const double iRt = __shfl_sync(0xffffffffu, iR, t), dt = __shfl_sync(0xffffffffu, dij, t);
+            const double mu = (ri - rj) * iRt;
+            double sv, ds, lam = 0.0;
+            becke_s_ds(mu, sv, ds);
+            if (rj > 0.0 && mu > -1.0 && mu < 1.0 && sv > 0.0) lam = fk * ds / sv * iRt;
+            S += lam;
+            Ds[(cb + t) * 32 + lane] -= lam;
+            if (dt < Rc) {
+              const double G = warp_sum(lam * mu);
+              if (lane < 3 && G != 0.0) {
+                const int j = list[cb + t];
+                const double e = G * (C[3 * i + lane] - C[3 * j + lane]) / dt;
+                atomicAdd(&Fa[3 * i + lane], -e);
+                atomicAdd(&Fa[3 * j + lane], e);
+              }
             }
           }
         }
+        if (S != 0.0) atomicAdd(&Ss[a * 32 + lane], S);
       }
-      Ds[a * 32 + lane] += A;
-    }
+    __syncthreads();
     // the u terms: per atom over the points, and per point to its owner
     double Fo[3] = {0.0, 0.0, 0.0};
-    for (int a = 0; a < nl; ++a) {
-      const double ra = rs[a * 32 + lane], D = Ds[a * 32 + lane];
+    for (int a = s0; a < s0 + nl; ++a) {
+      const double ra = rs[a * 32 + lane], D = Ds[a * 32 + lane] + Ss[a * 32 + lane];
       const double h = ra > 0.0 ? D / ra : 0.0;
       if (!__any_sync(0xffffffffu, h != 0.0)) continue;
       const int i = list[a];
@@ -640,21 +669,27 @@ __global__ void __launch_bounds__(32)
         if (lane == 0 && t != 0.0) atomicAdd(&Fa[3 * own + k], t);
       }
     }
-    __syncwarp();
   }
-  for (int e = lane; e < 3 * natoms; e += 32)
+  __syncthreads();
+  for (int e = threadIdx.x; e < 3 * natoms; e += blockDim.x)
     if (Fa[e] != 0.0) atomicAdd(&F[e], Fa[e]);
 }
 
 static void launch_becke_grad(Plan &P, const double *edens, double clamp, double *F, cudaStream_t s) {
   if (P.natoms <= kGradCap) {
-    const size_t smem = (size_t)P.natoms * (3 * 32 * sizeof(double) + 3 * sizeof(double) + sizeof(int));
-    NKX_CUDA(cudaFuncSetAttribute(becke_grad_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // as many warps as fit an SM's shared memory at once, at most 32
-    const long per_sm = std::min<long>(32, (long)((200 << 10) / (smem + 1024)));
-    const unsigned grid = (unsigned)std::min<long>(P.npad / 32, per_sm * P.nsm);
-    becke_grad_warp_kernel<<<grid, 32, smem, s>>>(P.d_centers, P.natoms, P.d_px, P.d_py, P.d_pz, P.d_w, P.d_owner,
-                                                  edens, P.npad, clamp, F);
+    auto go = [&](auto warps) {
+      constexpr int W = decltype(warps)::value;
+      const size_t smem = (size_t)((P.natoms + W - 1) / W * W) * kGradAtomBytes;
+      // the limit is the same for every call, so that threads cannot lower it for one another
+      NKX_CUDA(cudaFuncSetAttribute(becke_grad_warp_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(kGradCap * kGradAtomBytes)));
+      int per_sm = 1;
+      NKX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, becke_grad_warp_kernel<W>, 32 * W, smem));
+      const unsigned grid = (unsigned)std::min<long>(P.npad / 32, (long)std::max(1, per_sm) * P.nsm);
+      becke_grad_warp_kernel<W><<<grid, 32 * W, smem, s>>>(P.d_centers, P.natoms, P.d_px, P.d_py, P.d_pz, P.d_w,
+                                                          P.d_owner, edens, P.npad, clamp, F);
+    };
+    P.natoms <= kGradNarrow ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 8>{});
   } else {
     const size_t fs_bytes = sizeof(double) * 3 * (size_t)P.natoms;
     const bool smem = fs_bytes <= 48 * 1024;

@@ -46,3 +46,30 @@ def test_gradient_along_a_direction(n, nocc, nspin, lda):
         assert abs((F * d).sum() - ref) <= tol
         assert np.abs(F.sum(0)).max() <= 1e-9 * max(1.0, np.abs(F).max())
     fb.close()
+
+
+# the last and first sizes of four warps, of eight and of a thread per point for
+# the weights' term; one s function an atom, the bounds of the test above
+@pytest.mark.parametrize("natoms", [3, 48, 49, 192, 193])
+def test_weight_term_along_a_direction(natoms):
+    rng = np.random.default_rng(natoms)
+    c = 2.4 * np.array([[i % 6, i // 6 % 6, i // 36] for i in range(natoms)]) + rng.uniform(-0.3, 0.3, (natoms, 3))
+    Z, Cm, occ = np.ones(natoms, np.int32), M.random_orbitals(natoms, 2, seed=1), np.ones(2)
+
+    def plan(x):
+        g = A.make_flat_grid(x, Z, 20, 11, weight_threshold=-1.0, radial="ta")
+        return A.FockBuilder(x, Z, A.make_manual_basis([(1, 0, 0, 1.1, *r) for r in x]), g)
+
+    def energy(x):
+        fb = plan(x)
+        E = fb.build([Cm], [occ], precision="fp64")[0]
+        fb.close()
+        return E
+    d = rng.normal(size=c.shape)
+    d /= np.linalg.norm(d)
+    fd = [(energy(c + h * d) - energy(c - h * d)) / (2 * h) for h in (2e-3, 1e-3)]
+    fb = plan(c)
+    F = fb.xc_gradient([Cm], [occ])
+    fb.close()
+    assert abs((F * d).sum() - (4 * fd[1] - fd[0]) / 3) <= 2e-7
+    assert np.abs(F.sum(0)).max() <= 1e-9 * max(1.0, np.abs(F).max())
