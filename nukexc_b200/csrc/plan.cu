@@ -707,7 +707,7 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
         wr[k] = (k == 0 || hb) ? w[g] * r : 0.0;
 #pragma unroll
         for (int q = 0; q < QM; ++q) t[k][q] = q < G.n ? tab[(size_t)q * npad + g] : 0.0f;
-        solid_harmonics_all<L>(px[g] - G.cx, py[g] - G.cy, pz[g] - G.cz, S[k]);
+        solid_harmonics_const<L>(px[g] - G.cx, py[g] - G.cy, pz[g] - G.cz, S[k]);
       }
 #pragma unroll
       for (int q = 0; q < QM; ++q) {
@@ -724,7 +724,7 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
     if (wr == 0.0) continue;
     const double dx = px[g] - G.cx, dy = py[g] - G.cy, dz = pz[g] - G.cz;
     double S[NM];
-    solid_harmonics_all<L>(dx, dy, dz, S);
+    solid_harmonics_const<L>(dx, dy, dz, S);
     {
       const double rr = sqrt(dx * dx + dy * dy + dz * dz);
       const double r2l1inv = rr < 1e-12 ? 0.0 : ipow_c<2 * L + 1>(1.0 / rr);
@@ -761,7 +761,8 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
 
 // every group of every l in one launch (block x = group): with few centres
 // the launches of single l leave most SMs idle (one water, FP64: 149 us in
-// four launches, 107 in one; (H2O)_8, tables: 790 and 707).  The fixed-count shell loops come in quarters
+// four launches, 107 in one; (H2O)_8, tables: 790 and 707; 97 and 324 with the
+// harmonics chosen at compile time).  The fixed-count shell loops come in quarters
 // of the l's largest group, so that a group of 6 s shells does not pay for 16.
 template <bool TAB>
 __global__ void __launch_bounds__(256, TAB ? 2 : 1)

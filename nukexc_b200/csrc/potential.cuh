@@ -9,6 +9,8 @@
 // the potential is the exact multipole C S_lm (n+l+1)! / (zeta^(n+l+2) r^(2l+1)).
 #pragma once
 
+#include <utility>
+
 #include "sto.cuh"
 
 namespace nkx {
@@ -132,6 +134,17 @@ template <int L>
 NKX_HD inline void solid_harmonics_all(double x, double y, double z, double S[2 * L + 1]) {
 #pragma unroll
   for (int m = -L; m <= L; ++m) S[m + L] = solid_harmonic(L, m, x, y, z);
+}
+// the same with every (l, m) a constant of its call, so that the case is chosen at
+// compile time (above, the switch stays in the code, which keeps the registers
+// of kernels low that hold little else)
+template <int L, int... K>
+NKX_HD inline void solid_harmonics_const(std::integer_sequence<int, K...>, double x, double y, double z, double *S) {
+  ((S[K] = solid_harmonic(L, K - L, x, y, z)), ...);
+}
+template <int L>
+NKX_HD inline void solid_harmonics_const(double x, double y, double z, double S[2 * L + 1]) {
+  solid_harmonics_const<L>(std::make_integer_sequence<int, 2 * L + 1>{}, x, y, z, S);
 }
 
 }  // namespace nkx
