@@ -707,7 +707,7 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
         wr[k] = (k == 0 || hb) ? w[g] * r : 0.0;
 #pragma unroll
         for (int q = 0; q < QM; ++q) t[k][q] = q < G.n ? tab[(size_t)q * npad + g] : 0.0f;
-        solid_harmonics_const<L>(px[g] - G.cx, py[g] - G.cy, pz[g] - G.cz, S[k]);
+        solid_harmonics_all<L>(px[g] - G.cx, py[g] - G.cy, pz[g] - G.cz, S[k]);
       }
 #pragma unroll
       for (int q = 0; q < QM; ++q) {
@@ -724,7 +724,7 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
     if (wr == 0.0) continue;
     const double dx = px[g] - G.cx, dy = py[g] - G.cy, dz = pz[g] - G.cz;
     double S[NM];
-    solid_harmonics_const<L>(dx, dy, dz, S);
+    solid_harmonics_all<L>(dx, dy, dz, S);
     {
       const double rr = sqrt(dx * dx + dy * dy + dz * dz);
       const double r2l1inv = rr < 1e-12 ? 0.0 : ipow_c<2 * L + 1>(1.0 / rr);
@@ -835,6 +835,16 @@ __global__ void __launch_bounds__(256) aux_y_reduce_kernel(const double *__restr
   if (lane == 0) y[a] = s;
 }
 
+// sum_m c_m S_lm of a loose shell (any l): a call, so that the switch over all
+// harmonics takes no registers from the groups' loops
+__device__ __noinline__ double aux_loose_sum(const AuxShell &sh, const double *__restrict__ c, double dx, double dy,
+                                             double dz) {
+  double a = 0.0;
+#pragma unroll 1
+  for (int m = 0; m < sh.nm; ++m) a += c[sh.first + m] * solid_harmonic(sh.f.l, sh.f.m + m, dx, dy, dz);
+  return a;
+}
+
 // v_g = w_g sum_a c_a V_a(g) over the groups, then the loose shells
 // (coulomb.hpp:90-95)
 // v of two points (ga, gb) from one group with the C R table: the group's
@@ -849,6 +859,7 @@ __device__ __forceinline__ void aux_group_v2_tab(const AuxGroup &G, const AuxShe
   double S[2][NM];
   solid_harmonics_all<L>(x[0] - G.cx, y[0] - G.cy, z[0] - G.cz, S[0]);
   solid_harmonics_all<L>(x[1] - G.cx, y[1] - G.cy, z[1] - G.cz, S[1]);
+#pragma unroll 2
   for (int q = 0; q < G.n; ++q) {
     const int f0 = shells[G.first + q].first;
     const float *row = rtab + (size_t)(G.first + q) * npad;
@@ -865,44 +876,50 @@ __device__ __forceinline__ void aux_group_v2_tab(const AuxGroup &G, const AuxShe
   }
 }
 
-// the table form of aux_v_group_kernel: two points per thread
-__global__ void aux_v_group_tab_kernel(const AuxGroup *__restrict__ groups, int4 goff,
-                                       const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
-                                       const double *__restrict__ c, const double *__restrict__ px,
-                                       const double *__restrict__ py, const double *__restrict__ pz,
-                                       const double *__restrict__ w, long npad, const float *__restrict__ rtab,
-                                       double *__restrict__ v) {
+// the table form of aux_v_group_kernel: two points per thread.  ((H2O)_8, 1144
+// functions: 672 us with the harmonics' switch in the loops, 500 now; the bounds
+// on the registers, here and below, are for aux_loose_sum, which alone would take
+// 160: without them 742 us, and 78 instead of 52 for one water in FP64)
+__global__ void __launch_bounds__(256, 3)
+    aux_v_group_tab_kernel(const AuxGroup *__restrict__ groups, int4 goff,
+                           const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
+                           const double *__restrict__ c, const double *__restrict__ px,
+                           const double *__restrict__ py, const double *__restrict__ pz,
+                           const double *__restrict__ w, long npad, const float *__restrict__ rtab,
+                           double *__restrict__ v) {
   const long ga = blockIdx.x * 2L * blockDim.x + threadIdx.x;
   if (ga >= npad) return;
   const long gb = min(ga + (long)blockDim.x, npad - 1);  // a duplicate of the last point when past the end
   const double x[2] = {px[ga], px[gb]}, y[2] = {py[ga], py[gb]}, z[2] = {pz[ga], pz[gb]};
   double s[2] = {0.0, 0.0};
+#pragma unroll 1
   for (int k = 0; k < goff.x; ++k) aux_group_v2_tab<0>(groups[k], shells, c, x, y, z, rtab, npad, ga, gb, s);
+#pragma unroll 1
   for (int k = goff.x; k < goff.y; ++k) aux_group_v2_tab<1>(groups[k], shells, c, x, y, z, rtab, npad, ga, gb, s);
+#pragma unroll 1
   for (int k = goff.y; k < goff.z; ++k) aux_group_v2_tab<2>(groups[k], shells, c, x, y, z, rtab, npad, ga, gb, s);
+#pragma unroll 1
   for (int k = goff.z; k < goff.w; ++k) aux_group_v2_tab<3>(groups[k], shells, c, x, y, z, rtab, npad, ga, gb, s);
   for (int k = 0; k < nloose; ++k) {
     const AuxShell &sh = shells[loose[k]];
     const AuxFunc &f = sh.f;
     const float *row = rtab + (size_t)loose[k] * npad;
-    for (int e = 0; e < 2; ++e) {
-      double a = 0.0;
-      for (int m = 0; m < sh.nm; ++m)
-        a += c[sh.first + m] * solid_harmonic(f.l, f.m + m, x[e] - f.cx, y[e] - f.cy, z[e] - f.cz);
-      s[e] += a * (double)row[e ? gb : ga];
-    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      s[e] += aux_loose_sum(sh, c, x[e] - f.cx, y[e] - f.cy, z[e] - f.cz) * (double)row[e ? gb : ga];
   }
   v[ga] = s[0] * w[ga];
   if (ga + (long)blockDim.x < npad) v[gb] = s[1] * w[gb];
 }
 
 template <bool TAB>
-__global__ void aux_v_group_kernel(const AuxGroup *__restrict__ groups, int4 goff,
-                                   const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
-                                   const double *__restrict__ c, const double *__restrict__ px,
-                                   const double *__restrict__ py, const double *__restrict__ pz,
-                                   const double *__restrict__ w, long npad, const float *__restrict__ rtab,
-                                   double *__restrict__ v) {
+__global__ void __launch_bounds__(128, 6)
+    aux_v_group_kernel(const AuxGroup *__restrict__ groups, int4 goff,
+                       const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
+                       const double *__restrict__ c, const double *__restrict__ px,
+                       const double *__restrict__ py, const double *__restrict__ pz,
+                       const double *__restrict__ w, long npad, const float *__restrict__ rtab,
+                       double *__restrict__ v) {
   const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (g >= npad) return;
   if (w[g] == 0.0) {
@@ -912,16 +929,19 @@ __global__ void aux_v_group_kernel(const AuxGroup *__restrict__ groups, int4 gof
   const double x = px[g], y = py[g], z = pz[g];
   double s = 0.0;
   // groups sorted by l: [0, goff.x) l = 0, [goff.x, goff.y) l = 1, ...
+#pragma unroll 1
   for (int k = 0; k < goff.x; ++k) s += aux_group_v<0, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+#pragma unroll 1
   for (int k = goff.x; k < goff.y; ++k) s += aux_group_v<1, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+#pragma unroll 1
   for (int k = goff.y; k < goff.z; ++k) s += aux_group_v<2, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+#pragma unroll 1
   for (int k = goff.z; k < goff.w; ++k) s += aux_group_v<3, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
   for (int k = 0; k < nloose; ++k) {
     const AuxShell &sh = shells[loose[k]];
     const AuxFunc &f = sh.f;
     const double dx = x - f.cx, dy = y - f.cy, dz = z - f.cz;
-    double a = 0.0;
-    for (int m = 0; m < sh.nm; ++m) a += c[sh.first + m] * solid_harmonic(f.l, f.m + m, dx, dy, dz);
+    const double a = aux_loose_sum(sh, c, dx, dy, dz);
     if (a != 0.0)
       s += a * (TAB ? (double)rtab[(size_t)loose[k] * npad + g] : f.C * aux_radial(f, sqrt(dx * dx + dy * dy + dz * dz)));
   }

@@ -129,22 +129,16 @@ struct AuxGroup {
 };
 NKX_HD constexpr int aux_group_max(int l) { return (32 / (2 * l + 1)) < 16 ? (32 / (2 * l + 1)) : 16; }
 
-// the 2L+1 real solid harmonics of degree L at (x, y, z), m = -L..L
-template <int L>
-NKX_HD inline void solid_harmonics_all(double x, double y, double z, double S[2 * L + 1]) {
-#pragma unroll
-  for (int m = -L; m <= L; ++m) S[m + L] = solid_harmonic(L, m, x, y, z);
-}
-// the same with every (l, m) a constant of its call, so that the case is chosen at
-// compile time (above, the switch stays in the code, which keeps the registers
-// of kernels low that hold little else)
+// the 2L+1 real solid harmonics of degree L at (x, y, z), m = -L..L; every call
+// has constant (l, m), so its case is chosen at compile time (in an unrolled
+// loop over m the switch itself stayed in the code)
 template <int L, int... K>
-NKX_HD inline void solid_harmonics_const(std::integer_sequence<int, K...>, double x, double y, double z, double *S) {
+NKX_HD inline void solid_harmonics_all(std::integer_sequence<int, K...>, double x, double y, double z, double *S) {
   ((S[K] = solid_harmonic(L, K - L, x, y, z)), ...);
 }
 template <int L>
-NKX_HD inline void solid_harmonics_const(double x, double y, double z, double S[2 * L + 1]) {
-  solid_harmonics_const<L>(std::make_integer_sequence<int, 2 * L + 1>{}, x, y, z, S);
+NKX_HD inline void solid_harmonics_all(double x, double y, double z, double S[2 * L + 1]) {
+  solid_harmonics_all<L>(std::make_integer_sequence<int, 2 * L + 1>{}, x, y, z, S);
 }
 
 }  // namespace nkx
