@@ -386,8 +386,9 @@ NKX_API nkx_status nkx_plan_set_half_inverse(nkx_plan *plan, int K, const double
  * around one graph launch, so the caller may pass other buffers each time,
  * as an SCF loop on the device does.  Any other build, or any change of the
  * plan (functional, metric, half inverse, wait limit, tuning, chunking),
- * drops the graphs; a kind that cannot be recorded keeps running ordinary
- * builds.  Replays record no stage times (nkx_get_last_timing gives the
+ * drops the graphs, and so does a mixed nuclear gradient that needs larger
+ * buffers than the builds have; a kind that cannot be recorded keeps running
+ * ordinary builds.  Replays record no stage times (nkx_get_last_timing gives the
  * total); nkx_plan_info.graph_replays counts them. */
 NKX_API nkx_status nkx_plan_set_graph(nkx_plan *plan, int enable);
 

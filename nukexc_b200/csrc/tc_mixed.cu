@@ -2023,9 +2023,13 @@ static void launch_colloc_z(Plan &P, MixedState &M, const Chunk &c, int nzs, int
 void mixed_gradient_begin(Plan &P, int nspin, int nocc, cudaStream_t s) {
   MixedState &M = mixed_state(P, nocc);
   const int nc = P.gga ? 4 : 1;
-  M.ensure_T((size_t)M.nbatch_chunk * nspin * nc * M.nocc_pad * 256);
-  M.ensure_qt0((size_t)M.nbatch_chunk * nspin * nc * 2 * 4 * 128 * M.nocc_pad,
-               (long)M.nbatch_chunk * nspin * nc * 2 * 4, M.nocc_pad);
+  const size_t T_need = (size_t)M.nbatch_chunk * nspin * nc * M.nocc_pad * 256;
+  const size_t qt0_need = (size_t)M.nbatch_chunk * nspin * nc * 2 * 4 * 128 * M.nocc_pad;
+  // the mixed builds use smaller T and qt0, whose addresses their recorded
+  // graphs hold: these go before the buffers do
+  if (T_need > M.T_cap || qt0_need > M.qt0_cap) P.drop_graphs();
+  M.ensure_T(T_need);
+  M.ensure_qt0(qt0_need, (long)M.nbatch_chunk * nspin * nc * 2 * 4, M.nocc_pad);
   M.ensure_X((size_t)M.cap * nspin * nc * kBatch * kBlockF);
   const long rows = (long)nspin * M.nocc_pad * P.nblk;
   quant_ct_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, s>>>(P.d_Ct, nocc, M.nocc_pad, nspin, P.nbf_pad,
