@@ -138,7 +138,8 @@ NKX_API nkx_status nkx_make_flat_grid(const nkx_molecule *mol, const nkx_grid_sp
  * on device buffers: weights[g] *= P_owner(g) / sum_i P_i.  clamp > 0 is the
  * Laqua-clamped team variant (R_ij = min(|A_i - A_j|, clamp)), clamp <= 0 the
  * original Becke.  centers[3*natoms], points[3*npts] (AoS, like
- * Kokkos::View<Point*>). */
+ * Kokkos::View<Point*>).  A point whose owner is outside [0, natoms) gets
+ * weight 0. */
 NKX_API nkx_status nkx_becke_partition(const double *d_centers, int natoms, const double *d_points,
                                        const int *d_owner, long npts, double *d_weights, double clamp,
                                        void *stream);

@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(32 * W)
 #pragma unroll
   for (int v = 0; v < W; ++v) r2min = fmin(r2min, red[0][v][lane]);
   const double rmin = sqrt(r2min), lim = rmin + 2.0 * Rc;
-  const bool live = in && dist3(pt, centers + 3 * own) < rmin + Rc;
+  // an owner outside [0, natoms) is no atom's index: nothing is read for it and the weight is 0
+  const bool live = in && (unsigned)own < (unsigned)natoms && dist3(pt, centers + 3 * own) < rmin + Rc;
   if (warp == 0 && in && !live) w[g] *= 0.0;  // P_owner == 0 exactly
   if (!__any_sync(0xffffffffu, live)) return;  // alike in every warp
   int nl = 0;
