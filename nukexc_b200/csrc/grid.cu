@@ -141,8 +141,9 @@ __global__ void __launch_bounds__(32 * W)
   const double *p = pts + 3 * (in ? g : npts - 1);
   const double pt[3] = {p[0], p[1], p[2]};
   const int own = owner[in ? g : npts - 1];
-  const double Rc = clamp > 0.0 ? clamp : 1e300;  // unclamped: no atom is screened
-  double r2min = 1e300;
+  const bool clamped = clamp > 0.0;  // else no atom is screened
+  const double Rc = clamped ? clamp : INFINITY;
+  double r2min = INFINITY;  // stays so where a coordinate is NaN or infinite
   for (int i = warp; i < natoms; i += W) {
     const double dx = pt[0] - centers[3 * i], dy = pt[1] - centers[3 * i + 1], dz = pt[2] - centers[3 * i + 2];
     r2min = fmin(r2min, dx * dx + dy * dy + dz * dz);
@@ -153,13 +154,14 @@ __global__ void __launch_bounds__(32 * W)
   for (int v = 0; v < W; ++v) r2min = fmin(r2min, red[0][v][lane]);
   const double rmin = sqrt(r2min), lim = rmin + 2.0 * Rc;
   // an owner outside [0, natoms) is no atom's index: nothing is read for it and the weight is 0
-  const bool live = in && (unsigned)own < (unsigned)natoms && dist3(pt, centers + 3 * own) < rmin + Rc;
-  if (warp == 0 && in && !live) w[g] *= 0.0;  // P_owner == 0 exactly
+  const bool live = in && (unsigned)own < (unsigned)natoms && (!clamped || dist3(pt, centers + 3 * own) < rmin + Rc);
+  // P_owner == 0 exactly; a point without a place keeps the 0 / 0 of the full loop, so that a build on it reports it
+  if (warp == 0 && in && !live) w[g] *= rmin < INFINITY ? 0.0 : NAN;
   if (!__any_sync(0xffffffffu, live)) return;  // alike in every warp
   int nl = 0;
   for (int j = warp; j < natoms; j += W) {
     const double r = dist3(pt, centers + 3 * j);
-    if (!__any_sync(0xffffffffu, live && r < lim)) continue;
+    if (!__any_sync(0xffffffffu, live && (!clamped || r < lim))) continue;
     rsm[(s0 + nl) * 32 + lane] = r;
     if (lane == 0) list[s0 + nl] = j;
     ++nl;
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(32 * W)
   double norm = 0.0, pown = 0.0;
   for (int a = s0; a < s0 + nl; ++a) {
     const double ri = rsm[a * 32 + lane];
-    const bool cell = live && ri < rmin + Rc;  // else P_i == 0 exactly
+    const bool cell = live && (!clamped || ri < rmin + Rc);  // else P_i == 0 exactly
     if (!__any_sync(0xffffffffu, cell)) continue;
     const int i = list[a];
     const double reach = cell ? ri + Rc : -1.0;  // factors of atoms at reach and beyond are 1
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(32 * W)
         if (lane < n && cb + lane != a) iR = 1.0 / fmin(dist3(centers + 3 * i, centers + 3 * list[cb + lane]), Rc);
         for (int t = 0; t < n; ++t) {
           const double rj = rsm[(cb + t) * 32 + lane];
-          if (!__any_sync(0xffffffffu, rj < reach) || cb + t == a) continue;
+          if ((clamped && !__any_sync(0xffffffffu, rj < reach)) || cb + t == a) continue;
           P *= becke_s((ri - rj) * __shfl_sync(0xffffffffu, iR, t));
         }
       }

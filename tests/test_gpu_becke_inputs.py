@@ -1,6 +1,7 @@
 """Becke weights of inputs that no grid should hold.  An owner outside
-[0, natoms) owns nothing: weight 0.  The other points of the same warp keep
-their weights.  Sizes of each path: four warps, eight, and
+[0, natoms) owns nothing: weight 0.  A point with a NaN or infinite coordinate
+has no weight: NaN, so that a build on it reports the point.  The other points
+of the same warp keep their weights.  Sizes of each path: four warps, eight, and
 a thread per point; with the clamp and without."""
 import numpy as np
 import pytest
@@ -36,3 +37,14 @@ def test_owner_of_no_atom_has_no_weight(natoms, clamp):
     got = _weights(c, pts, own, w, clamp)
     bad = np.isin(np.arange(70), [1, 33, 64])
     assert (got[bad] == 0.0).all() and (got[~bad] == ref[~bad]).all()
+
+
+@pytest.mark.parametrize("clamp", [5.0, 0.0])
+@pytest.mark.parametrize("natoms", SIZES)
+def test_point_without_a_place_has_no_finite_weight(natoms, clamp):
+    c, own, pts, w = _case(natoms)
+    ref = _weights(c, pts, own, w, clamp)
+    pts[2, 1], pts[40], pts[65, 0] = np.nan, np.nan, np.inf
+    got = _weights(c, pts, own, w, clamp)
+    bad = np.isin(np.arange(70), [2, 40, 65])
+    assert np.isnan(got[bad]).all() and (got[~bad] == ref[~bad]).all()
