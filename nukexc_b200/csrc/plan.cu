@@ -1424,9 +1424,15 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
   for (long b = 0; b < P.nbatch; ++b)
     for (int d = 0; d < 3; ++d) {
       const std::vector<double> &h = d == 0 ? hx : d == 1 ? hy : hz;
-      const auto mm = std::minmax_element(h.begin() + b * kBatch, h.begin() + (b + 1) * kBatch);
-      blo[3 * b + d] = *mm.first;
-      bhi[3 * b + d] = *mm.second;
+      // a NaN compares false and stays out of the box, so that its batch is
+      // not screened away and the point shows in the build
+      double lo = 1e300, hi = -1e300;
+      for (long p = b * kBatch; p < (b + 1) * kBatch; ++p) {
+        lo = std::min(lo, h[p]);
+        hi = std::max(hi, h[p]);
+      }
+      blo[3 * b + d] = lo;
+      bhi[3 * b + d] = hi;
     }
   if (P.nblk > 1) group_by_reach(*prim, tol, P.nbatch, blo, bhi, order, cut);
   std::vector<StoFunc> tab(P.nbf_pad);
