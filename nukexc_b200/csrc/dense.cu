@@ -175,7 +175,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int i = (t / ksteps) * NT + 8 * n + 2 * fk + h;
-          const double o = i < nocc ? occ[i] : 0.0;
+          if (i >= nocc) continue;  // a zero column, but 0 x Inf is NaN
+          const double o = occ[i];
 #pragma unroll
           for (int m = 0; m < 4; ++m) sm[m] += o * acc[GRAD ? 0 : m][n][h] * acc[m][n][h];
         }
