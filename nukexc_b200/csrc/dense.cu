@@ -24,15 +24,17 @@ nkx_status run_guarded(const char *where, const std::function<void()> &fn);
 // library's own, one per device, allocated and freed in stream order: a call
 // allocates and frees up to a few hundred megabytes, which took cudaMalloc /
 // cudaFree 1 to 3 ms (and a device-wide synchronisation) against 0.1 to 0.5 ms
-// of kernels.  The pool keeps at most kPoolKeep bytes between calls and gives
-// them back when a plan's allocation fails.
+// of kernels.  The pool keeps at most kPoolKeep bytes between calls: workspaces
+// are freed before a call's last synchronisation, which is when the pool gives
+// back what exceeds that.  What it keeps is not lost to the process: the driver
+// takes it back for a cudaMalloc that would fail otherwise.
 constexpr uint64_t kPoolKeep = (uint64_t)256 << 20;
-static cudaMemPool_t workspace_pool(int dev, bool create) {
+static cudaMemPool_t workspace_pool(int dev) {
   static std::mutex mu;
   static cudaMemPool_t pools[128] = {};
   NKX_REQUIRE(dev >= 0 && dev < 128, NKX_ERR_ARG, "device ordinal out of range");
   std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev] && create) {
+  if (!pools[dev]) {
     cudaMemPoolProps p{};
     p.allocType = cudaMemAllocationTypePinned;
     p.location.type = cudaMemLocationTypeDevice;
@@ -45,11 +47,6 @@ static cudaMemPool_t workspace_pool(int dev, bool create) {
   }
   return pools[dev];
 }
-void trim_workspace_pool() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  if (cudaMemPool_t pool = workspace_pool(dev, false)) cudaMemPoolTrimTo(pool, 0);
-}
 
 template <class T>
 struct DevBuf {
@@ -59,7 +56,7 @@ struct DevBuf {
     if (!n) return;
     int dev = 0;
     NKX_CUDA(cudaGetDevice(&dev));
-    NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev, true), s));
+    NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev), s));
   }
   ~DevBuf() {
     if (p) cudaFreeAsync(p, s);
@@ -67,6 +64,13 @@ struct DevBuf {
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
 };
+
+// fn's work on s, then the wait for it, with fn's workspaces freed in between
+template <class F>
+static void run_and_wait(cudaStream_t s, F &&fn) {
+  fn();
+  NKX_CUDA(cudaStreamSynchronize(s));
+}
 
 // fill_collocation / fill_grad_collocation, a thread per element (one water,
 // 68k points: 50 us with gradients; a thread per point and run of functions
@@ -666,18 +670,20 @@ extern "C" nkx_status nkx_xc_dense(int nbf, long npts, const double *d_phi, cons
     const bool gga = spec_is_gga(sp);
     NKX_REQUIRE(!gga || (d_gx && d_gy && d_gz), NKX_ERR_ARG, "GGA needs collocation gradients");
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf<double> rho((size_t)nspin * npts, s), grad((size_t)nspin * 3 * npts, s), Z((size_t)nspin * nbf * npts, s), Ed(1, s);
-    for (int sp_i = 0; sp_i < nspin; ++sp_i)
-      launch_density_dense(nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
-                           d_occ + (size_t)sp_i * nocc, rho.p + (size_t)sp_i * npts,
-                           gga ? grad.p + (size_t)sp_i * 3 * npts : nullptr, nullptr, s);
-    NKX_CUDA(cudaMemsetAsync(Ed.p, 0, sizeof(double), s));
-    launch_xc_z_dense(sp, gga, nbf, npts, nspin, d_phi, d_gx, d_gy, d_gz, d_w, rho.p, grad.p, Z.p, Ed.p, s);
-    for (int sp_i = 0; sp_i < nspin; ++sp_i)
-      launch_nt_gemm_sym(nbf, npts, d_phi, Z.p + (size_t)sp_i * nbf * npts, d_V + (size_t)sp_i * nbf * nbf, s);
-    NKX_LAUNCH_CHECK();
-    NKX_CUDA(cudaMemcpyAsync(E, Ed.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-    NKX_CUDA(cudaStreamSynchronize(s));
+    run_and_wait(s, [&] {
+      DevBuf<double> rho((size_t)nspin * npts, s), grad((size_t)nspin * 3 * npts, s), Z((size_t)nspin * nbf * npts, s),
+          Ed(1, s);
+      for (int sp_i = 0; sp_i < nspin; ++sp_i)
+        launch_density_dense(nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
+                             d_occ + (size_t)sp_i * nocc, rho.p + (size_t)sp_i * npts,
+                             gga ? grad.p + (size_t)sp_i * 3 * npts : nullptr, nullptr, s);
+      NKX_CUDA(cudaMemsetAsync(Ed.p, 0, sizeof(double), s));
+      launch_xc_z_dense(sp, gga, nbf, npts, nspin, d_phi, d_gx, d_gy, d_gz, d_w, rho.p, grad.p, Z.p, Ed.p, s);
+      for (int sp_i = 0; sp_i < nspin; ++sp_i)
+        launch_nt_gemm_sym(nbf, npts, d_phi, Z.p + (size_t)sp_i * nbf * npts, d_V + (size_t)sp_i * nbf * nbf, s);
+      NKX_LAUNCH_CHECK();
+      NKX_CUDA(cudaMemcpyAsync(E, Ed.p, sizeof(double), cudaMemcpyDeviceToHost, s));
+    });
   });
 }
 
@@ -764,17 +770,18 @@ extern "C" nkx_status nkx_coulomb_dense(int nbf, int naux, long npts, const doub
     // about eight blocks an SM over (32-function tiles) x (slices of 128 points and more)
     const long na = (naux + 31) / 32, nsl = std::max<long>(1, std::min<long>((8 * 148 + na - 1) / na, npts / 128));
     const long slice = (npts + nsl - 1) / nsl;
-    DevBuf<double> rho(npts, s), y(naux, s), t(K, s), c(naux, s), v(npts, s), part((size_t)nsl * naux, s);
-    launch_density_dense(nbf, npts, d_phi, nullptr, nullptr, nullptr, nocc, d_C, d_occ, rho.p, nullptr, nullptr, s);
-    vw_rho_kernel<<<dim3((unsigned)na, (unsigned)nsl), 256, 0, s>>>(naux, npts, slice, d_Vw, rho.p, part.p);
-    rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, (int)nsl, part.p, nullptr, y.p);
-    columns_dot_kernel<<<nblk(K * 32L, 256), 256, 0, s>>>(naux, K, d_X, y.p, t.p);
-    rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, K, d_X, t.p, c.p);
-    columns_dot_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(naux, npts, d_Vw, c.p, v.p);
-    NKX_LAUNCH_CHECK();
-    launch_nt_gemm_sym(nbf, npts, d_phi, d_phi, d_J, s, v.p);
-    NKX_LAUNCH_CHECK();
-    NKX_CUDA(cudaStreamSynchronize(s));
+    run_and_wait(s, [&] {
+      DevBuf<double> rho(npts, s), y(naux, s), t(K, s), c(naux, s), v(npts, s), part((size_t)nsl * naux, s);
+      launch_density_dense(nbf, npts, d_phi, nullptr, nullptr, nullptr, nocc, d_C, d_occ, rho.p, nullptr, nullptr, s);
+      vw_rho_kernel<<<dim3((unsigned)na, (unsigned)nsl), 256, 0, s>>>(naux, npts, slice, d_Vw, rho.p, part.p);
+      rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, (int)nsl, part.p, nullptr, y.p);
+      columns_dot_kernel<<<nblk(K * 32L, 256), 256, 0, s>>>(naux, K, d_X, y.p, t.p);
+      rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, K, d_X, t.p, c.p);
+      columns_dot_kernel<<<nblk(npts * 32, 256), 256, 0, s>>>(naux, npts, d_Vw, c.p, v.p);
+      NKX_LAUNCH_CHECK();
+      launch_nt_gemm_sym(nbf, npts, d_phi, d_phi, d_J, s, v.p);
+      NKX_LAUNCH_CHECK();
+    });
   });
 }
 
@@ -794,27 +801,30 @@ extern "C" nkx_status nkx_exchange_dense(int nbf, int naux, long npts, const dou
     std::vector<double> occ(nocc);
     NKX_CUDA(cudaMemcpyAsync(occ.data(), d_occ, sizeof(double) * nocc, cudaMemcpyDeviceToHost, s));
     NKX_CUDA(cudaStreamSynchronize(s));
-    DevBuf<double> T((size_t)npts * nocc, s), B((size_t)nbf * npts, s), P3((size_t)naux * nbf, s), Y((size_t)nbf * K, s);
-    cublasHandle_t h;
-    NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
-    cublasSetStream(h, s);
-    const double one = 1.0, zero = 0.0;
-    bool ok = cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, (int)npts, nocc, nbf, &one, d_phi, nbf, d_C, nbf, &zero, T.p,
-                          (int)npts) == CUBLAS_STATUS_SUCCESS;
-    ok = ok && cudaMemsetAsync(d_K, 0, sizeof(double) * nbf * nbf, s) == cudaSuccess;
-    for (int i = 0; i < nocc && ok; ++i) {
-      scale_columns_kernel<<<nblk((long)nbf * npts, 256), 256, 0, s>>>(nbf, npts, d_phi, T.p + (size_t)i * npts,
-                                                                        B.p);
-      ok = cudaGetLastError() == cudaSuccess;
-      ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, naux, nbf, (int)npts, &one, d_Vw, naux, B.p, nbf, &zero,
-                             P3.p, naux) == CUBLAS_STATUS_SUCCESS;
-      ok = ok && cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, nbf, K, naux, &one, P3.p, naux, d_X, naux, &zero, Y.p,
-                             nbf) == CUBLAS_STATUS_SUCCESS;
-      const double oi = occ[i];
-      ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, K, &oi, Y.p, nbf, Y.p, nbf, &one, d_K, nbf) ==
-                     CUBLAS_STATUS_SUCCESS;
-    }
-    NKX_CUDA(cudaStreamSynchronize(s));
+    cublasHandle_t h = nullptr;
+    bool ok = true;
+    run_and_wait(s, [&] {
+      DevBuf<double> T((size_t)npts * nocc, s), B((size_t)nbf * npts, s), P3((size_t)naux * nbf, s),
+          Y((size_t)nbf * K, s);
+      NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
+      cublasSetStream(h, s);
+      const double one = 1.0, zero = 0.0;
+      ok = cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, (int)npts, nocc, nbf, &one, d_phi, nbf, d_C, nbf, &zero, T.p,
+                       (int)npts) == CUBLAS_STATUS_SUCCESS;
+      ok = ok && cudaMemsetAsync(d_K, 0, sizeof(double) * nbf * nbf, s) == cudaSuccess;
+      for (int i = 0; i < nocc && ok; ++i) {
+        scale_columns_kernel<<<nblk((long)nbf * npts, 256), 256, 0, s>>>(nbf, npts, d_phi, T.p + (size_t)i * npts,
+                                                                          B.p);
+        ok = cudaGetLastError() == cudaSuccess;
+        ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, naux, nbf, (int)npts, &one, d_Vw, naux, B.p, nbf, &zero,
+                               P3.p, naux) == CUBLAS_STATUS_SUCCESS;
+        ok = ok && cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, nbf, K, naux, &one, P3.p, naux, d_X, naux, &zero, Y.p,
+                               nbf) == CUBLAS_STATUS_SUCCESS;
+        const double oi = occ[i];
+        ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, K, &oi, Y.p, nbf, Y.p, nbf, &one, d_K, nbf) ==
+                       CUBLAS_STATUS_SUCCESS;
+      }
+    });
     cublasDestroy(h);
     NKX_REQUIRE(ok, NKX_ERR_CUDA, "cuBLAS call in nkx_exchange_dense failed");
   });
@@ -851,47 +861,48 @@ extern "C" nkx_status nkx_core_hamiltonian_dense(const nkx_basis *basis, const n
     cudaStream_t s = (cudaStream_t)stream;
     const int nbf = basis->nbf;
     auto tab = make_sto_table(*basis);
-    DevBuf<StoFunc> df(tab.size(), s);
-    NKX_CUDA(cudaMemcpyAsync(df.p, tab.data(), sizeof(StoFunc) * tab.size(), cudaMemcpyHostToDevice, s));
     std::vector<double> zc(mol->natoms);
     for (int a = 0; a < mol->natoms; ++a) zc[a] = mol->Z[a];
-    DevBuf<double> dc(3 * (size_t)mol->natoms, s), dz(mol->natoms, s);
-    NKX_CUDA(cudaMemcpyAsync(dc.p, mol->xyz, sizeof(double) * 3 * mol->natoms, cudaMemcpyHostToDevice, s));
-    NKX_CUDA(cudaMemcpyAsync(dz.p, zc.data(), sizeof(double) * mol->natoms, cudaMemcpyHostToDevice, s));
-    // points in chunks holding 6 nbf x chunk matrices in about 1 GiB
-    const long chunk = std::max<long>(256, std::min<long>(npts, ((long)1 << 27) / (6L * nbf)));
-    DevBuf<double> phi((size_t)nbf * chunk, s), gx((size_t)nbf * chunk, s), gy((size_t)nbf * chunk, s),
-        gz((size_t)nbf * chunk, s), sc((size_t)nbf * chunk, s), wv(chunk, s);
-    NKX_CUDA(cudaMemsetAsync(d_S, 0, sizeof(double) * nbf * nbf, s));
-    NKX_CUDA(cudaMemsetAsync(d_T, 0, sizeof(double) * nbf * nbf, s));
-    NKX_CUDA(cudaMemsetAsync(d_V, 0, sizeof(double) * nbf * nbf, s));
-    cublasHandle_t h;
-    NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
-    cublasSetStream(h, s);
+    cublasHandle_t h = nullptr;
     bool ok = true;
-    const double one = 1.0, half = 0.5, mone = -1.0;
-    for (long g0 = 0; g0 < npts && ok; g0 += chunk) {
-      const long n = std::min(chunk, npts - g0);
-      const long tot = (long)nbf * n;
-      colloc_dense_kernel<<<nblk(tot, 128), 128, 0, s>>>(df.p, nbf, d_points + 3 * g0, n, phi.p, gx.p, gy.p, gz.p);
-      core_weights_kernel<<<nblk(n, 128), 128, 0, s>>>(d_points + 3 * g0, d_w + g0, n, dc.p, dz.p, mol->natoms, wv.p);
-      // S += phi (w phi)^T
-      scale_cols_kernel<<<nblk(tot, 256), 256, 0, s>>>(nbf, n, phi.p, d_w + g0, sc.p);
-      ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)n, &one, phi.p, nbf, sc.p, nbf, &one, d_S,
-                             nbf) == CUBLAS_STATUS_SUCCESS;
-      // V -= phi (w v phi)^T
-      scale_cols_kernel<<<nblk(tot, 256), 256, 0, s>>>(nbf, n, phi.p, wv.p, sc.p);
-      ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)n, &mone, phi.p, nbf, sc.p, nbf, &one, d_V,
-                             nbf) == CUBLAS_STATUS_SUCCESS;
-      // T += 1/2 sum_k g_k (w g_k)^T
-      for (double *gk : {gx.p, gy.p, gz.p}) {
-        scale_cols_kernel<<<nblk(tot, 256), 256, 0, s>>>(nbf, n, gk, d_w + g0, sc.p);
-        ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)n, &half, gk, nbf, sc.p, nbf, &one, d_T,
+    run_and_wait(s, [&] {
+      DevBuf<StoFunc> df(tab.size(), s);
+      NKX_CUDA(cudaMemcpyAsync(df.p, tab.data(), sizeof(StoFunc) * tab.size(), cudaMemcpyHostToDevice, s));
+      DevBuf<double> dc(3 * (size_t)mol->natoms, s), dz(mol->natoms, s);
+      NKX_CUDA(cudaMemcpyAsync(dc.p, mol->xyz, sizeof(double) * 3 * mol->natoms, cudaMemcpyHostToDevice, s));
+      NKX_CUDA(cudaMemcpyAsync(dz.p, zc.data(), sizeof(double) * mol->natoms, cudaMemcpyHostToDevice, s));
+      // points in chunks holding 6 nbf x chunk matrices in about 1 GiB
+      const long chunk = std::max<long>(256, std::min<long>(npts, ((long)1 << 27) / (6L * nbf)));
+      DevBuf<double> phi((size_t)nbf * chunk, s), gx((size_t)nbf * chunk, s), gy((size_t)nbf * chunk, s),
+          gz((size_t)nbf * chunk, s), sc((size_t)nbf * chunk, s), wv(chunk, s);
+      NKX_CUDA(cudaMemsetAsync(d_S, 0, sizeof(double) * nbf * nbf, s));
+      NKX_CUDA(cudaMemsetAsync(d_T, 0, sizeof(double) * nbf * nbf, s));
+      NKX_CUDA(cudaMemsetAsync(d_V, 0, sizeof(double) * nbf * nbf, s));
+      NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
+      cublasSetStream(h, s);
+      const double one = 1.0, half = 0.5, mone = -1.0;
+      for (long g0 = 0; g0 < npts && ok; g0 += chunk) {
+        const long n = std::min(chunk, npts - g0);
+        const long tot = (long)nbf * n;
+        colloc_dense_kernel<<<nblk(tot, 128), 128, 0, s>>>(df.p, nbf, d_points + 3 * g0, n, phi.p, gx.p, gy.p, gz.p);
+        core_weights_kernel<<<nblk(n, 128), 128, 0, s>>>(d_points + 3 * g0, d_w + g0, n, dc.p, dz.p, mol->natoms, wv.p);
+        // S += phi (w phi)^T
+        scale_cols_kernel<<<nblk(tot, 256), 256, 0, s>>>(nbf, n, phi.p, d_w + g0, sc.p);
+        ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)n, &one, phi.p, nbf, sc.p, nbf, &one, d_S,
                                nbf) == CUBLAS_STATUS_SUCCESS;
+        // V -= phi (w v phi)^T
+        scale_cols_kernel<<<nblk(tot, 256), 256, 0, s>>>(nbf, n, phi.p, wv.p, sc.p);
+        ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)n, &mone, phi.p, nbf, sc.p, nbf, &one, d_V,
+                               nbf) == CUBLAS_STATUS_SUCCESS;
+        // T += 1/2 sum_k g_k (w g_k)^T
+        for (double *gk : {gx.p, gy.p, gz.p}) {
+          scale_cols_kernel<<<nblk(tot, 256), 256, 0, s>>>(nbf, n, gk, d_w + g0, sc.p);
+          ok = ok && cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, nbf, nbf, (int)n, &half, gk, nbf, sc.p, nbf, &one, d_T,
+                                 nbf) == CUBLAS_STATUS_SUCCESS;
+        }
+        ok = ok && cudaGetLastError() == cudaSuccess;
       }
-      ok = ok && cudaGetLastError() == cudaSuccess;
-    }
-    NKX_CUDA(cudaStreamSynchronize(s));
+    });
     cublasDestroy(h);
     NKX_REQUIRE(ok, NKX_ERR_CUDA, "kernel or cuBLAS failure in nkx_core_hamiltonian_dense");
   });
@@ -901,26 +912,27 @@ extern "C" nkx_status nkx_half_inverse(int N, const double *d_S, double thr, dou
   return run_guarded("nkx_half_inverse", [&] {
     NKX_REQUIRE(N > 0 && d_S && d_X && K, NKX_ERR_ARG, "invalid arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf<double> A((size_t)N * N, s), D(N, s), lam(N, s);
-    DevBuf<int> info(1, s);
-    dim3 tb(16, 16), gb(nblk(N, 16), nblk(N, 16));
-    precondition_kernel<<<gb, tb, 0, s>>>(N, d_S, A.p, D.p);
-    NKX_LAUNCH_CHECK();
-    cusolverDnHandle_t h;
-    NKX_REQUIRE(cusolverDnCreate(&h) == CUSOLVER_STATUS_SUCCESS, NKX_ERR_CUDA, "cusolverDnCreate failed");
-    cusolverDnSetStream(h, s);
-    int lwork = 0;
-    cusolverDnDsyevd_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N, lam.p, &lwork);
-    DevBuf<double> work(lwork > 0 ? lwork : 1, s);
-    const cusolverStatus_t st =
-        cusolverDnDsyevd(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N, lam.p, work.p, lwork, info.p);
-    cusolverDnDestroy(h);
-    NKX_REQUIRE(st == CUSOLVER_STATUS_SUCCESS, NKX_ERR_CUDA, "cusolverDnDsyevd failed");
     std::vector<double> hl(N), hU((size_t)N * N), hD(N);
-    NKX_CUDA(cudaMemcpyAsync(hl.data(), lam.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
-    NKX_CUDA(cudaMemcpyAsync(hU.data(), A.p, sizeof(double) * N * N, cudaMemcpyDeviceToHost, s));
-    NKX_CUDA(cudaMemcpyAsync(hD.data(), D.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
-    NKX_CUDA(cudaStreamSynchronize(s));
+    run_and_wait(s, [&] {
+      DevBuf<double> A((size_t)N * N, s), D(N, s), lam(N, s);
+      DevBuf<int> info(1, s);
+      dim3 tb(16, 16), gb(nblk(N, 16), nblk(N, 16));
+      precondition_kernel<<<gb, tb, 0, s>>>(N, d_S, A.p, D.p);
+      NKX_LAUNCH_CHECK();
+      cusolverDnHandle_t h;
+      NKX_REQUIRE(cusolverDnCreate(&h) == CUSOLVER_STATUS_SUCCESS, NKX_ERR_CUDA, "cusolverDnCreate failed");
+      cusolverDnSetStream(h, s);
+      int lwork = 0;
+      cusolverDnDsyevd_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N, lam.p, &lwork);
+      DevBuf<double> work(lwork > 0 ? lwork : 1, s);
+      const cusolverStatus_t st = cusolverDnDsyevd(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N,
+                                                   lam.p, work.p, lwork, info.p);
+      cusolverDnDestroy(h);
+      NKX_REQUIRE(st == CUSOLVER_STATUS_SUCCESS, NKX_ERR_CUDA, "cusolverDnDsyevd failed");
+      NKX_CUDA(cudaMemcpyAsync(hl.data(), lam.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
+      NKX_CUDA(cudaMemcpyAsync(hU.data(), A.p, sizeof(double) * N * N, cudaMemcpyDeviceToHost, s));
+      NKX_CUDA(cudaMemcpyAsync(hD.data(), D.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
+    });
     // singular values of a symmetric matrix are |eigenvalues|; keep s > thr,
     // largest first (the reference's SVD ordering)
     std::vector<int> order(N);

@@ -59,7 +59,6 @@ nkx_status run_guarded(const char *where, const std::function<void()> &fn) {
   }
 }
 
-void trim_workspace_pool();  // dense.cu
 XcSpec make_spec(const nkx_plan_options *o);
 bool spec_is_gga(const XcSpec &s);
 
@@ -67,12 +66,7 @@ template <class T>
 static T *dalloc(size_t n) {
   T *p = nullptr;
   if (n == 0) return nullptr;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    trim_workspace_pool();  // give back what the dense entry points keep
-    e = cudaMalloc(&p, n * sizeof(T));
-  }
+  const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
   if (e != cudaSuccess) {
     cudaGetLastError();
     throw Error{NKX_ERR_ALLOC, "cudaMalloc of " + std::to_string(n * sizeof(T)) + " bytes failed"};
