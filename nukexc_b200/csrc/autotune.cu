@@ -168,8 +168,8 @@ static void autotune(Plan &P, int nspin, int nocc, const double *C, const double
     }
     for (int mult : {2, 4}) {
       if (base_chunk * mult > P.npairs * 2) break;  // already one chunk
-      size_t fr = 0, tot = 0;
-      NKX_CUDA(cudaMemGetInfo(&fr, &tot));
+      size_t fr = 0;
+      NKX_CUDA(device_free_bytes(&fr));
       const double extra = (double)(base_chunk * mult - best.chunk_pairs) * (4 << 20);  // generous per-pair bytes
       if (extra > 0.8 * (double)fr) break;
       nkx_tuning c = best;

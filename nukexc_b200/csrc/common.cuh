@@ -23,6 +23,10 @@ struct Error {
   std::string msg;
 };
 
+// Free memory of the current device, with what the dense entry points keep
+// between calls counted in (dense.cu)
+cudaError_t device_free_bytes(size_t *bytes);
+
 }  // namespace nkx
 
 // Throw-free status plumbing: inside the library every failing CUDA call is

@@ -29,12 +29,12 @@ nkx_status run_guarded(const char *where, const std::function<void()> &fn);
 // back what exceeds that.  What it keeps is not lost to the process: the driver
 // takes it back for a cudaMalloc that would fail otherwise.
 constexpr uint64_t kPoolKeep = (uint64_t)256 << 20;
-static cudaMemPool_t workspace_pool(int dev) {
+static cudaMemPool_t workspace_pool(int dev, bool create) {
   static std::mutex mu;
   static cudaMemPool_t pools[128] = {};
   NKX_REQUIRE(dev >= 0 && dev < 128, NKX_ERR_ARG, "device ordinal out of range");
   std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
+  if (!pools[dev] && create) {
     cudaMemPoolProps p{};
     p.allocType = cudaMemAllocationTypePinned;
     p.location.type = cudaMemLocationTypeDevice;
@@ -47,6 +47,18 @@ static cudaMemPool_t workspace_pool(int dev) {
   }
   return pools[dev];
 }
+cudaError_t device_free_bytes(size_t *bytes) {
+  size_t tot = 0;
+  uint64_t held = 0, used = 0;
+  int dev = 0;
+  cudaMemPool_t pool = nullptr;
+  const cudaError_t e = cudaMemGetInfo(bytes, &tot);
+  if (e == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess && (pool = workspace_pool(dev, false)) &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
+    *bytes += held - used;
+  return e;
+}
 
 template <class T>
 struct DevBuf {
@@ -56,7 +68,7 @@ struct DevBuf {
     if (!n) return;
     int dev = 0;
     NKX_CUDA(cudaGetDevice(&dev));
-    NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev), s));
+    NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev, true), s));
   }
   ~DevBuf() {
     if (p) cudaFreeAsync(p, s);

@@ -1591,8 +1591,8 @@ static void build_plan(Plan &P, const nkx_molecule *mol, const nkx_basis *prim, 
   // --- chunks of batches sized by the workspace
   size_t ws = opts->workspace_bytes;
   if (ws == 0) {
-    size_t fr = 0, tot = 0;
-    NKX_CUDA(cudaMemGetInfo(&fr, &tot));
+    size_t fr = 0;
+    NKX_CUDA(device_free_bytes(&fr));
     ws = std::min<size_t>(kDefaultWorkspace, fr / 3);
   }
   plan_chunks(P, std::max<long>(1, (long)(ws / kPairBytes)));
@@ -1738,8 +1738,8 @@ static const float *coulomb_table(Plan &P, bool mixed, cudaStream_t s) {
   if (!mixed || P.rtab_failed) return nullptr;
   if (!P.d_rtab) {
     const size_t bytes = (size_t)P.nashell * P.npad * sizeof(float);
-    size_t fr = 0, tot = 0;
-    NKX_CUDA(cudaMemGetInfo(&fr, &tot));
+    size_t fr = 0;
+    NKX_CUDA(device_free_bytes(&fr));
     if (bytes > kRtabMaxBytes || bytes > fr / 4 || cudaMalloc(&P.d_rtab, bytes) != cudaSuccess) {
       cudaGetLastError();
       P.d_rtab = nullptr;

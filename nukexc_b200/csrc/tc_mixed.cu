@@ -1765,8 +1765,8 @@ struct MixedState {
     sphT_res = nullptr;
     res_pairs = 0;
     const size_t bytes = (size_t)npairs * 4 * 4 * tile, sbytes = (size_t)npairs * 4 * 256 * sizeof(double);
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || bytes + sbytes > fr / 2) {
+    size_t fr = 0;
+    if (device_free_bytes(&fr) != cudaSuccess || bytes + sbytes > fr / 2) {
       cudaGetLastError();
       return false;
     }

@@ -1,7 +1,7 @@
 """Device memory between calls.  The dense entry points keep at most 256 MiB of
-their workspace, and an allocation that needs it gets it.  The card is filled by
-one allocation that leaves a few hundred MiB, which is what the call below then
-has."""
+their workspace, which a plan counts as free and an allocation that needs it
+gets.  The card is filled by one allocation that leaves little, which is what the
+calls below then have."""
 import contextlib
 
 import numpy as np
@@ -58,6 +58,18 @@ def _water(n, nrad, order, **kw):
     g = A.make_flat_grid(c, Z, nrad, order, weight_threshold=1e-15, radial="ta")
     plan = lambda: A.FockBuilder(c, Z, A.make_manual_basis(funcs), g, **kw)  # noqa: E731
     return plan, M.random_orbitals(len(funcs), 5 * n, seed=1), np.ones(5 * n)
+
+
+def test_plan_counts_kept_workspace_as_free():
+    plan, _, _ = _water(1, 20, 11)
+    plan().close()
+    with _card_with(3 << 30):
+        _dense_lda(128, 200 << 10)  # 192 to 256 MiB are kept
+        free = _free()
+        fb = plan()
+        pairs = fb.tuning()["chunk_pairs"]  # a third of the free memory, 2 MiB a pair
+        fb.close()
+    assert (free + 170 * MB) / (6 * MB) <= pairs <= (free + 256 * MB) / (6 * MB)  # the plan has a few MiB already
 
 
 def test_kept_workspace_goes_to_a_mixed_build():
