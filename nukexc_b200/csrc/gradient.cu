@@ -714,11 +714,14 @@ struct GradState {
     }
     return p;
   }
-  static void ensure(double *&p, size_t &cap, size_t n) {
-    if (n <= cap) return;
+  static void give_back(double *&p, size_t &cap) {
     cudaFree(p);
     p = nullptr;
     cap = 0;
+  }
+  static void ensure(double *&p, size_t &cap, size_t n) {
+    if (n <= cap) return;
+    give_back(p, cap);
     p = alloc(n);
     cap = n;
   }
@@ -748,8 +751,9 @@ static void launch_grad_pairs(Plan &P, long q0, long q1, int nspin, const double
   }
 }
 
-// T and X of the FP64 gradient go through buffers of at most this many bytes
-constexpr size_t kGradTBytes = (size_t)2 << 30, kGradXBytes = (size_t)4 << 30;
+// T and X of the FP64 gradient go through buffers of at most this many bytes, and
+// through smaller ones on a card that has no room for these
+constexpr size_t kGradTBytes = (size_t)512 << 20, kGradXBytes = (size_t)1536 << 20;
 
 // FP64 part of the gradient: per chunk the FP64 collocation, then per range
 // of its batches the orbital values T with the density, the functional,
@@ -759,24 +763,43 @@ static void fp64_gradient_chunks(Plan &P, GradState &G, int nspin, int nocc, cud
   int nn = 0;
   const int nocc_pad = fp64_orbital_pad(nocc, &nn);
   const size_t t1 = (size_t)nspin * NC * nocc_pad * kBatch, x1 = (size_t)nspin * NC * kBatch * kBlockF;
-  const long cap_b = std::max<long>(1, (long)(kGradTBytes / 8 / t1));
-  const long cap_q = std::max<long>(P.nblk, (long)(kGradXBytes / 8 / x1));
   fp64_density_begin(P, nspin, nocc, s);
   G.ensure(G.Cocc, G.C_cap, (size_t)nspin * nocc * P.nbf_pad);
   const long nC = (long)nspin * nocc * P.nbf_pad;
   scale_orbitals_kernel<<<gblk(nC, 256), 256, 0, s>>>(P.d_Ct, P.d_occ, P.nbf_pad, nC, G.Cocc);
   NKX_LAUNCH_CHECK();
   ++P.launches;
+  long cap_b = std::max<long>(1, (long)(kGradTBytes / 8 / t1));
+  long cap_q = std::max<long>(P.nblk, (long)(kGradXBytes / 8 / x1));
+  // end of the range of chunk c's batches that starts at b0
+  auto range_end = [&](const Chunk &c, long b0) {
+    long b1 = b0 + 1;
+    while (b1 < c.b1 && b1 - b0 < cap_b && P.h_pair_off[b1 + 1] - P.h_pair_off[b0] <= cap_q) ++b1;
+    return b1;
+  };
+  for (;; cap_b = std::max(1L, cap_b / 2), cap_q = std::max<long>(P.nblk, cap_q / 2)) {
+    long nb = 0, nq = 0;
+    for (const Chunk &c : P.chunks)
+      for (long b0 = c.b0, b1; b0 < c.b1; b0 = b1) {
+        b1 = range_end(c, b0);
+        nb = std::max(nb, b1 - b0);
+        nq = std::max<long>(nq, P.h_pair_off[b1] - P.h_pair_off[b0]);
+      }
+    try {
+      G.ensure(G.T, G.T_cap, (size_t)nb * t1);
+      G.ensure(G.X, G.X_cap, (size_t)nq * x1);
+      break;
+    } catch (const Error &e) {
+      if (e.code != NKX_ERR_ALLOC || (cap_b == 1 && cap_q == P.nblk)) throw;
+      G.give_back(G.T, G.T_cap);
+    }
+  }
   NKX_CUDA(cudaFuncSetAttribute(x_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem));
   for (const Chunk &c : P.chunks) {
     launch_colloc(P, c, s);
     for (long b0 = c.b0, b1; b0 < c.b1; b0 = b1) {
-      const long q0 = P.h_pair_off[b0];
-      b1 = b0 + 1;
-      while (b1 < c.b1 && b1 - b0 < cap_b && P.h_pair_off[b1 + 1] - q0 <= cap_q) ++b1;
-      const long q1 = P.h_pair_off[b1];
-      G.ensure(G.T, G.T_cap, (size_t)(b1 - b0) * t1);
-      G.ensure(G.X, G.X_cap, (size_t)(q1 - q0) * x1);
+      b1 = range_end(c, b0);
+      const long q0 = P.h_pair_off[b0], q1 = P.h_pair_off[b1];
       fp64_density_range(P, b0, b1, c.p0, nspin, nocc, G.T, s);
       const long g0 = b0 * kBatch, n = (b1 - b0) * kBatch;
       functional_kernel<<<gblk(n, 256), 256, 0, s>>>(P.xc, P.gga, nspin, P.npad, n, P.d_w + g0, P.d_rho + g0,

@@ -1,7 +1,8 @@
 """Device memory between calls.  The dense entry points keep at most 256 MiB of
 their workspace, which a plan counts as free and an allocation that needs it
-gets.  The card is filled by one allocation that leaves little, which is what the
-calls below then have."""
+gets; the FP64 gradient makes do with smaller pieces when the card is
+nearly full.  The card is filled by one allocation that leaves a few hundred
+MiB, which is what the calls below then have."""
 import contextlib
 
 import numpy as np
@@ -83,4 +84,16 @@ def test_kept_workspace_goes_to_a_mixed_build():
     with _card_with(320 * MB):
         E = fb.build([Cm], [occ], precision="mixed")[0]
     assert abs(E - E0) <= 1e-12 * abs(E0)
+    fb.close()
+
+
+def test_fp64_gradient_on_a_nearly_full_card():
+    plan, Cm, occ = _water(4, 75, 29)  # X of all pairs in one piece: 2 GB
+    ref = plan()
+    F0 = ref.xc_gradient([Cm], [occ])
+    ref.close()
+    fb = plan()
+    with _card_with(700 * MB):
+        F = fb.xc_gradient([Cm], [occ])
+    assert np.abs(F - F0).max() <= 1e-11 * np.abs(F0).max()
     fb.close()
