@@ -48,87 +48,6 @@ NKX_HD inline void sto_value_grad(const StoFunc &f, double px, double py, double
   gz = R * sz + s * dz * cR;
 }
 
-// value, gradient and Hessian (h = xx, xy, xz, yy, yz, zz):
-// with R(r) = N r^k e^(-zeta r), R' = (k/r - zeta) R, R'' = ((k/r - zeta)^2 - k/r^2) R,
-// d_j R = (R'/r) d_j and d_j d_k R = (R'/r) delta_jk + (R'' - R'/r) d_j d_k / r^2;
-// phi = R S gives d_j d_k phi = d_j d_k R S + d_j R d_k S + d_k R d_j S + R d_j d_k S.
-// The radial derivative terms are dropped at r = 0 (as in sto_value_grad).
-NKX_HD inline void sto_value_grad_hess(const StoFunc &f, double px, double py, double pz, double &v, double g[3],
-                                       double h[6]) {
-  const double d[3] = {px - f.cx, py - f.cy, pz - f.cz};
-  const double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-  const double R = f.norm * ipow(r, f.k) * exp(-f.zeta * r);
-  double s, sg[3], sh[6];
-  solid_harmonic_grad(f.l, f.m, d[0], d[1], d[2], s, sg[0], sg[1], sg[2]);
-  solid_harmonic_hess(f.l, f.m, d[0], d[1], d[2], sh[0], sh[1], sh[2], sh[3], sh[4], sh[5]);
-  double cR = 0.0, dd = 0.0;
-  if (r > 0.0) {
-    const double a = f.k / r - f.zeta;
-    cR = a * R / r;
-    dd = ((a * a - f.k / (r * r)) * R - cR) / (r * r);
-  }
-  v = R * s;
-  double dR[3];
-  for (int j = 0; j < 3; ++j) {
-    dR[j] = cR * d[j];
-    g[j] = dR[j] * s + R * sg[j];
-  }
-  const int ij[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
-  for (int e = 0; e < 6; ++e) {
-    const int j = ij[e][0], k = ij[e][1];
-    const double d2R = (j == k ? cR : 0.0) + dd * d[j] * d[k];
-    h[e] = d2R * s + dR[j] * sg[k] + dR[k] * sg[j] + R * sh[e];
-  }
-}
-
-// Radial factor cache for consecutive functions of one lane: functions of a
-// shell (same centre, zeta and n - l - 1) share r, R(r) and dR/dr / r.
-struct RadialCache {
-  double cx = 1e300, cy = 0, cz = 0, zeta = -1;
-  int k = -1;
-  double r, R, cR;
-};
-
-// value + gradient reusing the radial factor of the previous call when the
-// function shares centre, zeta and k with it (same results as sto_value_grad)
-NKX_HD inline void sto_value_grad_cached(const StoFunc &f, double px, double py, double pz, RadialCache &rc,
-                                         double &v, double &gx, double &gy, double &gz) {
-  const double dx = px - f.cx, dy = py - f.cy, dz = pz - f.cz;
-  if (!(f.cx == rc.cx && f.cy == rc.cy && f.cz == rc.cz && f.zeta == rc.zeta && f.k == rc.k)) {
-    rc.cx = f.cx;
-    rc.cy = f.cy;
-    rc.cz = f.cz;
-    rc.zeta = f.zeta;
-    rc.k = f.k;
-    rc.r = sqrt(dx * dx + dy * dy + dz * dz);
-    rc.R = ipow(rc.r, f.k) * exp(-f.zeta * rc.r);
-    rc.cR = rc.r > 0.0 ? (f.k / rc.r - f.zeta) / rc.r : 0.0;
-  }
-  const double R = f.norm * rc.R;
-  double s, sx, sy, sz;
-  solid_harmonic_grad(f.l, f.m, dx, dy, dz, s, sx, sy, sz);
-  v = R * s;
-  const double cR = rc.cR * R;
-  gx = R * sx + s * dx * cR;
-  gy = R * sy + s * dy * cR;
-  gz = R * sz + s * dz * cR;
-}
-
-NKX_HD inline double sto_value_cached(const StoFunc &f, double px, double py, double pz, RadialCache &rc) {
-  const double dx = px - f.cx, dy = py - f.cy, dz = pz - f.cz;
-  if (!(f.cx == rc.cx && f.cy == rc.cy && f.cz == rc.cz && f.zeta == rc.zeta && f.k == rc.k)) {
-    rc.cx = f.cx;
-    rc.cy = f.cy;
-    rc.cz = f.cz;
-    rc.zeta = f.zeta;
-    rc.k = f.k;
-    rc.r = sqrt(dx * dx + dy * dy + dz * dz);
-    rc.R = ipow(rc.r, f.k) * exp(-f.zeta * rc.r);
-    rc.cR = 0.0;
-  }
-  return f.norm * rc.R * solid_harmonic(f.l, f.m, dx, dy, dz);
-}
-
 // A radial shell of a function block: the functions sharing centre, zeta and
 // n - l - 1 share r^(n-l-1) e^(-zeta r) and its derivative.
 struct StoShell {
@@ -197,60 +116,6 @@ __device__ __forceinline__ double exp_neg(double x) {
   p = fma(p, t, 1.0);
   p = fma(p, t, 1.0);
   return p * __hiloint2double(((int)n + 1023) << 20, 0);
-}
-
-// Radial factor cache of sto_value_grad_hess for consecutive functions of
-// one thread at one point: functions of a shell share r, 1/r, r^k e^(-zeta r)
-// and k/r - zeta (the function's norm scales them).
-struct HessRadialCache {
-  double cx = 1e300, cy = 0, cz = 0, zeta = -1;
-  int k = -1;
-  double r = 0, ir = 0, Rn = 0, a = 0;
-};
-
-// sto_value_grad_hess with the radial factor shared over a shell's functions
-// (rc) and, with FAST, e^x by exp_neg (about 1e-14 relative; the
-// mixed-precision gradient); the same formulas, so the results differ from
-// sto_value_grad_hess by rounding only.
-template <bool FAST>
-__device__ __forceinline__ void sto_value_grad_hess_cached(const StoFunc &f, double px, double py, double pz,
-                                                           HessRadialCache &rc, double &v, double g[3],
-                                                           double h[6]) {
-  const double d[3] = {px - f.cx, py - f.cy, pz - f.cz};
-  if (!(f.cx == rc.cx && f.cy == rc.cy && f.cz == rc.cz && f.zeta == rc.zeta && f.k == rc.k)) {
-    rc.cx = f.cx;
-    rc.cy = f.cy;
-    rc.cz = f.cz;
-    rc.zeta = f.zeta;
-    rc.k = f.k;
-    rc.r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-    rc.ir = rc.r > 0.0 ? 1.0 / rc.r : 0.0;
-    rc.Rn = ipow(rc.r, f.k) * (FAST ? exp_neg(-f.zeta * rc.r) : exp(-f.zeta * rc.r));
-    rc.a = f.k * rc.ir - f.zeta;
-  }
-  const double R = f.norm * rc.Rn;
-  double s, sg[3], sh[6];
-  solid_harmonic_grad(f.l, f.m, d[0], d[1], d[2], s, sg[0], sg[1], sg[2]);
-  solid_harmonic_hess(f.l, f.m, d[0], d[1], d[2], sh[0], sh[1], sh[2], sh[3], sh[4], sh[5]);
-  double cR = 0.0, dd = 0.0;
-  if (rc.r > 0.0) {
-    cR = rc.a * R * rc.ir;
-    dd = ((rc.a * rc.a - f.k * rc.ir * rc.ir) * R - cR) * (rc.ir * rc.ir);
-  }
-  v = R * s;
-  double dR[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    dR[j] = cR * d[j];
-    g[j] = dR[j] * s + R * sg[j];
-  }
-  const int ij[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
-#pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const int j = ij[e][0], k = ij[e][1];
-    const double d2R = (j == k ? cR : 0.0) + dd * d[j] * d[k];
-    h[e] = d2R * s + dR[j] * sg[k] + dR[k] * sg[j] + R * sh[e];
-  }
 }
 
 // radial factors of every shell of the block at one point, shared by the
