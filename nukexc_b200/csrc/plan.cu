@@ -3,7 +3,7 @@
 // Once per geometry (nkx_plan_create): the grid is sorted into Morton order
 // and cut into 256-point batches (create_bounding_boxes,
 // nukexc/octree.hpp:70-141); basis functions are grouped into blocks of 128
-// in basis order and a block is significant for a batch when the cutoff
+// (by reach where that pays, then by centre in Morton order) and a block is significant for a batch when the cutoff
 // sphere of any of its functions meets the batch's bounding box
 // (build_neighbor_list, nukexc/octree.hpp:317-390); the aux Coulomb metric is
 // integrated on the grid and Cholesky-factorised in FP64.

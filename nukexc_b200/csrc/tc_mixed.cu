@@ -152,13 +152,13 @@ __device__ __forceinline__ double level_sum(uint32_t l0, uint32_t l1, uint32_t l
   return __longlong_as_double(S + 0x4338000000000000LL) - 0x1.8p52;
 }
 
-// The same sum for K <= 256 with fewer instructions: a = 2^8 L0 + L1 and
-// b = 2^8 L2 + L3 fit int32.  With |X| <= 2^30 the digits obey |d0| <= 64 and,
-// where |d0| = 64, d1 has the sign that brings X back, so per product
-// |d0 e0| <= 2^12, |d0 e1 + d1 e0| <= 2^14, |d0 e2 + d1 e1 + d2 e0| <= 32576
-// (d0 = 64, d1 = e1 = -128, e2 = 127, d2 = -128, e0 = -63) and |L3's four|
-// <= 49152, the last two not together: 256 (256 32576 + 49152) = 2^31 is not
-// reached.  (H2O)_64 PBE: V 325 -> 304 ms per build with this and the
+// The same sum for K <= 256 and no more, with fewer instructions: a = 2^8 L0 + L1
+// and b = 2^8 L2 + L3 fit int32.  With |X| <= 2^30 the digits obey |d0| <= 64 and,
+// where |d0| = 64, the rest has the sign that brings X back.  Over all such digit
+// words d and e (the sums are linear in each digit, so the ends of their ranges
+// decide) a product adds at most 2^20 to |a| and at most 8371968 to |b|, the
+// latter for d = e = (-63, -128, -128, -128): K = 256 gives 2143223808 in b, 0.2 %
+// below 2^31.  (H2O)_64 PBE: V 325 -> 304 ms per build with this and the
 // exponent-field scales below (the card is at its power limit during V, so every
 // instruction of the read-back counts even where it overlaps the MMAs).
 __device__ __forceinline__ double quad_sum(uint32_t l0, uint32_t l1, uint32_t l2, uint32_t l3) {
@@ -167,8 +167,10 @@ __device__ __forceinline__ double quad_sum(uint32_t l0, uint32_t l1, uint32_t l2
   return __longlong_as_double(S + 0x4338000000000000LL) - 0x1.8p52;
 }
 // Power-of-two scale s_a s_b 2^-36 from the high words of s_a and s_b: the
-// exponent fields add.  Clamped at 0 (a product below 2^-1022 is zero) and at
-// 0x7ff00000 (infinity).
+// exponent fields add.  A product below 2^-1022 becomes zero (the sum is clamped
+// at 0) and one of 2^1024 infinity (clamped at 0x7ff00000).  One of 2^1025 and
+// more would wrap: s_a, a row scale of phi or grad phi, is then above 2^38 beside
+// an s_b near the largest number there is.
 __device__ __forceinline__ int scale_row_word(double sa) { return __double2hiint(sa) - ((1023 + 36) << 20); }
 __device__ __forceinline__ double scale_product(int row_word, int col_word) {
   return __hiloint2double(__viaddmin_s32_relu(row_word, col_word, 0x7ff00000), 0);
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(TcShape<NW, EW>::kThreads, 1)
   __shared__ uint64_t full_bar[kStages], empty_bar[kStages], tfull_bar[NBUF], tempty_bar[NBUF], drain_bar, stall_bar;
   __shared__ uint32_t tmem_base_sh;
   __shared__ volatile int abort_flag;
-  // V and density: the column scales of each epilogue warp's current group
+  // V, density, rho: high words of the column scales of each epilogue warp's current group
   __shared__ __align__(16) int colscale[kRun ? Sh::EW * CW : 4];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1395,9 +1397,10 @@ __global__ void __launch_bounds__(256, 2) colloc_z_kernel(const StoFunc *__restr
 // separate Coulomb plane) are Z = 1/2 vJ phi.  Only planes with a gradient
 // part are staged (ZdShape::NS): the Coulomb plane, and every plane of an LDA
 // build, is one factor per point times phi and is formed again from phi's
-// digits when it is written, which lets two CTAs share an SM where two staged
-// planes allowed one ((H2O)_8 PBE + J: 2.71 -> 2.29 ms; one water LDA: 57 -> 43
-// us).  A row field of 0x7fd or more (values of 2^1022 and up, Inf, NaN)
+// digits when it is written: fewer bytes through shared memory ((H2O)_8 PBE + J:
+// 2.71 -> 2.29 ms) and, without a gradient, more CTAs an SM (one water LDA: 57 ->
+// 43 us).  A GRAD kernel of one plane takes 111 KB and shares its SM with another,
+// one of two planes takes 119 KB (Coulomb) or 183 KB and has it alone.  A row field of 0x7fd or more (values of 2^1022 and up, Inf, NaN)
 // is reported in *nonfinite.
 constexpr int kZdRanks = 4;
 template <bool GRAD, int NZ, bool JP>
@@ -1806,7 +1809,8 @@ struct MixedState {
     X_cap = doubles;
   }
   // T: the chunk's FP64 density tiles, nbatch x nspin x ncomp planes of
-  // nocc_pad x 256 (one component on the Y path); qt0: their T0 digits
+  // nocc_pad x 256 (one component on the Y path), or the fused density's column
+  // shares Rp; qt0: the T0 digits
   void ensure_T(size_t doubles) {
     if (doubles <= T_cap) return;
     cudaFree(T);
