@@ -126,7 +126,8 @@ __global__ void becke_thread_kernel(const double *__restrict__ centers, int nato
 // so four up to 96 atoms and eight beyond.  The list has room for every atom, up
 // to kBeckeCap (104 KB, two CTAs an SM).
 constexpr int kBeckeCap = 400, kBeckeNarrow = 96;  // kBeckeCap a multiple of every W
-template <int W>
+// CLAMPED: clamp > 0 (decided in the pair loop it cost 4 %)
+template <int W, bool CLAMPED>
 __global__ void __launch_bounds__(32 * W)
     becke_kernel(const double *__restrict__ centers, int natoms, const double *__restrict__ pts,
                  const int *__restrict__ owner, long npts, double *__restrict__ w, double clamp) {
@@ -141,8 +142,7 @@ __global__ void __launch_bounds__(32 * W)
   const double *p = pts + 3 * (in ? g : npts - 1);
   const double pt[3] = {p[0], p[1], p[2]};
   const int own = owner[in ? g : npts - 1];
-  const bool clamped = clamp > 0.0;  // else no atom is screened
-  const double Rc = clamped ? clamp : INFINITY;
+  const double Rc = CLAMPED ? clamp : INFINITY;  // without the clamp no atom is screened
   double r2min = INFINITY;  // stays so where a coordinate is NaN or infinite
   for (int i = warp; i < natoms; i += W) {
     const double dx = pt[0] - centers[3 * i], dy = pt[1] - centers[3 * i + 1], dz = pt[2] - centers[3 * i + 2];
@@ -154,14 +154,14 @@ __global__ void __launch_bounds__(32 * W)
   for (int v = 0; v < W; ++v) r2min = fmin(r2min, red[0][v][lane]);
   const double rmin = sqrt(r2min), lim = rmin + 2.0 * Rc;
   // an owner outside [0, natoms) is no atom's index: nothing is read for it and the weight is 0
-  const bool live = in && (unsigned)own < (unsigned)natoms && (!clamped || dist3(pt, centers + 3 * own) < rmin + Rc);
+  const bool live = in && (unsigned)own < (unsigned)natoms && (!CLAMPED || dist3(pt, centers + 3 * own) < rmin + Rc);
   // P_owner == 0 exactly; a point without a place keeps the 0 / 0 of the full loop, so that a build on it reports it
   if (warp == 0 && in && !live) w[g] *= rmin < INFINITY ? 0.0 : NAN;
   if (!__any_sync(0xffffffffu, live)) return;  // alike in every warp
   int nl = 0;
   for (int j = warp; j < natoms; j += W) {
     const double r = dist3(pt, centers + 3 * j);
-    if (!__any_sync(0xffffffffu, live && (!clamped || r < lim))) continue;
+    if (!__any_sync(0xffffffffu, live && (!CLAMPED || r < lim))) continue;
     rsm[(s0 + nl) * 32 + lane] = r;
     if (lane == 0) list[s0 + nl] = j;
     ++nl;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(32 * W)
   double norm = 0.0, pown = 0.0;
   for (int a = s0; a < s0 + nl; ++a) {
     const double ri = rsm[a * 32 + lane];
-    const bool cell = live && (!clamped || ri < rmin + Rc);  // else P_i == 0 exactly
+    const bool cell = live && (!CLAMPED || ri < rmin + Rc);  // else P_i == 0 exactly
     if (!__any_sync(0xffffffffu, cell)) continue;
     const int i = list[a];
     const double reach = cell ? ri + Rc : -1.0;  // factors of atoms at reach and beyond are 1
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(32 * W)
         if (lane < n && cb + lane != a) iR = 1.0 / fmin(dist3(centers + 3 * i, centers + 3 * list[cb + lane]), Rc);
         for (int t = 0; t < n; ++t) {
           const double rj = rsm[(cb + t) * 32 + lane];
-          if ((clamped && !__any_sync(0xffffffffu, rj < reach)) || cb + t == a) continue;
+          if ((CLAMPED && !__any_sync(0xffffffffu, rj < reach)) || cb + t == a) continue;
           P *= becke_s((ri - rj) * __shfl_sync(0xffffffffu, iR, t));
         }
       }
@@ -212,13 +212,12 @@ void launch_becke(const double *d_centers, int natoms, const double *d_pts, cons
   if (natoms <= kBeckeCap) {
     auto go = [&](auto warps) {
       constexpr int W = decltype(warps)::value;
+      auto *kernel = clamp > 0.0 ? becke_kernel<W, true> : becke_kernel<W, false>;
       constexpr size_t kAtomBytes = 32 * sizeof(double) + sizeof(int);
       const size_t smem = (size_t)((natoms + W - 1) / W * W) * kAtomBytes;
       // the limit is the same for every call, so that threads cannot lower it for one another
-      NKX_CUDA(cudaFuncSetAttribute(becke_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kBeckeCap * kAtomBytes)));
-      becke_kernel<W><<<(unsigned)((npts + 31) / 32), 32 * W, smem, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w,
-                                                                        clamp);
+      NKX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBeckeCap * kAtomBytes)));
+      kernel<<<(unsigned)((npts + 31) / 32), 32 * W, smem, s>>>(d_centers, natoms, d_pts, d_owner, npts, d_w, clamp);
     };
     natoms <= kBeckeNarrow ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 8>{});
   } else {
