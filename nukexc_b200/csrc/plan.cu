@@ -674,10 +674,10 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
                                    const double *__restrict__ px, const double *__restrict__ py,
                                    const double *__restrict__ pz, const double *__restrict__ w,
                                    const double *__restrict__ rho, int nspin, long npad, long slice,
-                                   const float *__restrict__ rtab, int naux, double *__restrict__ y,
+                                   const float *__restrict__ rtab, int naux, int sl, double *__restrict__ y,
                                    double (*red)[36]) {
   constexpr int NM = 2 * L + 1;
-  const long g0 = blockIdx.y * slice, g1 = min(npad, g0 + slice);
+  const long g0 = sl * slice, g1 = min(npad, g0 + slice);
   double acc[QM][NM];
 #pragma unroll
   for (int q = 0; q < QM; ++q)
@@ -749,34 +749,47 @@ __device__ __forceinline__ void aux_y_group(const AuxGroup &G, const AuxShell *_
   for (int e = threadIdx.x; e < G.n * NM; e += blockDim.x) {
     double s = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][e];
-    y[(size_t)blockIdx.y * naux + shells[G.first + e / NM].first + e % NM] = s;
+    y[(size_t)sl * naux + shells[G.first + e / NM].first + e % NM] = s;
   }
 }
 
-// every group of every l in one launch (block x = group): with few centres
+// every group of every l in one launch (a block per group and slice): with few centres
 // the launches of single l leave most SMs idle (one water, FP64: 149 us in
-// four launches, 107 in one; (H2O)_8, tables: 790 and 707; 97 and 324 with the
-// harmonics chosen at compile time).  The fixed-count shell loops come in quarters
-// of the l's largest group, so that a group of 6 s shells does not pay for 16.
+// four launches; (H2O)_8, tables: 790 and 707, 324 with the harmonics chosen at
+// compile time).  Block order: l, slice, group, so that the blocks on the chip read
+// the same points and run the same code.  With the tables the fixed-count shell loops
+// come in quarters of the l's largest group, so that a group of 6 s shells does not
+// pay for 16; without, a loop ends with its group, and one loop an l is all that the
+// instruction caches hold beside the incomplete gamma functions (J of an FP64
+// build, ms, with quarters and the groups fastest; with the order only; now):
+//   143 functions, one water    0.30   0.27   0.26
+//   1144, (H2O)_8               7.8    5.3    4.7
+//   4576, (H2O)_32              98     62     53
 template <bool TAB>
 __global__ void __launch_bounds__(256, TAB ? 2 : 1)
-    aux_y_groups_kernel(const AuxGroup *__restrict__ groups, const AuxShell *__restrict__ shells,
+    aux_y_groups_kernel(const AuxGroup *__restrict__ groups, int4 goff, const AuxShell *__restrict__ shells,
                         const double *__restrict__ px, const double *__restrict__ py, const double *__restrict__ pz,
                         const double *__restrict__ w, const double *__restrict__ rho, int nspin, long npad, long slice,
-                        const float *__restrict__ rtab, int naux, double *__restrict__ y) {
+                        const float *__restrict__ rtab, int naux, int nsl, double *__restrict__ y) {
   __shared__ double red[8][36];
-  const AuxGroup G = groups[blockIdx.x];
+  // block -> l (groups [o0, o1)), then slice, then group
+  const int b = blockIdx.x / nsl, o0 = b < goff.x ? 0 : b < goff.y ? goff.x : b < goff.z ? goff.y : goff.z,
+            o1 = b < goff.x ? goff.x : b < goff.y ? goff.y : b < goff.z ? goff.z : goff.w,
+            r = blockIdx.x - o0 * nsl, sl = r / (o1 - o0);
+  const AuxGroup G = groups[o0 + r % (o1 - o0)];
   auto go = [&](auto l) {
     constexpr int L = decltype(l)::value, QM = aux_group_max(L);
     const int quarter = (4 * G.n + QM - 1) / QM;
-    if (quarter <= 1)
-      aux_y_group<L, (QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+    if constexpr (!TAB)
+      aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
+    else if (quarter <= 1)
+      aux_y_group<L, (QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
     else if (quarter == 2)
-      aux_y_group<L, (2 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+      aux_y_group<L, (2 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
     else if (quarter == 3)
-      aux_y_group<L, (3 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+      aux_y_group<L, (3 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
     else
-      aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, y, red);
+      aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
   };
   switch (G.l) {
     case 0: return go(std::integral_constant<int, 0>{});
@@ -1755,6 +1768,11 @@ static const float *coulomb_table(Plan &P, bool mixed, cudaStream_t s) {
   return P.d_rtab;
 }
 
+// groups of l = 0 are [0, .x), of l = 1 [.x, .y), ...
+static int4 group_ends(const Plan &P) {
+  return make_int4(P.h_group_off[1], P.h_group_off[2], P.h_group_off[3], P.h_group_off[4]);
+}
+
 void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
     const float *rtab = coulomb_table(P, mixed, s);
     // point slices: 64 or one per 4096 points, and more (down to 1024 points
@@ -1769,9 +1787,9 @@ void coulomb_y(Plan &P, int nspin, cudaStream_t s, bool mixed) {
     if (!P.d_ypart) P.d_ypart = P.alloc<double>((size_t)nsl * P.naux);
     if (P.nagroup > 0) {
       auto *kernel = rtab ? aux_y_groups_kernel<true> : aux_y_groups_kernel<false>;
-      kernel<<<dim3((unsigned)P.nagroup, (unsigned)nsl), 256, 0, s>>>(P.d_agroup, P.d_ashell, P.d_px, P.d_py, P.d_pz,
-                                                                      P.d_w, P.d_rho, nspin, P.npad, slice, rtab,
-                                                                      P.naux, P.d_ypart);
+      kernel<<<(unsigned)(P.nagroup * nsl), 256, 0, s>>>(P.d_agroup, group_ends(P), P.d_ashell, P.d_px, P.d_py, P.d_pz,
+                                                        P.d_w, P.d_rho, nspin, P.npad, slice, rtab, P.naux, (int)nsl,
+                                                        P.d_ypart);
       NKX_LAUNCH_CHECK();
       ++P.launches;
     }
@@ -1810,7 +1828,7 @@ void coulomb_solve(Plan &P, cudaStream_t s, bool mixed) {
       NKX_LAUNCH_CHECK();
       P.launches += 2;
     }
-    const int4 goff = make_int4(P.h_group_off[1], P.h_group_off[2], P.h_group_off[3], P.h_group_off[4]);
+    const int4 goff = group_ends(P);
     if (rtab)
       aux_v_group_tab_kernel<<<nblk(P.npad, 256), 128, 0, s>>>(P.d_agroup, goff, P.d_ashell, P.d_loose, P.nloose,
                                                                P.d_c, P.d_px, P.d_py, P.d_pz, P.d_w, P.npad, rtab,
