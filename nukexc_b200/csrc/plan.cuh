@@ -127,12 +127,12 @@ struct Plan {
   // build status words, zeroed by every build: [0] code of the first
   // tensor-core wait that gave up, [1] non-finite input or operand seen
   int *d_status = nullptr;
-  // E_xc and the status words lie together on the device and come back in
-  // one copy to pinned memory
+  // E_xc and the status words lie together on the device and come back in one
+  // copy to page-locked memory (result_slot), or to own_result if there is none
   struct Result {
     double E;
     int status[2];
-  } *h_result = nullptr;
+  } own_result{}, *h_result = &own_result;
   // limit of the device waits that may be abandoned (nkx_plan_set_wait_limit)
   unsigned long long wait_ns = 2000000000ull;
   int stall_test = 0;  // tests of the error path: tensor-core kernels wait on a barrier nothing completes
