@@ -147,8 +147,8 @@ NKX_API nkx_status nkx_becke_partition(const double *d_centers, int natoms, cons
 /* ----------------------------------------------------- dense reference API */
 
 /* The entry points of this section take their workspace from a stream-ordered
- * memory pool of the library's own, one per device.  It keeps at most 256 MiB
- * between calls, which the driver gives to any cudaMalloc of the process that
+ * memory pool of the library's own, one per device (a call that needs more than
+ * 256 MiB takes it by cudaMalloc).  The pool keeps at most 256 MiB between calls, which the driver gives to any cudaMalloc of the process that
  * would fail without them (a pool of the host program's own made by other
  * means may not get them; nkx_xc_dense_noalloc keeps nothing but its array).
  * A pool does not outlive its context, so none of these may be used across a

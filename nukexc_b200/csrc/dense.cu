@@ -27,7 +27,9 @@ nkx_status run_guarded(const char *where, const std::function<void()> &fn);
 // of kernels.  The pool keeps at most kPoolKeep bytes between calls: workspaces
 // are freed before a call's last synchronisation, which is when the pool gives
 // back what exceeds that.  What it keeps is not lost to the process: the driver
-// takes it back for a cudaMalloc that would fail otherwise.
+// takes it back for a cudaMalloc that would fail otherwise.  A call that needs more
+// in all takes it by cudaMalloc: a pool that has to grow for every call is slower
+// (core Hamiltonian of three waters, 1.1 GB: 11.6 ms by the pool, 7.8 by cudaMalloc).
 constexpr uint64_t kPoolKeep = (uint64_t)256 << 20;
 static cudaMemPool_t workspace_pool(int dev, bool create) {
   static std::mutex mu;
@@ -60,18 +62,29 @@ cudaError_t device_free_bytes(size_t *bytes) {
   return e;
 }
 
+// where a call's workspaces come from, by the bytes of all of them
+struct Source {
+  cudaStream_t s;
+  bool pooled;
+  Source(cudaStream_t stream, size_t bytes = 0) : s(stream), pooled(bytes <= kPoolKeep) {}
+};
+
 template <class T>
 struct DevBuf {
   T *p = nullptr;
-  cudaStream_t s;
-  DevBuf(size_t n, cudaStream_t stream) : s(stream) {
+  Source from;
+  DevBuf(size_t n, Source source) : from(source) {
     if (!n) return;
     int dev = 0;
     NKX_CUDA(cudaGetDevice(&dev));
-    NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev, true), s));
+    if (from.pooled)
+      NKX_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), workspace_pool(dev, true), from.s));
+    else
+      NKX_CUDA(cudaMalloc(&p, n * sizeof(T)));
   }
   ~DevBuf() {
-    if (p) cudaFreeAsync(p, s);
+    if (p && from.pooled) cudaFreeAsync(p, from.s);
+    if (p && !from.pooled) cudaFree(p);
   }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
@@ -683,8 +696,9 @@ extern "C" nkx_status nkx_xc_dense(int nbf, long npts, const double *d_phi, cons
     NKX_REQUIRE(!gga || (d_gx && d_gy && d_gz), NKX_ERR_ARG, "GGA needs collocation gradients");
     cudaStream_t s = (cudaStream_t)stream;
     run_and_wait(s, [&] {
-      DevBuf<double> rho((size_t)nspin * npts, s), grad((size_t)nspin * 3 * npts, s), Z((size_t)nspin * nbf * npts, s),
-          Ed(1, s);
+      const Source ws(s, sizeof(double) * nspin * npts * (nbf + (size_t)4));
+      DevBuf<double> rho((size_t)nspin * npts, ws), grad((size_t)nspin * 3 * npts, ws),
+          Z((size_t)nspin * nbf * npts, ws), Ed(1, ws);
       for (int sp_i = 0; sp_i < nspin; ++sp_i)
         launch_density_dense(nbf, npts, d_phi, gga ? d_gx : nullptr, d_gy, d_gz, nocc, d_C + (size_t)sp_i * nbf * nocc,
                              d_occ + (size_t)sp_i * nocc, rho.p + (size_t)sp_i * npts,
@@ -783,7 +797,8 @@ extern "C" nkx_status nkx_coulomb_dense(int nbf, int naux, long npts, const doub
     const long na = (naux + 31) / 32, nsl = std::max<long>(1, std::min<long>((8 * 148 + na - 1) / na, npts / 128));
     const long slice = (npts + nsl - 1) / nsl;
     run_and_wait(s, [&] {
-      DevBuf<double> rho(npts, s), y(naux, s), t(K, s), c(naux, s), v(npts, s), part((size_t)nsl * naux, s);
+      const Source ws(s, sizeof(double) * (2 * (size_t)npts + (size_t)nsl * naux));
+      DevBuf<double> rho(npts, ws), y(naux, ws), t(K, ws), c(naux, ws), v(npts, ws), part((size_t)nsl * naux, ws);
       launch_density_dense(nbf, npts, d_phi, nullptr, nullptr, nullptr, nocc, d_C, d_occ, rho.p, nullptr, nullptr, s);
       vw_rho_kernel<<<dim3((unsigned)na, (unsigned)nsl), 256, 0, s>>>(naux, npts, slice, d_Vw, rho.p, part.p);
       rows_dot_kernel<<<nblk(naux * 32L, 256), 256, 0, s>>>(naux, (int)nsl, part.p, nullptr, y.p);
@@ -816,8 +831,9 @@ extern "C" nkx_status nkx_exchange_dense(int nbf, int naux, long npts, const dou
     cublasHandle_t h = nullptr;
     bool ok = true;
     run_and_wait(s, [&] {
-      DevBuf<double> T((size_t)npts * nocc, s), B((size_t)nbf * npts, s), P3((size_t)naux * nbf, s),
-          Y((size_t)nbf * K, s);
+      const Source ws(s, sizeof(double) * ((size_t)npts * (nocc + nbf) + (size_t)nbf * (naux + K)));
+      DevBuf<double> T((size_t)npts * nocc, ws), B((size_t)nbf * npts, ws), P3((size_t)naux * nbf, ws),
+          Y((size_t)nbf * K, ws);
       NKX_REQUIRE(cublasCreate(&h) == CUBLAS_STATUS_SUCCESS, NKX_ERR_CUDA, "cublasCreate failed");
       cublasSetStream(h, s);
       const double one = 1.0, zero = 0.0;
@@ -885,8 +901,9 @@ extern "C" nkx_status nkx_core_hamiltonian_dense(const nkx_basis *basis, const n
       NKX_CUDA(cudaMemcpyAsync(dz.p, zc.data(), sizeof(double) * mol->natoms, cudaMemcpyHostToDevice, s));
       // points in chunks holding 6 nbf x chunk matrices in about 1 GiB
       const long chunk = std::max<long>(256, std::min<long>(npts, ((long)1 << 27) / (6L * nbf)));
-      DevBuf<double> phi((size_t)nbf * chunk, s), gx((size_t)nbf * chunk, s), gy((size_t)nbf * chunk, s),
-          gz((size_t)nbf * chunk, s), sc((size_t)nbf * chunk, s), wv(chunk, s);
+      const Source ws(s, sizeof(double) * (5 * (size_t)nbf * chunk + chunk));
+      DevBuf<double> phi((size_t)nbf * chunk, ws), gx((size_t)nbf * chunk, ws), gy((size_t)nbf * chunk, ws),
+          gz((size_t)nbf * chunk, ws), sc((size_t)nbf * chunk, ws), wv(chunk, ws);
       NKX_CUDA(cudaMemsetAsync(d_S, 0, sizeof(double) * nbf * nbf, s));
       NKX_CUDA(cudaMemsetAsync(d_T, 0, sizeof(double) * nbf * nbf, s));
       NKX_CUDA(cudaMemsetAsync(d_V, 0, sizeof(double) * nbf * nbf, s));
@@ -926,7 +943,8 @@ extern "C" nkx_status nkx_half_inverse(int N, const double *d_S, double thr, dou
     cudaStream_t s = (cudaStream_t)stream;
     std::vector<double> hl(N), hU((size_t)N * N), hD(N);
     run_and_wait(s, [&] {
-      DevBuf<double> A((size_t)N * N, s), D(N, s), lam(N, s);
+      const Source ws(s, sizeof(double) * 4 * (size_t)N * N);  // the solver's own is about 2 N^2
+      DevBuf<double> A((size_t)N * N, ws), D(N, ws), lam(N, ws);
       DevBuf<int> info(1, s);
       dim3 tb(16, 16), gb(nblk(N, 16), nblk(N, 16));
       precondition_kernel<<<gb, tb, 0, s>>>(N, d_S, A.p, D.p);
@@ -936,7 +954,7 @@ extern "C" nkx_status nkx_half_inverse(int N, const double *d_S, double thr, dou
       cusolverDnSetStream(h, s);
       int lwork = 0;
       cusolverDnDsyevd_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N, lam.p, &lwork);
-      DevBuf<double> work(lwork > 0 ? lwork : 1, s);
+      DevBuf<double> work(lwork > 0 ? lwork : 1, ws);
       const cusolverStatus_t st = cusolverDnDsyevd(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A.p, N,
                                                    lam.p, work.p, lwork, info.p);
       cusolverDnDestroy(h);
