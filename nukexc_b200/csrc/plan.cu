@@ -349,7 +349,9 @@ __global__ void functional_kernel(XcSpec s, bool gga, int nspin, long npad, long
 
 // Z^T[pair][spin][g][f] = coef0 phi + coef1 dphi/dx + coef2 dphi/dy + coef3 dphi/dz.
 // Spin index nspin (when jonly) builds Z_J = 1/2 vJ phi for a separate J.
-template <bool GRAD>
+// SPLIT: a pair's points are dealt to gridDim.y CTAs (else a constant count, with
+// which LDA planes of many pairs take a tenth less)
+template <bool GRAD, bool SPLIT>
 __global__ void zbuild_fp64_kernel(const double *__restrict__ phiT, const double *__restrict__ coef,
                                    const double *__restrict__ vj, const int *__restrict__ pair_batch, long p0,
                                    int nz, int nspin, long npad, double *__restrict__ zT) {
@@ -358,7 +360,7 @@ __global__ void zbuild_fp64_kernel(const double *__restrict__ phiT, const double
   const int b = pair_batch[p0 + q];
   const size_t tile = (size_t)kBatch * kBlockF;
   const double *P = phiT + q * NC * tile;
-  const int ne = kBatch * kBlockF / gridDim.y, e0 = blockIdx.y * ne;  // this CTA's elements
+  const int ne = kBatch * kBlockF / (SPLIT ? gridDim.y : 1), e0 = SPLIT ? blockIdx.y * ne : 0;  // this CTA's elements
   for (int e = e0 + threadIdx.x; e < e0 + ne; e += blockDim.x) {
     const int g = e / kBlockF;
     const long gg = (long)b * kBatch + g;
@@ -2007,12 +2009,9 @@ void fock_build_fp64(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool s
     }
     T.begin(ST_ZBUILD, s);
     const dim3 zgrid((unsigned)np, point_split(np, P.nsm));
-    if (P.gga)
-      zbuild_fp64_kernel<true><<<zgrid, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs,
-                                                            nspin, P.npad, P.ws_z);
-    else
-      zbuild_fp64_kernel<false><<<zgrid, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs,
-                                                             nspin, P.npad, P.ws_z);
+    auto *zbuild = zgrid.y > 1 ? (P.gga ? zbuild_fp64_kernel<true, true> : zbuild_fp64_kernel<false, true>)
+                               : (P.gga ? zbuild_fp64_kernel<true, false> : zbuild_fp64_kernel<false, false>);
+    zbuild<<<zgrid, 256, 0, s>>>(P.ws_phi, P.d_coef, P.d_vj, P.d_pair_batch, c.p0, nzs, nspin, P.npad, P.ws_z);
     NKX_LAUNCH_CHECK();
     ++P.launches;
     T.end(s);
