@@ -30,8 +30,8 @@ __device__ __forceinline__ double dist3(const double *a, const double *b) {
 
 constexpr int kBeckeList = 128;
 
-// One thread per point, for molecules of more than kBeckeCap atoms.  With the
-// Laqua clamp R_ij = min(|A_i-A_j|, Rc)
+// One thread per point, for molecules of fewer than kBeckeFew or more than
+// kBeckeCap atoms.  With the Laqua clamp R_ij = min(|A_i-A_j|, Rc)
 // (partitioning.hpp:134-148) the cell functions are exactly 0 or 1 far from
 // the point: every atom with r_i >= r_min + Rc has P_i = 0 (its factor
 // against the nearest atom is s(1) = 0), and in P_i of the others every atom
@@ -123,9 +123,11 @@ __global__ void becke_thread_kernel(const double *__restrict__ centers, int nato
 //     96   0.93 M     9.4     4.5     2.57    2.82    3.90
 //    192   1.86 M    33.3             14.0    10.1    11.9
 //    384   3.72 M                     60.7    38.4    34.1
-// so four up to 96 atoms and eight beyond.  The list has room for every atom, up
+// so four up to 96 atoms and eight beyond.  With a handful of atoms a point has
+// too little to share (0.2 M points, us, W = 0 and 4: one atom 31 and 39, three 40
+// and 46, four 46 and 51, six 69 and 69, eight 98 and 81).  The list has room for every atom, up
 // to kBeckeCap (104 KB, two CTAs an SM).
-constexpr int kBeckeCap = 400, kBeckeNarrow = 96;  // kBeckeCap a multiple of every W
+constexpr int kBeckeFew = 6, kBeckeCap = 400, kBeckeNarrow = 96;  // kBeckeCap a multiple of every W
 // CLAMPED: clamp > 0 (decided in the pair loop it cost 4 %)
 template <int W, bool CLAMPED>
 __global__ void __launch_bounds__(32 * W)
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(32 * W)
 void launch_becke(const double *d_centers, int natoms, const double *d_pts, const int *d_owner, long npts,
                   double *d_w, double clamp, cudaStream_t s) {
   if (npts <= 0) return;
-  if (natoms <= kBeckeCap) {
+  if (natoms >= kBeckeFew && natoms <= kBeckeCap) {
     auto go = [&](auto warps) {
       constexpr int W = decltype(warps)::value;
       auto *kernel = clamp > 0.0 ? becke_kernel<W, true> : becke_kernel<W, false>;

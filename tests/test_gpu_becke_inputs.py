@@ -1,8 +1,9 @@
 """Becke weights of inputs that no grid should hold.  An owner outside
 [0, natoms) owns nothing: weight 0.  A point with a NaN or infinite coordinate
 has no weight: NaN, so that a build on it reports the point.  The other points
-of the same warp keep their weights.  Sizes of each path: four warps, eight, and
-a thread per point; with the clamp and without."""
+of the same warp keep their weights.  Sizes of each path: a thread
+per point for few atoms, four warps, eight, and a thread per point for many; with
+the clamp and without.  The first sizes of four warps also against the oracle."""
 import numpy as np
 import pytest
 
@@ -13,8 +14,9 @@ if not torch.cuda.is_available():
     pytest.skip("needs a CUDA GPU", allow_module_level=True)
 
 from nukexc_b200 import api as A  # noqa: E402
+from oracle import oracle as O  # noqa: E402
 
-SIZES = [3, 97, 401]
+SIZES = [3, 6, 97, 401]
 
 
 def _case(natoms):
@@ -48,3 +50,10 @@ def test_point_without_a_place_has_no_finite_weight(natoms, clamp):
     got = _weights(c, pts, own, w, clamp)
     bad = np.isin(np.arange(70), [2, 40, 65])
     assert np.isnan(got[bad]).all() and (got[~bad] == ref[~bad]).all()
+
+
+@pytest.mark.parametrize("clamp", [5.0, 0.0])
+@pytest.mark.parametrize("natoms", [5, 6, 7])
+def test_first_sizes_of_four_warps(natoms, clamp):
+    c, own, pts, w = _case(natoms)
+    assert np.abs(_weights(c, pts, own, w, clamp) - O.becke(c, pts, own, w, clamp_R=clamp)).max() <= 1e-13
