@@ -528,12 +528,6 @@ __device__ __forceinline__ void dense_load(const F *__restrict__ fn, const Dense
   __syncthreads();
 }
 
-// keeps the compiler from hoisting the products of all harmonics out of a
-// loop over a run's functions (it spilled a few hundred of them)
-__device__ __forceinline__ void opaque(double &x, double &y, double &z) {
-  asm volatile("" : "+d"(x), "+d"(y), "+d"(z));
-}
-
 // one chunk's tile [f][point] to its place in the output
 __device__ __forceinline__ void dense_store(const double *tile, int nf, int f0, int nfun, long g0, int np,
                                             double *__restrict__ out) {

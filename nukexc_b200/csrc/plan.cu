@@ -782,17 +782,19 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1)
   const AuxGroup G = groups[o0 + r % (o1 - o0)];
   auto go = [&](auto l) {
     constexpr int L = decltype(l)::value, QM = aux_group_max(L);
-    const int quarter = (4 * G.n + QM - 1) / QM;
-    if constexpr (!TAB)
+    if constexpr (TAB) {
+      const int quarter = (4 * G.n + QM - 1) / QM;
+      if (quarter <= 1)
+        aux_y_group<L, (QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
+      else if (quarter == 2)
+        aux_y_group<L, (2 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
+      else if (quarter == 3)
+        aux_y_group<L, (3 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
+      else
+        aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
+    } else {
       aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
-    else if (quarter <= 1)
-      aux_y_group<L, (QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
-    else if (quarter == 2)
-      aux_y_group<L, (2 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
-    else if (quarter == 3)
-      aux_y_group<L, (3 * QM + 3) / 4, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
-    else
-      aux_y_group<L, QM, TAB>(G, shells, px, py, pz, w, rho, nspin, npad, slice, rtab, naux, sl, y, red);
+    }
   };
   switch (G.l) {
     case 0: return go(std::integral_constant<int, 0>{});
@@ -802,33 +804,22 @@ __global__ void __launch_bounds__(256, TAB ? 2 : 1)
   }
 }
 
-template <int L, bool TAB>
+template <int L>
 __device__ __forceinline__ double aux_group_v(const AuxGroup &G, const AuxShell *__restrict__ shells,
-                                              const double *__restrict__ c, double x, double y, double z,
-                                              const float *__restrict__ rtab, long npad, long g) {
+                                              const double *__restrict__ c, double x, double y, double z) {
   constexpr int NM = 2 * L + 1;
   const double dx = x - G.cx, dy = y - G.cy, dz = z - G.cz;
   double S[NM];
   solid_harmonics_all<L>(dx, dy, dz, S);
   double s = 0.0;
-  if constexpr (TAB) {
-    for (int q = 0; q < G.n; ++q) {
-      const int f0 = shells[G.first + q].first;
-      double a = 0.0;
+  const double rr = sqrt(dx * dx + dy * dy + dz * dz);
+  const double r2l1inv = rr < 1e-12 ? 0.0 : ipow_c<2 * L + 1>(1.0 / rr);
+  for (int q = 0; q < G.n; ++q) {
+    const AuxShell &sh = shells[G.first + q];
+    double a = 0.0;
 #pragma unroll
-      for (int m = 0; m < NM; ++m) a = fma(c[f0 + m], S[m], a);
-      s = fma(a, (double)rtab[(size_t)(G.first + q) * npad + g], s);
-    }
-  } else {
-    const double rr = sqrt(dx * dx + dy * dy + dz * dz);
-    const double r2l1inv = rr < 1e-12 ? 0.0 : ipow_c<2 * L + 1>(1.0 / rr);
-    for (int q = 0; q < G.n; ++q) {
-      const AuxShell &sh = shells[G.first + q];
-      double a = 0.0;
-#pragma unroll
-      for (int m = 0; m < NM; ++m) a += c[sh.first + m] * (sh.f.C * S[m]);
-      if (a != 0.0) s += a * aux_radial_r(sh.f, rr, r2l1inv);
-    }
+    for (int m = 0; m < NM; ++m) a += c[sh.first + m] * (sh.f.C * S[m]);
+    if (a != 0.0) s += a * aux_radial_r(sh.f, rr, r2l1inv);
   }
   return s;
 }
@@ -845,18 +836,8 @@ __global__ void __launch_bounds__(256) aux_y_reduce_kernel(const double *__restr
   if (lane == 0) y[a] = s;
 }
 
-// sum_m c_m S_lm of a loose shell (any l): a call, so that the switch over all
-// harmonics takes no registers from the groups' loops
-__device__ __noinline__ double aux_loose_sum(const AuxShell &sh, const double *__restrict__ c, double dx, double dy,
-                                             double dz) {
-  double a = 0.0;
-#pragma unroll 1
-  for (int m = 0; m < sh.nm; ++m) a += c[sh.first + m] * solid_harmonic(sh.f.l, sh.f.m + m, dx, dy, dz);
-  return a;
-}
-
-// v_g = w_g sum_a c_a V_a(g) over the groups, then the loose shells
-// (coulomb.hpp:90-95)
+// v_g = w_g sum_a c_a V_a(g) over the groups; aux_v_loose_kernel adds the loose
+// shells (coulomb.hpp:90-95)
 // v of two points (ga, gb) from one group with the C R table: the group's
 // data and the fit coefficients are loaded once for both
 template <int L>
@@ -887,12 +868,10 @@ __device__ __forceinline__ void aux_group_v2_tab(const AuxGroup &G, const AuxShe
 }
 
 // the table form of aux_v_group_kernel: two points per thread.  ((H2O)_8, 1144
-// functions: 672 us with the harmonics' switch in the loops, 500 now; the bounds
-// on the registers, here and below, are for aux_loose_sum, which alone would take
-// 160: without them 742 us, and 78 instead of 52 for one water in FP64)
+// functions: 672 us with the harmonics' switch in the loops, 500 now)
 __global__ void __launch_bounds__(256, 3)
     aux_v_group_tab_kernel(const AuxGroup *__restrict__ groups, int4 goff,
-                           const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
+                           const AuxShell *__restrict__ shells,
                            const double *__restrict__ c, const double *__restrict__ px,
                            const double *__restrict__ py, const double *__restrict__ pz,
                            const double *__restrict__ w, long npad, const float *__restrict__ rtab,
@@ -910,26 +889,16 @@ __global__ void __launch_bounds__(256, 3)
   for (int k = goff.y; k < goff.z; ++k) aux_group_v2_tab<2>(groups[k], shells, c, x, y, z, rtab, npad, ga, gb, s);
 #pragma unroll 1
   for (int k = goff.z; k < goff.w; ++k) aux_group_v2_tab<3>(groups[k], shells, c, x, y, z, rtab, npad, ga, gb, s);
-  for (int k = 0; k < nloose; ++k) {
-    const AuxShell &sh = shells[loose[k]];
-    const AuxFunc &f = sh.f;
-    const float *row = rtab + (size_t)loose[k] * npad;
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-      s[e] += aux_loose_sum(sh, c, x[e] - f.cx, y[e] - f.cy, z[e] - f.cz) * (double)row[e ? gb : ga];
-  }
   v[ga] = s[0] * w[ga];
   if (ga + (long)blockDim.x < npad) v[gb] = s[1] * w[gb];
 }
 
-template <bool TAB>
 __global__ void __launch_bounds__(128, 6)
     aux_v_group_kernel(const AuxGroup *__restrict__ groups, int4 goff,
-                       const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
+                       const AuxShell *__restrict__ shells,
                        const double *__restrict__ c, const double *__restrict__ px,
                        const double *__restrict__ py, const double *__restrict__ pz,
-                       const double *__restrict__ w, long npad, const float *__restrict__ rtab,
-                       double *__restrict__ v) {
+                       const double *__restrict__ w, long npad, double *__restrict__ v) {
   const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (g >= npad) return;
   if (w[g] == 0.0) {
@@ -940,22 +909,46 @@ __global__ void __launch_bounds__(128, 6)
   double s = 0.0;
   // groups sorted by l: [0, goff.x) l = 0, [goff.x, goff.y) l = 1, ...
 #pragma unroll 1
-  for (int k = 0; k < goff.x; ++k) s += aux_group_v<0, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+  for (int k = 0; k < goff.x; ++k) s += aux_group_v<0>(groups[k], shells, c, x, y, z);
 #pragma unroll 1
-  for (int k = goff.x; k < goff.y; ++k) s += aux_group_v<1, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+  for (int k = goff.x; k < goff.y; ++k) s += aux_group_v<1>(groups[k], shells, c, x, y, z);
 #pragma unroll 1
-  for (int k = goff.y; k < goff.z; ++k) s += aux_group_v<2, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+  for (int k = goff.y; k < goff.z; ++k) s += aux_group_v<2>(groups[k], shells, c, x, y, z);
 #pragma unroll 1
-  for (int k = goff.z; k < goff.w; ++k) s += aux_group_v<3, TAB>(groups[k], shells, c, x, y, z, rtab, npad, g);
+  for (int k = goff.z; k < goff.w; ++k) s += aux_group_v<3>(groups[k], shells, c, x, y, z);
+  v[g] = s * w[g];
+}
+
+// The loose shells (l > 3, parts of a shell) are added to v by a kernel of their own,
+// so that the switch over all harmonics takes no registers from the groups' loops;
+// opaque coordinates keep it from forming the products of all harmonics for each
+// shell ((H2O)_4, 1296 functions in random order: 21.5 ms in FP64 and 17.6 with the
+// table where it does, 4.9 and 2.7 now).  rtab: C R from the mixed build's table.
+template <bool TAB>
+__global__ void aux_v_loose_kernel(const AuxShell *__restrict__ shells, const int *__restrict__ loose, int nloose,
+                                   const double *__restrict__ c, const double *__restrict__ px,
+                                   const double *__restrict__ py, const double *__restrict__ pz,
+                                   const double *__restrict__ w, long npad, const float *__restrict__ rtab,
+                                   double *__restrict__ v) {
+  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (g >= npad || w[g] == 0.0) return;
+  const double x = px[g], y = py[g], z = pz[g];
+  double s = 0.0;
   for (int k = 0; k < nloose; ++k) {
     const AuxShell &sh = shells[loose[k]];
     const AuxFunc &f = sh.f;
     const double dx = x - f.cx, dy = y - f.cy, dz = z - f.cz;
-    const double a = aux_loose_sum(sh, c, dx, dy, dz);
+    double a = 0.0;
+#pragma unroll 1
+    for (int m = 0; m < sh.nm; ++m) {
+      double hx = dx, hy = dy, hz = dz;
+      opaque(hx, hy, hz);
+      a += c[sh.first + m] * solid_harmonic(f.l, f.m + m, hx, hy, hz);
+    }
     if (a != 0.0)
       s += a * (TAB ? (double)rtab[(size_t)loose[k] * npad + g] : f.C * aux_radial(f, sqrt(dx * dx + dy * dy + dz * dz)));
   }
-  v[g] = s * w[g];
+  v[g] += s * w[g];
 }
 
 // Aux collocation phi_A(g) and weighted potential Vw_B(g) of a slice of
@@ -1857,15 +1850,20 @@ void coulomb_solve(Plan &P, cudaStream_t s, bool mixed) {
     }
     const int4 goff = group_ends(P);
     if (rtab)
-      aux_v_group_tab_kernel<<<nblk(P.npad, 256), 128, 0, s>>>(P.d_agroup, goff, P.d_ashell, P.d_loose, P.nloose,
-                                                               P.d_c, P.d_px, P.d_py, P.d_pz, P.d_w, P.npad, rtab,
-                                                               P.d_vj);
+      aux_v_group_tab_kernel<<<nblk(P.npad, 256), 128, 0, s>>>(P.d_agroup, goff, P.d_ashell, P.d_c, P.d_px, P.d_py,
+                                                               P.d_pz, P.d_w, P.npad, rtab, P.d_vj);
     else
-      aux_v_group_kernel<false><<<nblk(P.npad, 128), 128, 0, s>>>(P.d_agroup, goff, P.d_ashell, P.d_loose, P.nloose,
-                                                                  P.d_c, P.d_px, P.d_py, P.d_pz, P.d_w, P.npad, rtab,
-                                                                  P.d_vj);
+      aux_v_group_kernel<<<nblk(P.npad, 128), 128, 0, s>>>(P.d_agroup, goff, P.d_ashell, P.d_c, P.d_px, P.d_py, P.d_pz,
+                                                           P.d_w, P.npad, P.d_vj);
     NKX_LAUNCH_CHECK();
     ++P.launches;
+    if (P.nloose > 0) {
+      auto *kernel = rtab ? aux_v_loose_kernel<true> : aux_v_loose_kernel<false>;
+      kernel<<<nblk(P.npad, 128), 128, 0, s>>>(P.d_ashell, P.d_loose, P.nloose, P.d_c, P.d_px, P.d_py, P.d_pz, P.d_w,
+                                               P.npad, rtab, P.d_vj);
+      NKX_LAUNCH_CHECK();
+      ++P.launches;
+    }
 }
 
 template <bool GRAD, int NN>

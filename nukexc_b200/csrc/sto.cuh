@@ -56,6 +56,13 @@ struct StoShell {
 };
 
 #ifdef __CUDACC__
+// keeps the compiler from hoisting the products of all harmonics out of a
+// loop over functions (it spilled a few hundred of them, or formed them all for
+// a single one)
+__device__ __forceinline__ void opaque(double &x, double &y, double &z) {
+  asm volatile("" : "+d"(x), "+d"(y), "+d"(z));
+}
+
 // One 128-function block in shared memory, laid out for kernels in which lane
 // l of a warp evaluates functions 4l .. 4l+3: field[c][l] holds function
 // 4l + c, so the 32 reads of one field by a warp are consecutive; sh[c][l]
