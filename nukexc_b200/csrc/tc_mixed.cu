@@ -2150,9 +2150,15 @@ void fock_build_mixed(Plan &P, int nspin, int nocc, bool needJ, bool fuse, bool 
   // Without the Y path, and at N = 64, the density contraction sums over the
   // orbitals in its own epilogue: no T is written and read back ((H2O)_8 PBE,
   // 40 orbitals: 999 us for both kernels, 809 now).  The Y path needs T_0
-  // itself, and N = 128 has no registers or shared memory left for it.
-  const bool fused_rho = !grad_mode && density_width(P, nocc) == 64;
+  // itself, and N = 128 has no registers or shared memory left for it.  A unit
+  // takes the four components of a GGA one after the other, so with few units and
+  // few orbitals T and its contraction are shorter (three blocks, us, T and fused:
+  // 5 orbitals, 4 batches 20 and 42, 74 batches 48 and 46; 40 orbitals, 4 batches 34
+  // and 42, 32 batches 43 and 43; 100 orbitals, 4 batches 56 and 42).
   const int rho_parts = 2 * ((nocc + 63) / 64);
+  const long rho_units = (long)M.nbatch_chunk * nspin * rho_parts;
+  const bool fused_rho = !grad_mode && density_width(P, nocc) == 64 &&
+                         (nc == 1 || nocc > 64 || rho_units >= (nocc > 16 ? M.nsm / 2 : M.nsm));
   if (phase != 2) {
     M.ensure_T(fused_rho ? (size_t)M.nbatch_chunk * kBatch * nspin * nc * rho_parts
                          : (size_t)M.nbatch_chunk * nspin * (grad_mode ? 1 : nc) * M.nocc_pad * 256);

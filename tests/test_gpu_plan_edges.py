@@ -1,7 +1,7 @@
 """Edges of the plan's choices: the FP64 V tile at 64 and 65 functions (the last
 basis that fills two slots of its block and the first that does not), in the
 build and in the core Hamiltonian; blocks sorted by reach, at two screening
-tolerances.  Oracle gates as for screened builds: FP64 1e-10 relative on E and
+tolerances; the mixed density on either side of its rule for few batches.  Oracle gates as for screened builds: FP64 1e-10 relative on E and
 1e-11 absolute on V unscreened; the tolerance of the dropped terms otherwise."""
 import numpy as np
 import pytest
@@ -68,4 +68,20 @@ def test_blocks_sorted_by_reach(tol, monkeypatch):
     for precision, e, v in (("fp64", 1e-10, 1e-10), ("mixed", 1e-6, 1e-7)):
         E, V, _ = fb.build([Cm], [occ], precision=precision)
         assert abs(E - Eo) <= max(e, tol) and np.abs(V[0] - Vo[0]).max() <= max(v, tol)
+    fb.close()
+
+
+@pytest.mark.parametrize("nbatch,nocc,nspin", [(1, 5, 1), (30, 16, 2), (40, 16, 2), (30, 40, 1), (40, 17, 1), (3, 65, 1)])
+def test_mixed_density_of_few_batches(nbatch, nocc, nspin):
+    c, Z = M.water_cluster(3, seed=5)
+    funcs = M.sto_basis(c, Z)
+    g = A.make_flat_grid(c, Z, 30, 17, weight_threshold=1e-15, radial="ta")
+    pick = np.argsort(np.linalg.norm(g.quad_points - c.mean(0), axis=1))[:256 * nbatch - 7]
+    pts, w = g.quad_points[pick], g.weights[pick]
+    Cs = [M.random_orbitals(len(funcs), nocc, seed=s) for s in range(nspin)]
+    occ = [np.linspace(1.0, 0.3, nocc)] * nspin
+    fb = A.FockBuilder(c, Z, A.make_manual_basis(funcs), (pts, w))
+    E, V, _ = fb.build(Cs, occ, precision="mixed")
+    Eo, Vo = O.xc_build(O.make_manual_basis(funcs), pts, w, PBE, Cs, occ)
+    assert abs(E - Eo) <= 1e-6 and max(np.abs(a - b).max() for a, b in zip(V, Vo)) <= 1e-7
     fb.close()
