@@ -761,7 +761,7 @@ def run_nkx(args):
             # measured in this run
             pd = fp64_gemm_peak(torch)
             v64 = flops / (fp64["stage_ms"]["vgemm_ms"] * 1e-3) / 1e12
-            fp64["roofline"] = {"kernel": "vgemm_fp64_kernel (V = Phi Z^T, FP64 CUDA cores)", "achieved": v64,
+            fp64["roofline"] = {"kernel": "vgemm_fp64_kernel (V = Phi Z^T, FP64 tensor instruction)", "achieved": v64,
                                 "peak": pd, "unit": "TFLOP/s", "frac": v64 / pd,
                                 "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (torch.matmul f64)"}
         # the measurements below build plans of their own: the headline plan's

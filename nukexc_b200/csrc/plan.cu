@@ -407,10 +407,10 @@ __device__ __forceinline__ bool block_has(const uint32_t *m, int I) { return (m[
 // (thread-major, coalesced); vpart_reduce_kernel adds the parts in order, so
 // the result does not depend on scheduling.
 //
-// Bound: FP64 pipe.  Whole FP64 builds, before (CUDA-core tiles, one CTA per
-// output tile, 64-column density, a radial factor per function) and after:
-// one water LDA + J 14.3 -> 0.77 ms (the V contraction was 13.4 of it, on two
-// SMs), (H2O)_5 open-shell PBE 70.3 -> 6.3 ms (64.3 of it, on eight SMs).
+// Bound: FP64 tensor pipe (80 % active at (H2O)_16).  V alone, before
+// (CUDA-core tiles, one CTA per output tile) and after: one water 13.4 ms (on
+// two SMs) -> 78 us, (H2O)_5 open-shell PBE 64.3 ms (on eight) -> 3.15 ms,
+// (H2O)_64 now 2.43 s (25.6 TFLOP/s, 72 % of a cuBLAS DGEMM).
 constexpr int kVKs = 16, kVStages = 4, kVLd = kBlockF + 4;
 constexpr int kVStageDoubles = 2 * kVKs * kVLd;
 constexpr int kVSmemBytes = kVStages * kVStageDoubles * 8;

@@ -44,14 +44,14 @@ def test_replayed_builds_equal_ordinary_builds(precision, jmode):
         E, V, J = fb.build([C2], [occ], precision=precision, **kw)
         Eo, Vo, Jo = ref.build([C2], [occ], precision=precision, **kw)
         assert abs(E - Eo) <= 1e-12 * abs(Eo)
-        # with J fused, V holds the Coulomb potential, whose fit vector varies
-        # at rounding level from build to build (below)
+        # with J fused, V holds the Coulomb potential of the fit (below)
         vtol = 1e-10 if jmode == "fused" else 1e-12
         assert float((V[0] - Vo[0]).abs().max()) <= vtol * float(Vo[0].abs().max())
         if jmode == "separate":
-            # the fit vector y is summed with atomic FP64 adds in varying order
-            # and the solve with the grid metric (condition number about 1e5 for
-            # this aux set) magnifies that rounding in J
+            # rounding in the density or in the fit vector y is magnified in J by
+            # the solve with the grid metric (condition number about 1e5 for this
+            # aux set).  y itself is summed slice by slice in a fixed order, so
+            # replays usually agree far closer
             assert float((J - Jo).abs().max()) <= 1e-10 * float(Jo.abs().max())
     assert fb.info()["graph_replays"] >= 2
     ref.close()
